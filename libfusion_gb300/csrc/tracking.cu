@@ -25,161 +25,11 @@
 #include "gbf_device.cuh"
 #include "gbf_internal.h"
 #include "gbf_kernels.h"
+#include "gn_step.cuh"
 
 namespace gbf {
 
 namespace {
-
-// ---------------------------------------------------------------------------
-// The Gauss-Newton step in FP64, spread over one warp: the 6x6 LDL^T with
-// symmetric diagonal pivoting (the documented method of Eigen::LDLT used at
-// icp_tracker.cpp:92; zero pivots act as a pseudo-inverse), the SE(3)
-// exponential of xi = (rho, phi), translation first (Sophus convention), and
-// the pose composition.  A dependent FP64 operation takes about 70 cycles on
-// this part and a division about 600: one thread doing the step alone took
-// ~26 us (and spilled the pivoted matrix to local memory), one warp takes
-// ~12 us.  Each value sees the same operations in the same order as in the
-// one-thread form (row-by-row elimination, forward and back substitution,
-// W^2, I + A W + B W^2 and V), which 4,000 generated cases reproduced bit for
-// bit, zero pivots and ties in the pivot search included.
-
-// Full-warp shuffles: every lane must reach each call (none may sit inside a
-// lane-dependent branch or operand).
-__device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ int shfl_i(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-// lane holding the unordered pair {a, b} of a symmetric 6x6 matrix (lower triangle, 21 lanes)
-__device__ __forceinline__ int tri6(int a, int b) { return a >= b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a; }
-__device__ __forceinline__ int diag6(int a) { return a * (a + 1) / 2 + a; }
-
-// x = A^-1 b.  In: lane tri6(r, c) holds A[r][c] (r >= c) in a,
-// lane o < 6 holds b[o] in bv.  Out: lane o < 6 gets x[o].  The symmetric
-// pivoting is a permutation the lanes track -- lane q < 6 holds perm[q] (the
-// original index at logical position q) and pos[q] (the logical position of
-// original index q) -- instead of moving rows and columns.
-__device__ double ldlt_solve6_warp(double a, double bv) {
-    const int lane = threadIdx.x & 31;
-    int r = 0;
-    while (r < 5 && (r + 1) * (r + 2) / 2 <= lane) ++r;
-    const int c = lane < 21 ? lane - r * (r + 1) / 2 : 0;
-    if (lane >= 21) r = 0;
-    int perm = lane, pos = lane;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        // the first logical i >= k with the largest |A(i,i)| (strictly larger replaces)
-        int p = k;
-        double best = fabs(shfl_d(a, diag6(shfl_i(perm, k))));
-#pragma unroll
-        for (int i = k + 1; i < 6; ++i) {
-            const double v = fabs(shfl_d(a, diag6(shfl_i(perm, i))));
-            if (v > best) {
-                best = v;
-                p = i;
-            }
-        }
-        if (p != k) {
-            const int ok = shfl_i(perm, k), op = shfl_i(perm, p);
-            if (lane == k) perm = op;
-            if (lane == p) perm = ok;
-            if (lane == ok) pos = p;
-            if (lane == op) pos = k;
-        }
-        const int pk = shfl_i(perm, k);
-        const double Dk = shfl_d(a, diag6(pk));
-        const int li = shfl_i(pos, r), lj = shfl_i(pos, c);
-        const int hi = max(li, lj), lo = min(li, lj);
-        const bool mine = lane < 21;
-        if (fabs(Dk) <= DBL_MIN) {
-            if (mine && lo == k && hi > k) a = 0.0;
-            continue;
-        }
-        if (mine && lo == k && hi > k) a = a / Dk;  // L(hi, k) = A(hi, k) / D(k)
-        const double Lh = shfl_d(a, tri6(shfl_i(perm, hi), pk));
-        const double Ll = shfl_d(a, tri6(shfl_i(perm, lo), pk));
-        if (mine && lo > k) a -= Lh * Ll * Dk;
-    }
-    // forward: z[i] -= L(i, k) z[k], k ascending; lane q < 6 holds z[q] (logical)
-    const int src = lane < 6 ? perm : 0;
-    double z = shfl_d(bv, src);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const double zk = shfl_d(z, k);
-        const int pk = shfl_i(perm, k);  // every lane takes part in every shuffle
-        const double L = shfl_d(a, lane < 6 ? tri6(perm, pk) : 0);
-        if (lane > k && lane < 6) z -= L * zk;
-    }
-    {
-        const double Dq = shfl_d(a, lane < 6 ? diag6(perm) : 0);
-        if (lane < 6) z = (fabs(Dq) > DBL_MIN) ? z / Dq : 0.0;
-    }
-    // backward: z[i] -= L(k, i) z[k], k = i+1 .. 5 ascending
-#pragma unroll
-    for (int i = 4; i >= 0; --i) {
-        const int pi = shfl_i(perm, i);
-        double zi = shfl_d(z, i);
-#pragma unroll
-        for (int k = i + 1; k < 6; ++k) zi -= shfl_d(a, tri6(shfl_i(perm, k), pi)) * shfl_d(z, k);
-        if (lane == i) z = zi;
-    }
-    return shfl_d(z, lane < 6 ? pos : 0);  // x[perm[q]] = z[q]
-}
-
-// element idx of W = [w]x (row-major 3x3)
-__device__ __forceinline__ double skew_at(int idx, double wx, double wy, double wz) {
-    return idx == 1 ? -wz : idx == 2 ? wy : idx == 3 ? wz : idx == 5 ? -wx : idx == 6 ? -wy : idx == 7 ? wx : 0.0;
-}
-
-// T = exp(xi) (lane o < 6 holds xi[o]); lane p < 12 gets T[p] (3x4 row-major).
-__device__ double se3_exp_warp(double xi) {
-    const int lane = threadIdx.x & 31;
-    const double x0 = shfl_d(xi, 0), x1 = shfl_d(xi, 1), x2 = shfl_d(xi, 2);
-    const double wx = shfl_d(xi, 3), wy = shfl_d(xi, 4), wz = shfl_d(xi, 5);
-    const double th2 = wx * wx + wy * wy + wz * wz;
-    const double th = sqrt(th2);
-    double A, B, C;
-    if (th < 1e-5) {
-        const double q = th2 / (lane == 0 ? 6.0 : lane == 1 ? 24.0 : 120.0);
-        A = 1.0 - shfl_d(q, 0);
-        B = 0.5 - shfl_d(q, 1);
-        C = 1.0 / 6.0 - shfl_d(q, 2);
-    } else {
-        double s, co;
-        sincos(th, &s, &co);  // the values of sin(th) and cos(th), one range reduction
-        // A = s / th, B = (1 - c) / th^2, C = (th - s) / (th^2 th): three lanes, one division
-        const double num = lane == 0 ? s : lane == 1 ? 1.0 - co : th - s;
-        const double den = lane == 0 ? th : lane == 1 ? th2 : th2 * th;
-        const double q = num / den;
-        A = shfl_d(q, 0);
-        B = shfl_d(q, 1);
-        C = shfl_d(q, 2);
-    }
-    // lane e < 9: rotation and V element (i, j) = (e / 3, e % 3)
-    const int e = lane < 9 ? lane : 0, i = e / 3, j = e % 3;
-    const double w2 = skew_at(i * 3, wx, wy, wz) * skew_at(j, wx, wy, wz) +
-                      skew_at(i * 3 + 1, wx, wy, wz) * skew_at(3 + j, wx, wy, wz) +
-                      skew_at(i * 3 + 2, wx, wy, wz) * skew_at(6 + j, wx, wy, wz);
-    const double I = (i == j) ? 1.0 : 0.0, w = skew_at(e, wx, wy, wz);
-    const double rot = I + A * w + B * w2;
-    const double V = I + B * w + C * w2;
-    // lane i < 3: translation V[i] . (x0, x1, x2)
-    const int t = lane < 3 ? lane : 0;
-    const double tr = shfl_d(V, t * 3) * x0 + shfl_d(V, t * 3 + 1) * x1 + shfl_d(V, t * 3 + 2) * x2;
-    // pose layout: lane p = ri * 4 + rj
-    const int ri = lane < 12 ? lane / 4 : 0, rj = lane < 12 ? lane % 4 : 0;
-    const double rv = shfl_d(rot, ri * 3 + (rj < 3 ? rj : 0));
-    const double tv = shfl_d(tr, ri);
-    return rj == 3 ? tv : rv;
-}
-
-// c = a b (pose_mul) with a spread over the warp (lane p < 12 holds a[p]) and b in
-// memory; lane p < 12 gets c[p].
-__device__ double pose_mul_warp(double ap, const double *b) {
-    const int lane = threadIdx.x & 31;
-    const int i = lane < 12 ? lane / 4 : 0, j = lane < 12 ? lane % 4 : 0;
-    const double a0 = shfl_d(ap, i * 4), a1 = shfl_d(ap, i * 4 + 1), a2 = shfl_d(ap, i * 4 + 2);
-    const double a3 = shfl_d(ap, i * 4 + 3);
-    if (j < 3) return (a0 * b[0 * 4 + j] + a1 * b[1 * 4 + j]) + a2 * b[2 * 4 + j];
-    return ((a0 * b[3] + a1 * b[7]) + a2 * b[11]) + a3;
-}
 
 // |log(T)| of an SE(3) element (the success test, icp_tracker.cpp:145)
 __device__ double se3_log_norm(const double T[12]) {
@@ -216,12 +66,6 @@ __device__ double se3_log_norm(const double T[12]) {
     return sqrt(rho[0] * rho[0] + rho[1] * rho[1] + rho[2] * rho[2] + th2);
 }
 
-__device__ __forceinline__ bool finite_pose(const double *T) {
-    for (int i = 0; i < 12; ++i)
-        if (!isfinite(T[i])) return false;
-    return true;
-}
-
 // ---------------------------------------------------------------------------
 // per-pixel rows
 __device__ __forceinline__ float interp2(const float *img, int w, float x, float y) {
@@ -245,10 +89,22 @@ __device__ __forceinline__ float3 interp2_igd(const float4 *img, int w, float x,
                        (a.z * bx + b.z * ax) * by + (c.z * bx + d.z * ax) * ay);
 }
 
-// ICPReduction::searchPoint + getRow (pose_estimator.cu:168-222)
-__device__ __forceinline__ bool icp_row(const SessionView &sv, int level, int cs, const M34 &T, const float4 vl,
-                                        const float4 nl4, float row[7]) {
+// What the rows of one level read besides the reference pixel.
+struct LevelIn {
+    int w, h;
+    float fx, fy, cx, cy;
+    float angle, dist;                    // the ICP gates
+    const float4 *__restrict__ vcur, *__restrict__ ncur, *__restrict__ igd;  // current frame
+};
+__device__ __forceinline__ LevelIn level_in(const SessionView &sv, int level, int cs) {
     const LevelK &K = sv.lv[level];
+    return LevelIn{K.w, K.h, K.fx, K.fy, K.cx, K.cy, sv.icp_angle, sv.icp_dist,
+                   sv.vmap[cs][level], sv.nmap[cs][level], sv.igd[cs][level]};
+}
+
+// ICPReduction::searchPoint + getRow (pose_estimator.cu:168-222)
+__device__ __forceinline__ bool icp_row(const LevelIn &K, const M34 &T, const float4 vl, const float4 nl4,
+                                        float row[7]) {
     if (isnan(vl.x)) return false;
     const float3 vg = T.apply(vl.x, vl.y, vl.z);
     // float invz = 1.0 / vlast_g.z in the reference: a double division rounded to
@@ -260,13 +116,13 @@ __device__ __forceinline__ bool icp_row(const SessionView &sv, int level, int cs
     const int v = __float2int_rd(((vg.y * invz) * K.fy + K.cy) + 0.5f);
     if (u < 0 || v < 0 || u >= K.w || v >= K.h) return false;
     const int q = v * K.w + u;
-    const float4 vc4 = sv.vmap[cs][level][q];
+    const float4 vc4 = K.vcur[q];
     const float3 ng = T.rotate(nl4.x, nl4.y, nl4.z);
-    const float4 nc4 = sv.nmap[cs][level][q];
+    const float4 nc4 = K.ncur[q];
     const float dist = norm3(vg.x - vc4.x, vg.y - vc4.y, vg.z - vc4.z);
     const float3 cr = cross3(make_float3(nc4.x, nc4.y, nc4.z), ng);
     const float sine = norm3(cr.x, cr.y, cr.z);
-    if (!(sine < sv.icp_angle && dist <= sv.icp_dist && !isnan(nc4.x) && !isnan(ng.x))) return false;
+    if (!(sine < K.angle && dist <= K.dist && !isnan(nc4.x) && !isnan(ng.x))) return false;
     const float3 vxn = cross3(vg, ng);
     row[0] = ng.x; row[1] = ng.y; row[2] = ng.z;
     row[3] = vxn.x; row[4] = vxn.y; row[5] = vxn.z;
@@ -274,18 +130,23 @@ __device__ __forceinline__ bool icp_row(const SessionView &sv, int level, int cs
     return true;
 }
 
-// Photometric constants of one reduction, evaluated once per CTA in the
-// reference's double precision (m_estimator.cu:366-373).
+// Photometric constants of one reduction (m_estimator.cu:366-373).  The
+// reference compares and scales in double; each FP64 instruction of a warp holds
+// its quarter of the SM for 64 cycles, so the comparisons use the floats that
+// divide at the same place (1e-4f and 1e-5f lie just below 1e-4 and 1e-5), and
+// one thread of a CTA makes the product (photo_huber).
 struct PhotoConst {
-    float stddev, huber;
+    float stddev, huber, inv;
     bool normalise, robust;
 };
-__device__ __forceinline__ PhotoConst photo_const(float stddev) {
+__device__ __forceinline__ float photo_huber(float stddev) { return (float)(1.345 * (double)stddev); }
+__device__ __forceinline__ PhotoConst photo_const(float stddev, float huber) {
     PhotoConst c;
     c.stddev = stddev;
-    c.normalise = (double)stddev > 10e-5;
-    c.robust = (double)stddev > 10e-6;
-    c.huber = (float)(1.345 * (double)stddev);
+    c.inv = __frcp_rn(stddev);
+    c.normalise = stddev > 1e-4f;
+    c.robust = stddev > 1e-5f;
+    c.huber = huber;
     return c;
 }
 
@@ -293,10 +154,9 @@ __device__ __forceinline__ PhotoConst photo_const(float stddev) {
 // PACKED: the current frame's intensity and gradients from its packed image
 // (sessions); otherwise from the three separate images (caller-owned images).
 template <bool PACKED>
-__device__ __forceinline__ bool rgb_row(const SessionView &sv, int level, int cs, const M34 &T,
+__device__ __forceinline__ bool rgb_row(const SessionView &sv, int level, int cs, const LevelIn &K, const M34 &T,
                                         const PhotoConst &pc, const float4 pt, const float il, float row[7]) {
     const float stddev = pc.stddev;
-    const LevelK &K = sv.lv[level];
     if (pt.w < 0 || isnan(pt.x)) return false;
     if (!isfinite(il)) return false;
     const float3 q = T.apply(pt.x, pt.y, pt.z);
@@ -305,7 +165,7 @@ __device__ __forceinline__ bool rgb_row(const SessionView &sv, int level, int cs
     if (!(u0 >= 2 && u0 < (float)(K.w - 2) && v0 >= 2 && v0 < (float)(K.h - 2))) return false;
     float ic, dx, dy;
     if (PACKED) {
-        const float3 g = interp2_igd(sv.igd[cs][level], K.w, u0, v0);
+        const float3 g = interp2_igd(K.igd, K.w, u0, v0);
         ic = g.x;
         dx = g.y;
         dy = g.z;
@@ -449,11 +309,12 @@ __device__ __forceinline__ void stage_ref_tile(ReduceSmem &sm, const SessionView
 
 template <bool PACKED>
 __device__ __forceinline__ void cta_partial(ReduceSmem &sm, const SessionView &sv, int level, int rs, int cs,
-                                            const M34 &T, float stddev, int cta, int tile, float *part) {
+                                            const M34 &T, float stddev, float huber, int cta, int tile, float *part) {
     auto &warp_sums = sm.warp_sums;
     float4 *s_v = sm.s_v, *s_n = sm.s_n;
     float *s_i = sm.s_i;
-    const PhotoConst pc = photo_const(stddev);
+    const PhotoConst pc = photo_const(stddev, huber);
+    const LevelIn in = level_in(sv, level, cs);
     const int P = sv.lv[level].w * sv.lv[level].h;
     const int first = cta * tile;
     const int n = min(tile, P - first);
@@ -475,8 +336,8 @@ __device__ __forceinline__ void cta_partial(ReduceSmem &sm, const SessionView &s
         for (int i = 0; i < kCtaPixels / kHalfThreads; ++i) {
             const int c = t + i * kHalfThreads;
             float row[7];
-            const bool ok = half == 0 ? icp_row(sv, level, cs, T, s_v[c], s_n[c], row)
-                                      : rgb_row<PACKED>(sv, level, cs, T, pc, s_v[c], s_i[c], row);
+            const bool ok = half == 0 ? icp_row(in, T, s_v[c], s_n[c], row)
+                                      : rgb_row<PACKED>(sv, level, cs, in, T, pc, s_v[c], s_i[c], row);
             if (ok) accumulate(acc, row);
         }
     } else {
@@ -485,8 +346,8 @@ __device__ __forceinline__ void cta_partial(ReduceSmem &sm, const SessionView &s
             const int c = t + i * kHalfThreads;
             if (c >= n) break;
             float row[7];
-            const bool ok = half == 0 ? icp_row(sv, level, cs, T, s_v[c], s_n[c], row)
-                                      : rgb_row<PACKED>(sv, level, cs, T, pc, s_v[c], s_i[c], row);
+            const bool ok = half == 0 ? icp_row(in, T, s_v[c], s_n[c], row)
+                                      : rgb_row<PACKED>(sv, level, cs, in, T, pc, s_v[c], s_i[c], row);
             if (ok) accumulate(acc, row);
         }
     }
@@ -567,7 +428,7 @@ struct ReduceArgs {
     float stddev;
 };
 
-__device__ void gn_epilogue(const SessionView &sv, int level, int iter, const double *s);
+__device__ __forceinline__ void gn_epilogue(const SessionView &sv, TrackState *ts, int level, int iter, const double *s);
 
 // Whether session `sv` runs this (level, iteration): the schedule of
 // compute_transform (icp_tracker.cpp:33-50) with its early `break` per level.
@@ -594,19 +455,18 @@ __global__ void __launch_bounds__(kReduceThreads, 4) gn_reduce_kernel(const Sess
     __shared__ ReduceSmem sm;
     stage_ref_tile(sm, sv, level, rs, blockIdx.x, sv.red_tile[level]);
     __shared__ M34 T;
-    __shared__ float stddev_s;
-    if (threadIdx.x == 0) {
+    __shared__ float stddev_s, huber_s;
+    if (!a.once && threadIdx.x < 12) T.m[threadIdx.x] = (float)ts->est[threadIdx.x];  // one conversion, not twelve
+    if (threadIdx.x == 32) {
         if (a.once) {
 #pragma unroll
             for (int i = 0; i < 12; ++i) T.m[i] = a.pose[i];
-            stddev_s = a.stddev;
-        } else {
-            T = pose_to_float(ts->est);
-            stddev_s = (a.iter == 0) ? 0.f : ts->stddev;
         }
+        stddev_s = a.once ? a.stddev : a.iter == 0 ? 0.f : ts->stddev;
+        huber_s = photo_huber(stddev_s);
     }
     __syncthreads();
-    cta_partial<true>(sm, sv, level, rs, cs, T, stddev_s, blockIdx.x, sv.red_tile[level],
+    cta_partial<true>(sm, sv, level, rs, cs, T, stddev_s, huber_s, blockIdx.x, sv.red_tile[level],
                 sv.partials + (size_t)blockIdx.x * kPartialStride);
     if (a.defer) return;  // gn_step_kernel, launched next, sums the partials and takes the step
     __threadfence();
@@ -620,7 +480,7 @@ __global__ void __launch_bounds__(kReduceThreads, 4) gn_reduce_kernel(const Sess
     sum_partials(sm, sv.partials, sv.red_ctas[level], total);
     if (threadIdx.x < kReduceWidth) ts->last_sums[threadIdx.x] = total[threadIdx.x];
     if (threadIdx.x == 0) sv.ctr[C_TICKET] = 0;
-    if (!a.once && threadIdx.x < 32) gn_epilogue(sv, level, a.iter, total);  // one warp
+    if (!a.once && threadIdx.x < 64) gn_epilogue(sv, ts, level, a.iter, total);  // two warps
 }
 
 // The session's sum of the partial records and the Gauss-Newton step, as the
@@ -634,70 +494,37 @@ __global__ void __launch_bounds__(kReduceThreads) gn_step_kernel(const SessionVi
     __shared__ double total[kReduceWidth];
     sum_partials(sm, sv.partials, sv.red_ctas[a.level], total);
     if (threadIdx.x < kReduceWidth) sv.ts->last_sums[threadIdx.x] = total[threadIdx.x];
-    if (threadIdx.x < 32) gn_epilogue(sv, a.level, a.iter, total);
+    if (threadIdx.x < 64) gn_epilogue(sv, sv.ts, a.level, a.iter, total);
 }
 
-// Host loop body of DenseTracking::compute_transform (icp_tracker.cpp:52-139),
-// run by the 32 lanes of one warp: create_jtjjtr (reduce_sum.h:48-61) into the
-// float matrices, A = w_icp H_icp + w_rgb H_rgb and b likewise widened to
-// double, the LDL^T solve, T <- exp(xi) T; then lane 0 keeps the books.
-__device__ void gn_epilogue(const SessionView &sv, int level, int iter, const double *s) {
-    TrackState *ts = sv.ts;
-    const int lane = threadIdx.x & 31;
-    // lane tri6(r, c) (r >= c): A[r][c]; lane o < 6: b[o].  The packed index of
-    // (i, j), i <= j < 7, is 7 i - i (i - 1) / 2 + (j - i).
-    double a = 0.0, bv = 0.0;
-    {
-        int r = 0;
-        while (r < 5 && (r + 1) * (r + 2) / 2 <= lane) ++r;
-        const int c = lane - r * (r + 1) / 2;  // c <= r
-        if (lane < 21) {
-            const int k = 7 * c - c * (c - 1) / 2 + (r - c);
-            a = (double)(sv.w_icp * (float)s[k] + sv.w_rgb * (float)s[29 + k]);
-        }
-        if (lane < 6) {
-            const int k = 7 * lane - lane * (lane - 1) / 2 + (6 - lane);
-            bv = (double)(sv.w_icp * (float)s[k] + sv.w_rgb * (float)s[29 + k]);
-        }
-    }
-    const double xi = ldlt_solve6_warp(a, bv);
-    const double E = se3_exp_warp(xi);
-    const double next = pose_mul_warp(E, ts->est);
-    const double old = lane < 12 ? ts->est[lane] : 0.0;
-    __syncwarp();
-    if (lane < 12) {
-        ts->est_prev[lane] = old;
-        ts->est[lane] = next;
-    }
-    __syncwarp();
-    if (lane != 0) return;
+// The bookkeeping of DenseTracking::compute_transform (icp_tracker.cpp:93-139)
+// after the step of (level, iter): errors, counts and the break of the level.
+// True when the step is taken back (Revertable::revert).
+__device__ __forceinline__ bool gn_books(const SessionView &sv, TrackState *ts, int level, int iter, const double *s) {
     const float r_icp = (float)s[27], n_icp = (float)s[28];
     const float r_rgb = (float)s[29 + 27], n_rgb = (float)s[29 + 28];
-    const float stddev_next = sqrtf(r_rgb / (n_rgb - 6.0f));
+    const float last_icp = (iter == 0) ? FLT_MAX : ts->icp_error;
+    const float last_rgb = (iter == 0) ? FLT_MAX : ts->rgb_error;
+    int icp_count = (iter == 0) ? 0 : ts->icp_count;
+    int rgb_count = (iter == 0) ? 0 : ts->rgb_count;
     ts->iterations += 1;
     ts->level_iters[level] += 1;
     ts->pixel_iterations += (long long)sv.lv[level].w * sv.lv[level].h;
     ts->icp_inliers = n_icp;
     ts->rgb_inliers = n_rgb;
-
-    const float last_icp = (iter == 0) ? FLT_MAX : ts->icp_error;
-    const float last_rgb = (iter == 0) ? FLT_MAX : ts->rgb_error;
-    int icp_count = (iter == 0) ? 0 : ts->icp_count;
-    int rgb_count = (iter == 0) ? 0 : ts->rgb_count;
     ts->level_done = 0;
-    ts->stddev = stddev_next;
+    ts->stddev = sqrtf(r_rgb / (n_rgb - 6.0f));
     float icp_error = sqrtf(r_icp) / n_icp;
     if (isnan(icp_error)) {
         ts->invalid = 1;
         ts->level_done = 1;
         ts->icp_error = icp_error;
-        return;
+        return false;
     }
     if (icp_error > last_icp) {
         if (icp_count >= 2) {
-            pose_copy(ts->est_prev, ts->est);
             ts->level_done = 1;
-            return;
+            return true;
         }
         icp_count++;
         icp_error = last_icp;
@@ -711,13 +538,12 @@ __device__ void gn_epilogue(const SessionView &sv, int level, int iter, const do
         ts->invalid = 1;
         ts->level_done = 1;
         ts->rgb_error = rgb_error;
-        return;
+        return false;
     }
     if (rgb_error > last_rgb) {
         if (rgb_count >= 2) {
-            pose_copy(ts->est_prev, ts->est);
             ts->level_done = 1;
-            return;
+            return true;
         }
         rgb_count++;
         rgb_error = last_rgb;
@@ -726,13 +552,43 @@ __device__ void gn_epilogue(const SessionView &sv, int level, int iter, const do
     }
     ts->rgb_error = rgb_error;
     ts->rgb_count = rgb_count;
+    return false;
+}
+
+// Host loop body of DenseTracking::compute_transform (icp_tracker.cpp:52-139),
+// run by the first two warps of a CTA: create_jtjjtr (reduce_sum.h:48-61) into
+// the float matrices, A = w_icp H_icp + w_rgb H_rgb and b likewise widened to
+// double, the LDL^T solve and T <- exp(xi) T on the first warp; the books on
+// the second, which has the other FP32 and memory work to itself meanwhile.
+__device__ __forceinline__ void gn_epilogue(const SessionView &sv, TrackState *ts, int level, int iter, const double *s) {
+    const int lane = threadIdx.x & 31;
+    __shared__ int revert;
+    if (threadIdx.x >= 32) {
+        if (lane == 0) revert = gn_books(sv, ts, level, iter, s) ? 1 : 0;
+        __syncwarp();
+        asm volatile("bar.sync 5, 64;" ::: "memory");
+        return;
+    }
+    // lane p = 4 i + j < 12 holds column j of the estimate
+    const int i = lane < 12 ? lane / 4 : 0, j = lane & 3;
+    const double t0 = ts->est[j], t1 = ts->est[4 + j], t2 = ts->est[8 + j];
+    // lane tri6(r, c) (r >= c, r < 6): A[r][c]; lane 21 + c: b[c].  The packed
+    // index of (i, j), i <= j < 7, is 7 i - i (i - 1) / 2 + (j - i); b is column 6.
+    const int r = tri_row(lane), c = lane < 27 ? lane - r * (r + 1) / 2 : 0;
+    const int k = 7 * c - c * (c - 1) / 2 + (r - c);
+    const double a = lane < 27 ? (double)(sv.w_icp * (float)s[k] + sv.w_rgb * (float)s[29 + k]) : 0.0;
+    const double xi = ldlt_solve6_warp(a);
+    const double next = se3_exp_mul_warp(xi, t0, t1, t2);
+    asm volatile("bar.sync 5, 64;" ::: "memory");
+    if (lane < 12) {
+        const double old = i == 0 ? t0 : i == 1 ? t1 : t2;
+        ts->est_prev[lane] = old;
+        ts->est[lane] = revert ? old : next;
+    }
 }
 
 // frame_mode 1: System frame (track only when a reference exists); 0: gbf_track.
-__global__ void track_begin_kernel(const SessionView *__restrict__ svs, int frame_mode) {
-    const SessionView &sv = svs[blockIdx.x];
-    if (!sv.active || threadIdx.x != 0) return;
-    TrackState *ts = sv.ts;
+__device__ __forceinline__ void track_begin(TrackState *ts, int frame_mode) {
     ts->tracking = frame_mode ? ts->has_ref : 1;
     // Revertable(initial_estimate): curr = init, prev = identity
     pose_copy(ts->init, ts->est);
@@ -745,54 +601,129 @@ __global__ void track_begin_kernel(const SessionView *__restrict__ svs, int fram
     ts->rgb_error = FLT_MAX;
     ts->stddev = 0.f;
     ts->icp_count = ts->rgb_count = 0;
-    sv.ctr[C_TICKET] = 0;
 }
 
-// Tracking result (icp_tracker.cpp:143-155); frame_mode 1 also applies the
-// System / DenseOdometry bookkeeping (rgbd_odometry.cpp:39-41): pose update
-// and reference swap.
-__global__ void track_finish_kernel(const SessionView *__restrict__ svs, int frame_mode) {
-    const SessionView &sv = svs[blockIdx.x];
-    if (!sv.active || threadIdx.x != 0) return;
-    TrackState *ts = sv.ts;
-    if (ts->tracking) {
-        double inv[12], rel[12];
-        pose_inverse(ts->est, inv);
-        pose_mul(inv, ts->init, rel);
-        const double n = se3_log_norm(rel);
-        const bool finite = finite_pose(ts->est);
-        const bool fail = ts->invalid || !(n <= 0.1) || !finite;
-        if (!finite) raise_flag(sv, GBF_FLAG_NAN_POSE);
-        if (fail) {
-            pose_identity(ts->update);
-            ts->success = 0;
-        } else {
-            pose_copy(inv, ts->update);
-            ts->success = 1;
+// The success test of the tracking result (icp_tracker.cpp:145), |log(est^-1 init)| <= 0.1.
+__device__ __noinline__ bool moved_too_far(const double *est, const double *init) {
+    double inv[12], rel[12];
+    pose_inverse(est, inv);
+    pose_mul(inv, init, rel);
+    return !(se3_log_norm(rel) <= 0.1);
+}
+
+// The same test decided in FP32 where the norm is clearly on one side: -1 when it
+// is not (near the bound, large rotations or coordinates, non-finite poses).  With
+// |elements| <= 50 and a rotation below 0.46 rad (trace > 2.8) every step is
+// within a few 1e-6 of the FP64 one, against a margin of 1e-3.
+__device__ __forceinline__ int moved_too_far_f32(const float *e, const float *init) {
+    float m = 0.f;
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+        m = fmaxf(m, fmaxf(fabsf(e[i]), fabsf(init[i])));
+        finite = finite && isfinite(e[i]) && isfinite(init[i]);
+    }
+    float R[9], t[3], d[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) d[k] = init[k * 4 + 3] - e[k * 4 + 3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        t[i] = e[i] * d[0] + e[4 + i] * d[1] + e[8 + i] * d[2];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) R[i * 3 + j] = e[i] * init[j] + e[4 + i] * init[4 + j] + e[8 + i] * init[8 + j];
+    }
+    if (!finite || !(m <= 50.f) || !(R[0] + R[4] + R[8] > 2.8f)) return -1;
+    float wx = 0.5f * (R[7] - R[5]), wy = 0.5f * (R[2] - R[6]), wz = 0.5f * (R[3] - R[1]);
+    const float s = norm3(wx, wy, wz);
+    const float k = s > 1e-4f ? asinf(fminf(s, 1.f)) / s : 1.f;
+    wx *= k;
+    wy *= k;
+    wz *= k;
+    const float th2 = wx * wx + wy * wy + wz * wz;
+    // rho = t - w x t / 2 + f w x (w x t), f = 1/12 + th^2/720 + ...
+    const float3 w = make_float3(wx, wy, wz), tv = make_float3(t[0], t[1], t[2]);
+    const float3 c1 = cross3(w, tv), c2 = cross3(w, c1);
+    const float f = 1.f / 12.f + th2 * (1.f / 720.f + th2 * (1.f / 30240.f));
+    const float rx = tv.x - 0.5f * c1.x + f * c2.x, ry = tv.y - 0.5f * c1.y + f * c2.y, rz = tv.z - 0.5f * c1.z + f * c2.z;
+    const float n = sqrtf(rx * rx + ry * ry + rz * rz + th2);
+    return n < 0.099f ? 0 : n > 0.101f ? 1 : -1;
+}
+
+// Tracking result (icp_tracker.cpp:143-155), by one warp (all lanes); frame_mode 1
+// also applies the System / DenseOdometry bookkeeping (rgbd_odometry.cpp:39-41): pose update
+// and reference swap.  The pose products take one lane per element; with one
+// thread, and the FP64 logarithm of every frame's motion, this took 18 us.
+__device__ __forceinline__ void track_finish(const SessionView &sv, TrackState *ts, int frame_mode) {
+    const int lane = threadIdx.x & 31, p = lane < 12 ? lane : 0;
+    const double identity = (p == 0 || p == 5 || p == 10) ? 1.0 : 0.0;
+    const bool tracking = ts->tracking;
+    double pose = ts->pose[p], update = ts->update[p], init = ts->init[p];
+    bool success = ts->success;
+    if (tracking) {
+        const double est = ts->est[p];
+        float e[12], f[12];
+#pragma unroll
+        for (int i = 0; i < 12; ++i) {
+            e[i] = __shfl_sync(0xffffffffu, (float)est, i);
+            f[i] = __shfl_sync(0xffffffffu, (float)init, i);
         }
-        if (frame_mode) {
-            double np[12];
-            pose_mul(ts->pose, ts->update, np);
-            pose_copy(np, ts->pose);
-            if (fail) raise_flag(sv, GBF_FLAG_TRACK_FAILED);
+        int far = moved_too_far_f32(e, f);
+        if (far < 0) {
+            if (lane == 0) far = moved_too_far(ts->est, ts->init) ? 1 : 0;
+            far = __shfl_sync(0xffffffffu, far, 0);
+        }
+        const bool finite = __all_sync(0xffffffffu, isfinite(est));
+        success = !(ts->invalid || far || !finite);
+        update = pose_inverse_warp(est);
+        if (!success) update = identity;
+        if (frame_mode) pose = pose_mul_warp(pose, update);
+        if (lane == 0) {
+            if (!finite) raise_flag(sv, GBF_FLAG_NAN_POSE);
+            if (!success && frame_mode) raise_flag(sv, GBF_FLAG_TRACK_FAILED);
         }
     } else if (frame_mode) {
-        ts->success = 1;
-        pose_identity(ts->update);
+        success = true;
+        update = identity;
     }
+    const double inv = pose_inverse_warp(frame_mode ? pose : update);
     if (frame_mode) {
         // the next frame's initial estimate: no motion (the reference), or
         // with the constant-velocity prior the motion this frame tracked
-        if (sv.motion_prior && ts->tracking && ts->success)
-            pose_inverse(ts->update, ts->init);
-        else
-            pose_identity(ts->init);
-        ts->idx = 1 - ts->idx;
-        ts->has_ref = 1;
-        pose_copy(ts->pose, ts->map_pose);
-        update_map_floats(ts);
-        ts->frame_index += 1;
+        init = identity;
+        if (sv.motion_prior && tracking && success) init = pose_inverse_warp(update);
     }
+    __syncwarp();
+    if (lane < 12) {
+        if (tracking || frame_mode) ts->update[p] = update;
+        if (frame_mode) {
+            ts->pose[p] = pose;
+            ts->init[p] = init;
+            ts->map_pose[p] = pose;
+            ts->map_twc[p] = (float)pose;  // update_map_floats
+            ts->map_tcw[p] = (float)inv;
+        }
+    }
+    if (lane == 0) {
+        if (tracking || frame_mode) ts->success = success ? 1 : 0;
+        if (frame_mode) {
+            ts->idx = 1 - ts->idx;
+            ts->has_ref = 1;
+            ts->frame_index += 1;
+        }
+    }
+    __syncwarp();
+}
+
+__global__ void track_begin_kernel(const SessionView *__restrict__ svs, int frame_mode) {
+    const SessionView &sv = svs[blockIdx.x];
+    if (!sv.active || threadIdx.x != 0) return;
+    track_begin(sv.ts, frame_mode);
+    sv.ctr[C_TICKET] = 0;
+}
+
+__global__ void track_finish_kernel(const SessionView *__restrict__ svs, int frame_mode) {
+    const SessionView &sv = svs[blockIdx.x];
+    if (sv.active) track_finish(sv, sv.ts, frame_mode);
 }
 
 }  // namespace
@@ -912,11 +843,14 @@ __global__ void __launch_bounds__(kReduceThreads, 3) reduce_static_kernel(Sessio
     __shared__ ReduceSmem sm;
     stage_ref_tile(sm, sv, 0, 0, blockIdx.x, kCtaPixels);
     __shared__ M34 T;
-    if (threadIdx.x == 0)
+    __shared__ float huber_s;
+    if (threadIdx.x == 0) {
 #pragma unroll
         for (int i = 0; i < 12; ++i) T.m[i] = a.pose[i];
+        huber_s = photo_huber(a.stddev);
+    }
     __syncthreads();
-    cta_partial<false>(sm, sv, 0, 0, 1, T, a.stddev, blockIdx.x, kCtaPixels, scratch + (size_t)blockIdx.x * kPartialStride);
+    cta_partial<false>(sm, sv, 0, 0, 1, T, a.stddev, huber_s, blockIdx.x, kCtaPixels, scratch + (size_t)blockIdx.x * kPartialStride);
     __threadfence();
     __syncthreads();
     __shared__ unsigned int ticket;
