@@ -25,7 +25,7 @@ gbf_status check_cuda(const char *where);
 struct ArenaLayout {
     size_t total;
     size_t table, bcoord, bstamp, bfresh, vis, mesh_off, vox_sw, vox_rgb, ctr, ts;
-    size_t in_depth, in_rgb, depth_raw, rgb4, nmap_ext, fuse_px, zr_min, zr_max, partials;
+    size_t in_depth, in_rgb, depth_raw, rgb4, nmap_ext, fuse_px, zr_min, zr_max, partials, track_rec;
     size_t depth[kMaxLevels], inten[2][kMaxLevels], gx[kMaxLevels], gy[kMaxLevels];
     size_t vmap[2][kMaxLevels], nmap[2][kMaxLevels], igd[2][kMaxLevels];
 };
@@ -93,6 +93,7 @@ struct gbf_batch {
     std::vector<char> owed;                         // slot owes the second half of its last frame
     static constexpr int kMaxGroups = 4;
     int groups = 2;                                // concurrent session groups per tick
+    int groups_set = 0;                            // by the caller or the tuner (else see tick_groups)
     cudaStream_t side[kMaxGroups - 1] = {};        // branch streams of groups 1..
     cudaEvent_t fork = nullptr, join[kMaxGroups - 1] = {};
     int ray_tw = 8;                                // raycast tile width (64-pixel tiles)

@@ -72,9 +72,15 @@ void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, cudaStre
 
 // ---- tracking (tracking.cu) -----------------------------------------------------
 // mode 0: full Gauss-Newton (gbf_track / process frame), stops at the schedule end
+// alone: no other launch of this library runs beside it (not one of several
+// branches of a tick), so a few sessions may take the whole chip.
 // kernel launches of one launch_track over nslots sessions
-int track_launches(int nslots, const Extent &ex);
-void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, cudaStream_t st);
+int track_launches(int nslots, const Extent &ex, bool alone);
+void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, bool alone, cudaStream_t st);
+// sessions up to which a launch alone on the chip tracks in one cooperative kernel
+int track_run_sessions();
+// what launch_track needs of the current device, asked once (before any stream capture)
+void prepare_track();
 // single reduction for gbf_reduce: pose given as float 3x4 in the kernel args
 void launch_reduce_once(const SessionView *d_sv, const Extent &ex, int level, const float *pose12, float stddev,
                         cudaStream_t st);

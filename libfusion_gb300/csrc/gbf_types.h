@@ -55,7 +55,9 @@ enum Counter {
     C_MESH_BLOCKS = 6,
     C_MESH_TRIS = 7,
     C_GC_DELETED = 8, // blocks deleted by the last garbage collection
-    C_COUNT = 16
+    C_COUNT = 16,     // counters proper (reported, kept by snapshots)
+    C_TRACK_PUB = 16, // 14 8-byte words published within a tracking run (gn_track_kernel)
+    C_WORDS = 64      // ints in the arena
 };
 
 // Tracking and pose state of a session, resident on the device.
@@ -133,6 +135,7 @@ struct SessionView {
 
     TrackState *ts;
     float *partials;       // [red_ctas][kPartialStride]
+    unsigned long long *track_rec;  // [red_ctas][kPartialStride] (gn_track_kernel)
     int *mesh_off;         // per-block triangle counts / offsets (pool + 1)
 };
 

@@ -96,7 +96,7 @@ ArenaLayout plan_arena(const gbf_config &c, const gbf_intrinsics &K) {
     a.mesh_off = take((pool + 1) * sizeof(int));
     a.vox_sw = take(nv * (c.voxel_layout == GBF_VOXEL_REF ? 8 : 4));
     a.vox_rgb = take(nv * 4);
-    a.ctr = take(C_COUNT * sizeof(int));
+    a.ctr = take(C_WORDS * sizeof(int));
     a.ts = take(sizeof(TrackState));
     const size_t P = (size_t)K.width * K.height;
     a.in_depth = take(P * 2);
@@ -126,6 +126,7 @@ ArenaLayout plan_arena(const gbf_config &c, const gbf_intrinsics &K) {
     for (int l = 0, lw = K.width, lh = K.height; l < c.num_levels; ++l, lw /= 2, lh /= 2)
         max_ctas = std::max(max_ctas, (lw * lh + reduce_tile(l) - 1) / reduce_tile(l));
     a.partials = take((size_t)max_ctas * kPartialStride * 4);
+    a.track_rec = take((size_t)max_ctas * kPartialStride * 8);
     a.total = off;
     return a;
 }
@@ -225,9 +226,12 @@ TrackState initial_track_state() {
 
 gbf_status reset_session(gbf_session *s, cudaStream_t st, bool keep_track = false) {
     reset_table_kernel<<<512, 256, 0, st>>>(s->view.table, s->cfg.num_buckets);
-    cudaError_t e = cudaMemsetAsync(s->view.ctr, 0, C_COUNT * sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(s->view.ctr, 0, C_WORDS * sizeof(int), st);
     if (e != cudaSuccess) return cuda_error(e, "reset");
     e = cudaMemsetAsync(s->view.bfresh, 0, (size_t)s->cfg.num_blocks, st);
+    if (e != cudaSuccess) return cuda_error(e, "reset");
+    // the tracking run's words, numbered from the counters just cleared
+    e = cudaMemsetAsync(s->view.track_rec, 0, s->lay.total - s->lay.track_rec, st);
     if (e != cudaSuccess) return cuda_error(e, "reset");
     if (!keep_track) {
         const TrackState t = initial_track_state();
@@ -283,13 +287,13 @@ struct PhaseMarks {
 
 // First half of a frame: ingest and tracking (the pose of the frame is final
 // after it).
-void enqueue_first_half(const SessionView *d_sv, int nslots, const Extent &ex, const IngestArgs &in, cudaStream_t st,
-                        cudaEvent_t *ev = nullptr) {
+void enqueue_first_half(const SessionView *d_sv, int nslots, const Extent &ex, const IngestArgs &in, bool alone,
+                        cudaStream_t st, cudaEvent_t *ev = nullptr) {
     PhaseMarks mark(ev, st);
     mark(0, st);
     launch_ingest(d_sv, nslots, ex, in, st);
     mark(1, st);
-    launch_track(d_sv, nslots, ex, 1, st);
+    launch_track(d_sv, nslots, ex, 1, alone, st);
     mark(2, st);
 }
 
@@ -311,16 +315,16 @@ void enqueue_second_half(const SessionView *d_sv, int nslots, const Extent &ex, 
 }
 
 void enqueue_frame(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, const IngestArgs &in,
-                   cudaStream_t st, cudaEvent_t *ev = nullptr) {
-    enqueue_first_half(d_sv, nslots, ex, in, st, ev);
+                   bool alone, cudaStream_t st, cudaEvent_t *ev = nullptr) {
+    enqueue_first_half(d_sv, nslots, ex, in, alone, st, ev);
     enqueue_second_half(d_sv, nslots, ex, layouts, st, ev);
 }
 
 // kernels launched by enqueue_frame
-int kernels_per_frame(const Extent &ex, const int *layouts, int nslots) {
+int kernels_per_frame(const Extent &ex, const int *layouts, int nslots, bool alone) {
     int nl = 0;
     for (int l = 0; l < kNumLayouts; ++l) nl += layouts[l];
-    return (1 + (ex.levels - 1) + 1) + track_launches(nslots, ex) + 3 + nl + 2 + nl + post_launches(ex);
+    return (1 + (ex.levels - 1) + 1) + track_launches(nslots, ex, alone) + 3 + nl + 2 + nl + post_launches(ex);
 }
 
 }  // namespace
@@ -461,6 +465,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     v.zr_w = K->width / 8;
     v.zr_h = K->height / 8;
     v.partials = reinterpret_cast<float *>(base + a.partials);
+    v.track_rec = reinterpret_cast<unsigned long long *>(base + a.track_rec);
 
     Extent &ex = s->ex;
     memset(&ex, 0, sizeof(ex));
@@ -473,6 +478,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
         ex.max_iter[l] = cfg->max_iterations[l];
     }
     s->layouts[cfg->voxel_layout] = 1;
+    prepare_track();
 
     e = cudaMemcpy(s->d_view, &v, sizeof(v), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -744,7 +750,7 @@ GBF_API gbf_status gbf_track(gbf_session *s, const double init[16], gbf_track_re
     to34(init, p);
     cudaError_t e = cudaMemcpyAsync(s->view.ts->init, p, sizeof(p), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_error(e, "gbf_track");
-    launch_track(s->d_view, 1, s->ex, 0, st);
+    launch_track(s->d_view, 1, s->ex, 0, true, st);
     gbf_status r = check_cuda("gbf_track");
     if (r != GBF_OK) return r;
     TrackState t;
@@ -792,14 +798,14 @@ GBF_API gbf_status gbf_process_frame(gbf_session *s, const uint16_t *depth, int6
     if (!rows_aligned(depth, depth_pitch, 2))
         return set_error(GBF_ERR_INVALID_ARG, "gbf_process_frame: depth rows must be 2-byte aligned");
     IngestArgs a{0, 1, depth, depth_pitch, rgb, rgb_pitch};
-    enqueue_frame(s->d_view, 1, s->ex, s->layouts, a, (cudaStream_t)stream);
+    enqueue_frame(s->d_view, 1, s->ex, s->layouts, a, true, (cudaStream_t)stream);
     return check_cuda("gbf_process_frame");
 }
 
 GBF_API gbf_status gbf_process_frame_staged(gbf_session *s, void *stream) {
     if (!s) return set_error(GBF_ERR_INVALID_ARG, "gbf_process_frame_staged: null");
     IngestArgs a{0, 0, nullptr, 0, nullptr, 0};
-    enqueue_frame(s->d_view, 1, s->ex, s->layouts, a, (cudaStream_t)stream);
+    enqueue_frame(s->d_view, 1, s->ex, s->layouts, a, true, (cudaStream_t)stream);
     return check_cuda("gbf_process_frame_staged");
 }
 
@@ -1125,7 +1131,16 @@ static void batch_results(gbf_batch *b, int k, cudaStream_t st) {
     cudaMemcpyAsync(b->h_res[k], b->d_res[k], sizeof(gbf_slot_result) * b->nslots, cudaMemcpyDeviceToHost, st);
 }
 
-static int effective_groups(const gbf_batch *b) { return b->timing ? 1 : std::min(b->groups, b->nslots); }
+// Branches of a tick.  Where the caller or the tuner has not set a number, few
+// sessions run as one: they then track in one launch that takes the chip
+// (launch_track), 0.73 against 0.83 ms per tick for two 640x480 sessions, 0.87
+// against 0.92 for three, 1.01 against 1.03 for four; from six on two branches
+// are faster (1.42 against 1.45 ms).
+static int tick_groups(const gbf_batch *b) {
+    if (!b->groups_set && !b->stagger && b->nslots <= track_run_sessions()) return 1;
+    return std::max(1, std::min(b->groups, b->nslots));
+}
+static int effective_groups(const gbf_batch *b) { return b->timing ? 1 : tick_groups(b); }
 static bool staggered(const gbf_batch *b) { return b->stagger && effective_groups(b) >= 2; }
 static int group_lo(const gbf_batch *b, int g, int groups) { return b->nslots * g / groups; }
 
@@ -1137,7 +1152,7 @@ static void batch_enqueue(gbf_batch *b, int k, cudaStream_t st) {
     if (stag)
         cudaMemcpyAsync(b->d_views_b, b->h_views_b[k], sizeof(SessionView) * b->nslots, cudaMemcpyHostToDevice, st);
     if (groups <= 1) {
-        enqueue_frame(b->d_views, b->nslots, b->ex, b->layouts, a, st, b->timing ? b->pev[k] : nullptr);
+        enqueue_frame(b->d_views, b->nslots, b->ex, b->layouts, a, true, st, b->timing ? b->pev[k] : nullptr);
         batch_results(b, k, st);
         return;
     }
@@ -1151,9 +1166,9 @@ static void batch_enqueue(gbf_batch *b, int k, cudaStream_t st) {
             // then this frame's ingest and tracking, so that this group's tracking
             // runs beside the even groups' fusion and raycast and the other way round
             enqueue_second_half(b->d_views_b + lo, hi - lo, b->ex, b->layouts, gs);
-            enqueue_first_half(b->d_views + lo, hi - lo, b->ex, a, gs);
+            enqueue_first_half(b->d_views + lo, hi - lo, b->ex, a, false, gs);
         } else {
-            enqueue_frame(b->d_views + lo, hi - lo, b->ex, b->layouts, a, gs);
+            enqueue_frame(b->d_views + lo, hi - lo, b->ex, b->layouts, a, false, gs);
         }
     }
     for (int g = 1; g < groups; ++g) {
@@ -1288,7 +1303,7 @@ void tune_collect(gbf_batch *b, int k, bool wait) {
 
 // Switch the launch shape: owed halves run, ticks in flight end, graphs go.
 gbf_status apply_shape(gbf_batch *b, const gbf_batch::Shape &c, cudaStream_t st) {
-    if (c.groups == b->groups && c.stagger == b->stagger && c.ray_tw == b->ray_tw) return GBF_OK;
+    if (b->groups_set && c.groups == b->groups && c.stagger == b->stagger && c.ray_tw == b->ray_tw) return GBF_OK;
     gbf_status fs = batch_flush(b, st);
     if (fs != GBF_OK) return fs;
     for (int k = 0; k < 2; ++k)
@@ -1299,6 +1314,7 @@ gbf_status apply_shape(gbf_batch *b, const gbf_batch::Shape &c, cudaStream_t st)
         }
     batch_invalidate(b);
     b->groups = c.groups;
+    b->groups_set = 1;
     b->stagger = c.stagger;
     b->ray_tw = c.ray_tw;
     b->ex.ray_tw = c.ray_tw;
@@ -1529,8 +1545,9 @@ GBF_API gbf_status gbf_batch_set_groups(gbf_batch *b, int32_t groups) {
     for (int k = 0; k < 2; ++k)
         if (b->ev_used[k]) cudaEventSynchronize(b->ev[k]);
     tune_off(b);
-    if (groups != b->groups) batch_invalidate(b);
+    if (groups != b->groups || !b->groups_set) batch_invalidate(b);
     b->groups = groups;
+    b->groups_set = 1;
     return GBF_OK;
 }
 
@@ -1666,9 +1683,10 @@ GBF_API gbf_status gbf_batch_kernels(gbf_batch *b, int32_t *n) {
     if (!b || !n) return set_error(GBF_ERR_INVALID_ARG, "gbf_batch_kernels: null");
     std::lock_guard<std::mutex> lock(b->mu);
     int total = 0;
-    const int groups = std::max(1, std::min(b->groups, b->nslots));
+    const int groups = tick_groups(b);
     for (int g = 0; g < groups; ++g)
-        total += kernels_per_frame(b->ex, b->layouts, b->nslots * (g + 1) / groups - b->nslots * g / groups);
+        total += kernels_per_frame(b->ex, b->layouts, b->nslots * (g + 1) / groups - b->nslots * g / groups,
+                                   groups == 1);
     *n = b->nslots ? total + 1 : 0;
     return GBF_OK;
 }

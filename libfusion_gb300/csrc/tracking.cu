@@ -20,6 +20,7 @@
 #include <float.h>
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "gbf_device.cuh"
@@ -726,6 +727,449 @@ __global__ void track_finish_kernel(const SessionView *__restrict__ svs, int fra
     if (sv.active) track_finish(sv, sv.ts, frame_mode);
 }
 
+// ---------------------------------------------------------------------------
+// A whole tracking run (every level and iteration, from the initial estimate to
+// the frame's pose) in one cooperative launch, for launches of few sessions.
+//
+// What bounds such a run is latency.  A launch per iteration costs one 640x480
+// session about 18 us: the launch, the dependent loads from the descriptor to the
+// first pixel, four rounds of gathers one after another, a last CTA that sums
+// the records and the step, of which the chip is busy for a quarter.  Here one
+// CTA per SM stays for the run, its code and the maps it gathers from in its
+// caches.  512 threads make the two rows of two pixels each of a 1024-pixel tile,
+// every gather of the tile in flight at once, into shared memory (zeros for a
+// rejected row); then two threads sum the 29 products of each eight-pixel chain,
+// where holding 29 sums while gathering leaves registers for two pixels in
+// flight.  CTA 0 makes no rows: it sums the tiles' records as they arrive, takes
+// the step on the tracking state in its shared memory and publishes the next
+// pose, so that the step's code stays in one SM's instruction cache.
+// An iteration then takes 10 us at 160x120 and 320x240 and 15 us at 640x480
+// (two tiles per CTA: 7 us; step 3.7; each hop between CTAs 0.7), the run of a
+// 640x480 frame 0.25 -> 0.16 ms.  1024 threads of 64 registers spilled (0.25 ms);
+// the step by whichever CTA came last ran 25% slower from cold instruction
+// caches; coarse tiles split over two or four CTAs cost more in records than they saved.
+//
+// Every sum keeps the terms and the order of gn_reduce_kernel: a chain adds
+// pixels t, t + 128, ... of the tile in turn (fused multiply-adds; a zero row
+// adds nothing), a warp adds its 32 chains in a butterfly (xor 16, 8, 4, 2, 1),
+// the tile adds its four warps in order, the records follow as in sum_partials.
+constexpr int kTrackThreads = 512;
+constexpr int kTrackPixels = kCtaPixels / kTrackThreads;  // of a tile per thread
+struct TrackSmem {
+    float4 lo[2][kCtaPixels];  // ICP, photometric: row[0..3]
+    float4 hi[2][kCtaPixels];  // row[4..6], 1 for a valid row
+    float warp_sums[4][kReduceWidth];
+    float2 grp[kSumGroups][kReduceWidth];
+    double total[kReduceWidth];
+    TrackState ts;  // CTA 0: the run's tracking state
+    float pose[12];
+    float stddev, huber;
+    int item, seen, lost;
+};
+
+// icp_row and rgb_row of one pixel, with their gathers issued together (a row
+// rejected before its gather reads pixel 0 and is masked after).
+__device__ __forceinline__ void pixel_rows(const LevelIn &K, const M34 &T, const PhotoConst &pc, const float4 pt,
+                                           const float4 nr, float il, float4 *icp_lo, float4 *icp_hi, float4 *rgb_lo,
+                                           float4 *rgb_hi) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float3 p = T.apply(pt.x, pt.y, pt.z);
+    const float zi = __frcp_rn(p.z);
+    const int u = __float2int_rd(((p.x * zi) * K.fx + K.cx) + 0.5f);
+    const int w = __float2int_rd(((p.y * zi) * K.fy + K.cy) + 0.5f);
+    bool ok = !isnan(pt.x) && !(u < 0 || w < 0 || u >= K.w || w >= K.h);
+    const int q = ok ? w * K.w + u : 0;
+    // p.x / p.z and p.y / p.z from the reciprocal at hand (div_rn_by; where z has none,
+    // the quotient is outside the image or NaN either way)
+    const float u0 = div_rn_by(p.x, p.z, zi) * K.fx + K.cx;
+    const float v0 = div_rn_by(p.y, p.z, zi) * K.fy + K.cy;
+    bool okr = !(pt.w < 0 || isnan(pt.x)) && isfinite(il) &&
+               (u0 >= 2 && u0 < (float)(K.w - 2) && v0 >= 2 && v0 < (float)(K.h - 2));
+    const int iu = (int)floorf(u0), iv = (int)floorf(v0);
+    const float4 *r0 = K.igd + (okr ? iv * K.w + iu : 0);
+    const float4 vc = K.vcur[q], nc = K.ncur[q];
+    const float4 a = r0[0], b = r0[1], c = r0[K.w], d = r0[K.w + 1];
+    {
+        const float3 ng = T.rotate(nr.x, nr.y, nr.z);
+        const float dist = norm3(p.x - vc.x, p.y - vc.y, p.z - vc.z);
+        const float3 cr = cross3(make_float3(nc.x, nc.y, nc.z), ng);
+        const float sine = norm3(cr.x, cr.y, cr.z);
+        ok = ok && sine < K.angle && dist <= K.dist && !isnan(nc.x) && !isnan(ng.x);
+        const float3 x = cross3(p, ng);
+        const float r = dot3(ng, make_float3(vc.x - p.x, vc.y - p.y, vc.z - p.z));
+        *icp_lo = ok ? make_float4(ng.x, ng.y, ng.z, x.x) : zero;
+        *icp_hi = ok ? make_float4(x.y, x.z, r, 1.f) : zero;
+    }
+    {
+        const float ax = u0 - (float)iu, ay = v0 - (float)iv, bx = 1.0f - ax, by = 1.0f - ay;
+        const float ic = (a.x * bx + b.x * ax) * by + (c.x * bx + d.x * ax) * ay;
+        const float dx = (a.y * bx + b.y * ax) * by + (c.y * bx + d.y * ax) * ay;
+        const float dy = (a.z * bx + b.z * ax) * by + (c.z * bx + d.z * ax) * ay;
+        okr = okr && (dx > 2 || dy > 2) && isfinite(ic) && isfinite(dx) && isfinite(dy);
+        const float lx = (dx * K.fx) * zi, ly = (dy * K.fy) * zi;
+        const float lz = (-(lx * p.x + ly * p.y)) * zi;
+        float res = ic - il;
+        if (pc.normalise) res = div_rn_by(res, pc.stddev, pc.inv);
+        float wt = 1.f;
+        if (fabsf(res) > pc.huber && pc.robust) wt = sqrtf(pc.huber / fabsf(res));
+        const float3 x = cross3(p, make_float3(lx, ly, lz));
+        *rgb_lo = okr ? make_float4(lx * wt, ly * wt, lz * wt, x.x * wt) : zero;
+        *rgb_hi = okr ? make_float4(x.y * wt, x.z * wt, wt * (-res), 1.f) : zero;
+    }
+}
+
+// The products of PART of the eight rows of a chain, summed: the 29 sums of the
+// packed upper triangle by the words they multiply, PART 0 the ten products
+// within row[0..3] (lo) and the six within row[4..6] (hi), PART 1 the twelve
+// across and the count.
+template <int PART>
+__device__ __forceinline__ void chain_sums(const float4 *lo, const float4 *hi, int t, float (&acc)[16]) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) acc[k] = 0.f;
+#pragma unroll
+    for (int i = 0; i < kCtaPixels / kHalfThreads; ++i) {
+        const float4 a = lo[t + i * kHalfThreads], b = hi[t + i * kHalfThreads];
+        const float x[4] = {a.x, a.y, a.z, a.w}, y[3] = {b.x, b.y, b.z};
+        int k = 0;
+        if (PART == 0) {
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+                for (int q = p; q < 4; ++q, ++k) acc[k] = __fmaf_rn(x[p], x[q], acc[k]);
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int q = p; q < 3; ++q, ++k) acc[k] = __fmaf_rn(y[p], y[q], acc[k]);
+        } else {
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+                for (int q = 0; q < 3; ++q, ++k) acc[k] = __fmaf_rn(x[p], y[q], acc[k]);
+            acc[12] += b.w;
+        }
+    }
+}
+// the packed index of sum k of a part (29 and above: none)
+__device__ __forceinline__ int packed_index(int part, int k) {
+    if (part == 0) {
+        const int p = (k >= 4) + (k >= 7) + (k >= 9), q = p + k - (p == 0 ? 0 : p == 1 ? 4 : p == 2 ? 7 : 9);
+        return k < 10 ? 7 * p - p * (p - 1) / 2 + (q - p) : 12 + k;  // then (4,4) (4,5) (4,6) (5,5) (5,6) (6,6): 22 ..
+    }
+    const int p = k / 3, q = 4 + k % 3;
+    return k < 12 ? 7 * p - p * (p - 1) / 2 + (q - p) : k == 12 ? 28 : 32;
+}
+
+// Warp sums of 16 values: after xor 16, 8, 4, 2 a lane holds one of them,
+// completed by xor 1; lane bits 4..1, most significant first, are its index.
+template <int N>
+__device__ __forceinline__ void part_step(float (&v)[16], int lane, int mask) {
+    const bool upper = (lane & mask) != 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const float send = upper ? v[i] : v[i + N];
+        const float keep = upper ? v[i + N] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
+    }
+}
+__device__ __forceinline__ float part_sum(float (&v)[16], int lane) {
+    part_step<8>(v, lane, 16);
+    part_step<4>(v, lane, 8);
+    part_step<2>(v, lane, 4);
+    part_step<1>(v, lane, 2);
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// A CTA of the run waits for another at most this long.  Every CTA is resident
+// and a step takes microseconds: the limit only bounds a wait that cannot happen.
+constexpr long long kTrackWaitNs = 2000000000ll;
+struct WaitLimit {
+    long long t0 = 0;
+    int n = 0;
+    bool ran_out = false;
+    __device__ __forceinline__ bool over() {
+        if (++n & 63) return false;
+        long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (!t0) t0 = t;
+        return ran_out = t - t0 > kTrackWaitNs;
+    }
+};
+
+__device__ __forceinline__ int ld_acquire(const int *p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_release(int *p) {
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+// two words at once from L2; each carries its own number, so they need not arrive together
+__device__ __forceinline__ uint4 ld_l2(const unsigned long long *p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed(unsigned long long *p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// What one CTA of a run hands to another travels as 8-byte words of (value,
+// sequence number): a word that carries its own number needs no fence and no
+// second round trip, and leaves the readers' L1, with the maps they gather from,
+// alone.  CTA 0 publishes 14 of them after each step -- the estimate's 12 floats, the
+// photometric deviation and the work item; the others write the sums of their
+// tile, numbered like the publication that will follow.
+constexpr int kPubWords = 14;
+__device__ __forceinline__ unsigned long long tagged(int number, unsigned value) {
+    return ((unsigned long long)(unsigned)number << 32) | value;
+}
+
+// A run's work items are (level, iteration) packed; 0 is its end.
+__device__ __forceinline__ int first_item(const SessionView &sv, int level) {
+    while (level >= 0 && sv.max_iter[level] == 0) --level;
+    return (level + 1) << 10;
+}
+
+// One tile's sums: word q of record `rec`.
+__device__ __forceinline__ unsigned long long *record_word(const SessionView &sv, int rec, int q) {
+    return sv.track_rec + (size_t)rec * kPartialStride + q;
+}
+
+// The sums of the item numbered `number`, by all threads of CTA 0: warp g waits
+// for records g, g + 16, ... (a lane per record looks at its first word), then
+// lane q adds columns 2 q and 2 q + 1 of them in turn; the 16 groups follow in
+// order (the sums and the order of sum_partials).  The words are read by plain
+// L2 loads, ten in flight, which moved five times the bytes of relaxed ones, and checked by their
+// numbers.  Records past the last count as zeros, which add nothing.
+static_assert(kTrackThreads == 32 * kSumGroups, "a warp per record group");
+__device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv, int n, int number) {
+    const int g = threadIdx.x >> 5, lane = threadIdx.x & 31, q = min(2 * lane, kReduceWidth - 2);
+    WaitLimit limit;
+    FSum s0, s1;
+    constexpr int kBatch = 10, kChunk = 3 * kBatch * kSumGroups;  // at most a record per lane
+    for (int first = g; first < n; first += kChunk) {
+        const int r = first + lane * kSumGroups, end = min(n, first + kChunk);
+        while (!__all_sync(0xffffffffu, r >= end || (int)(ld_relaxed(record_word(sv, r, 0)) >> 32) == number) &&
+               !__any_sync(0xffffffffu, limit.over())) {}
+        for (int c = first; c < end; c += kBatch * kSumGroups) {
+            uint4 w[kBatch];
+            bool all;
+            do {
+                all = true;
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) {
+                    w[i] = make_uint4(0u, (unsigned)number, 0u, (unsigned)number);
+                    if (c + i * kSumGroups < end) w[i] = ld_l2(record_word(sv, c + i * kSumGroups, q));
+                }
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) all = all && (int)w[i].y == number && (int)w[i].w == number;
+            } while (!__all_sync(0xffffffffu, all) && !__any_sync(0xffffffffu, limit.over()));
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                s0.add(__uint_as_float(w[i].x));
+                s1.add(__uint_as_float(w[i].z));
+            }
+        }
+    }
+    sm.grp[g][q] = make_float2(s0.s, s0.c);
+    sm.grp[g][q + 1] = make_float2(s1.s, s1.c);
+    const bool ok = __syncthreads_and(!limit.ran_out);
+    if (threadIdx.x < kReduceWidth) {
+        FSum t;
+#pragma unroll 4
+        for (int h = 0; h < kSumGroups; ++h) {
+            const float2 v = sm.grp[h][threadIdx.x];
+            FSum o;
+            o.s = v.x;
+            o.c = v.y;
+            t.add(o);
+        }
+        sm.total[threadIdx.x] = (double)t.s + (double)t.c;
+    }
+    __syncthreads();
+    return ok;
+}
+
+// The newest publication after number `seen`, by one warp: lanes < 14 get the
+// values.  False when the wait ran out.
+__device__ __forceinline__ bool read_pub(const unsigned long long *pub, int &seen, unsigned &value) {
+    const int lane = threadIdx.x & 31;
+    WaitLimit limit;
+    for (;;) {
+        const unsigned long long w = lane < kPubWords ? ld_relaxed(pub + lane) : 0ull;
+        const int n = (int)(w >> 32), n0 = __shfl_sync(0xffffffffu, n, 0);
+        if (__all_sync(0xffffffffu, lane >= kPubWords || n == n0) && n0 - seen > 0) {
+            seen = n0;
+            value = (unsigned)w;
+            return true;
+        }
+        if (__any_sync(0xffffffffu, lane == 0 && limit.over())) return false;
+    }
+}
+
+// The steps of a run: CTA 0 adds each item's records, takes the step on the
+// tracking state in shared memory and publishes what follows.
+__device__ __forceinline__ void track_steps(TrackSmem &sm, const SessionView &sv, int item, int seen, bool lost,
+                                            int frame_mode) {
+    TrackState *ts = &sm.ts;
+    const int tid = threadIdx.x, lane = tid & 31;
+    unsigned long long *pub = reinterpret_cast<unsigned long long *>(sv.ctr + C_TRACK_PUB);
+    while (item > 0 && !lost) {
+        const int level = (item >> 10) - 1, iter = item & 1023;
+        lost = !sum_records(sm, sv, sv.red_ctas[level], ++seen);
+        if (lost) break;
+        if (tid >= 64 && tid < 64 + kReduceWidth) ts->last_sums[tid - 64] = sm.total[tid - 64];
+        if (tid < 64) gn_epilogue(sv, ts, level, iter, sm.total);
+        __syncthreads();
+        item = ts->level_done || iter + 1 >= sv.max_iter[level] ? first_item(sv, level - 1) : item + 1;
+        if (tid < kPubWords) {
+            const float dev = level == (item >> 10) - 1 ? ts->stddev : 0.f;  // each level starts without one
+            const float x = lane < 12 ? (float)ts->est[lane] : dev;
+            st_relaxed(pub + lane, tagged(seen, lane < 13 ? __float_as_uint(x) : (unsigned)item));
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    if (tid < 32) {
+        if (lost) ts->invalid = 1;  // a wait ran out: the frame counts as not tracked
+        __syncwarp();
+        track_finish(sv, ts, frame_mode);
+    }
+    __syncthreads();
+    for (int i = tid; i < (int)(sizeof(TrackState) / 4); i += kTrackThreads)
+        reinterpret_cast<int *>(sv.ts)[i] = reinterpret_cast<const int *>(ts)[i];
+    if (tid == 0) sv.ctr[C_TICKET] = 0;
+}
+
+// The tiles of a run: CTA cta of the ctas that follow CTA 0 makes its tiles' records of each item.
+__device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv, int item, int seen, int rs, int cta,
+                                            int ctas) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned long long *pub = reinterpret_cast<const unsigned long long *>(sv.ctr + C_TRACK_PUB);
+    const float qnan = __int_as_float(0x7fffffff);
+    const float4 nan4 = make_float4(qnan, qnan, qnan, -1.f);
+    float4 v[kTrackPixels], m[kTrackPixels];  // this thread's reference pixels of the CTA's next tile
+    float il[kTrackPixels];
+    int loaded = -1;  // the level they belong to
+    while (item > 0) {
+        const int level = (item >> 10) - 1;
+        const LevelIn in = level_in(sv, level, 1 - rs);
+        const int tiles = sv.red_ctas[level], P = in.w * in.h;
+        const float4 *gv = sv.vmap[rs][level], *gn = sv.nmap[rs][level];
+        const float *gi = sv.inten[rs][level];
+        const auto load = [&](int tile) {
+#pragma unroll
+            for (int j = 0; j < kTrackPixels; ++j) {
+                const int c = tile * kCtaPixels + tid + j * kTrackThreads;
+                v[j] = m[j] = nan4;
+                il[j] = qnan;
+                if (c < P) {
+                    v[j] = gv[c];
+                    m[j] = gn[c];
+                    il[j] = gi[c];
+                }
+            }
+        };
+        if (cta < tiles) {
+            if (loaded != level) load(cta);
+            loaded = level;
+            M34 T;
+#pragma unroll
+            for (int i = 0; i < 12; ++i) T.m[i] = sm.pose[i];
+            const PhotoConst pc = photo_const(sm.stddev, sm.huber);
+            for (int tile = cta; tile < tiles; tile += ctas) {
+#pragma unroll
+                for (int j = 0; j < kTrackPixels; ++j) {
+                    const int k = tid + j * kTrackThreads;
+                    pixel_rows(in, T, pc, v[j], m[j], il[j], sm.lo[0] + k, sm.hi[0] + k, sm.lo[1] + k, sm.hi[1] + k);
+                }
+                // meanwhile the next tile's pixels, or the first one's again for the next iteration
+                load(tile + ctas < tiles ? tile + ctas : cta);
+                __syncwarp();
+                __syncthreads();
+                {
+                    // a warp per half (ICP, photometric), part of the products and chain warp
+                    const int half = warp & 1, part = (warp >> 1) & 1, cw = warp >> 2;
+                    float acc[16];
+                    if (part == 0) chain_sums<0>(sm.lo[half], sm.hi[half], 32 * cw + lane, acc);
+                    else chain_sums<1>(sm.lo[half], sm.hi[half], 32 * cw + lane, acc);
+                    const float s = part_sum(acc, lane);
+                    const int k = packed_index(part, lane >> 1);
+                    if (!(lane & 1) && k < 29) sm.warp_sums[cw][half * 29 + k] = s;
+                }
+                __syncwarp();
+                __syncthreads();
+                if (tid < kReduceWidth) {
+                    float s = 0.f;
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) s += sm.warp_sums[w][tid];
+                    st_relaxed(record_word(sv, tile, tid), tagged(seen + 1, __float_as_uint(s)));
+                }
+            }
+        }
+        if (warp == 0) {
+            unsigned value = 0;
+            const bool ok = read_pub(pub, seen, value);
+            if (lane < 12) sm.pose[lane] = __uint_as_float(value);
+            if (lane == 12) {
+                sm.stddev = __uint_as_float(value);
+                sm.huber = photo_huber(sm.stddev);
+            }
+            if (lane == 13) {
+                sm.item = ok ? (int)value : -1;
+                sm.seen = seen;
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        item = sm.item;
+        seen = sm.seen;
+    }
+}
+
+__global__ void __launch_bounds__(kTrackThreads, 1)
+    gn_track_kernel(const SessionView *__restrict__ svs, int frame_mode) {
+    extern __shared__ __align__(16) unsigned char track_smem[];
+    TrackSmem &sm = *reinterpret_cast<TrackSmem *>(track_smem);
+    const SessionView &sv = svs[blockIdx.y];
+    if (!sv.active) return;
+    const int tid = threadIdx.x;
+    const bool head = blockIdx.x == 0;
+    // Every CTA reads these before it arrives, and CTA 0 goes on once all have:
+    // what it publishes, and the frame's end, change them.
+    const int rs = sv.ts->idx;
+    const int seen = (int)(ld_relaxed(reinterpret_cast<const unsigned long long *>(sv.ctr + C_TRACK_PUB)) >> 32);
+    const int item = frame_mode && !sv.ts->has_ref ? 0 : first_item(sv, sv.levels - 1);
+    if (tid < 12) sm.pose[tid] = (float)sv.ts->init[tid];
+    if (tid == 12) sm.stddev = sm.huber = 0.f;
+    if (head)
+        for (int i = tid; i < (int)(sizeof(TrackState) / 4); i += kTrackThreads)
+            reinterpret_cast<int *>(&sm.ts)[i] = reinterpret_cast<const int *>(sv.ts)[i];
+    __syncwarp();
+    __syncthreads();
+    if (!head) {
+        if (tid == 0) red_release(sv.ctr + C_TICKET);
+        __syncwarp();
+        track_tiles(sm, sv, item, seen, rs, blockIdx.x - 1, gridDim.x - 1);
+        return;
+    }
+    if (tid == 0) {
+        track_begin(&sm.ts, frame_mode);
+        WaitLimit limit;
+        while (ld_acquire(sv.ctr + C_TICKET) != (int)gridDim.x - 1 && !limit.over()) {}
+        sm.lost = ld_acquire(sv.ctr + C_TICKET) != (int)gridDim.x - 1;
+    }
+    __syncwarp();
+    __syncthreads();
+    track_steps(sm, sv, item, seen, sm.lost, frame_mode);
+}
+
 }  // namespace
 
 // Sessions whose Gauss-Newton iterations run back to back before the next
@@ -743,7 +1187,43 @@ constexpr int kTrackSubgroup = 64;
 constexpr int kDeferStepSessions = 32;
 static bool defer_step(int sessions) { return sessions >= kDeferStepSessions; }
 
-int track_launches(int nslots, const Extent &ex) {
+// Sessions up to which a launch that has the chip to itself takes the tracking
+// run in one cooperative kernel: track 0.25 -> 0.16 ms for one 640x480 session,
+// 0.28 -> 0.19 for two, 0.34 -> 0.26 for three, 0.39 -> 0.33 for four.  With more
+// the CTAs are busy with their tiles most of the time, and what is left to gain
+// (0.49 -> 0.43 ms for six) is less than concurrent groups give.
+constexpr int kTrackRunSessions = 4;
+int track_run_sessions() { return kTrackRunSessions; }
+
+// CTAs of one cooperative launch of gn_track_kernel on the current device (one
+// per SM), or 0 where it cannot be launched.
+static int track_run_ctas() {
+    static std::atomic<int> known[64];  // per device: CTAs + 1
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::atomic<int> &k = known[dev & 63];
+    int c = k.load(std::memory_order_acquire);
+    if (c == 0) {
+        int sms = 0, coop = 0, per = 0;
+        c = 1;
+        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+            cudaFuncSetAttribute(gn_track_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(TrackSmem)) ==
+                cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, gn_track_kernel, kTrackThreads, sizeof(TrackSmem)) ==
+                cudaSuccess)
+            c = sms * per + 1;
+        k.store(c, std::memory_order_release);
+    }
+    return c - 1;
+}
+
+static bool takes_run(int nslots, bool alone) {
+    return alone && nslots <= kTrackRunSessions && track_run_ctas() >= 2 * nslots;
+}
+
+int track_launches(int nslots, const Extent &ex, bool alone) {
+    if (takes_run(nslots, alone)) return 1;
     int it = 0;
     for (int l = 0; l < ex.levels; ++l) it += ex.max_iter[l];
     int n = 0;
@@ -752,7 +1232,15 @@ int track_launches(int nslots, const Extent &ex) {
     return 2 + n;
 }
 
-void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, cudaStream_t st) {
+void prepare_track() { track_run_ctas(); }
+
+void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, bool alone, cudaStream_t st) {
+    if (takes_run(nslots, alone)) {
+        void *args[] = {(void *)&d_sv, (void *)&frame_mode};
+        cudaLaunchCooperativeKernel((const void *)gn_track_kernel, dim3(track_run_ctas() / nslots, nslots),
+                                    dim3(kTrackThreads), args, sizeof(TrackSmem), st);
+        return;
+    }
     track_begin_kernel<<<nslots, 32, 0, st>>>(d_sv, frame_mode);
     ReduceArgs a{};
     a.once = 0;

@@ -754,3 +754,91 @@ def test_prune_between_graph_ticks_matches_session_alone(gbf):
             assert np.array_equal(x, y), i
     b.close()
     assert n_before > 0
+
+
+@pytest.mark.parametrize("w,h,levels,iters,prior", [
+    (64, 64, 2, [10, 5], 0),              # four tiles, most CTAs without one
+    (96, 64, 1, [3], 0),                  # a last tile that ends ragged
+    (328, 248, 3, [10, 5, 3], 1),         # tiles that are no multiple of the CTAs
+    (640, 480, 3, [4, 0, 3], 0),          # a level without iterations
+    (640, 480, 2, [0, 0], 0),             # no iteration at all
+    (1280, 720, 4, [10, 5, 3, 3], 0),     # several tiles per CTA
+])
+def test_tracking_run_matches_launches_per_iteration(gbf, w, h, levels, iters, prior):
+    """A session alone tracks in one cooperative launch (gn_track_kernel); a session
+    of a batch in two branches in a launch per iteration.  Same poses, outcomes
+    and work counters, bit for bit."""
+    import torch
+    L = gbf
+    K = H.intrinsics(L, w, h)
+    cfg = H.small_config(L, 2, num_levels=levels, max_iterations=iters + [0] * (5 - len(iters)), motion_prior=prior,
+                         num_blocks=1 << 14, num_buckets=1 << 16)
+    nf = 5
+    fr = H.frames(L, K, nf, seed=4)
+    one, a, b = (L.System(K, cfg) for _ in range(3))
+    batch = L.FusionBatch(2)
+    batch.set_groups(2)
+    for i, s in enumerate((a, b)):
+        batch.set(i, s)
+    for s in (one, a, b):
+        s.set_pose(fr[0][2])
+    for d, c, _ in fr:
+        d, c = H.cuda(d), H.cuda(c)
+        one.process_images(d, c)
+        for s in (a, b):
+            s.stage(d, c)
+        torch.cuda.synchronize()
+        batch.process([True, True])
+        torch.cuda.synchronize()
+        x, y = one.stats(), a.stats()
+        assert np.array_equal(one.get_camera_pose(), a.get_camera_pose())
+        assert np.array_equal(one.get_camera_pose(), b.get_camera_pose())
+        assert list(x.level_iterations) == list(y.level_iterations) and x.pixel_iterations == y.pixel_iterations
+        assert (x.status, x.track.success, x.track.iterations) == (y.status, y.track.success, y.track.iterations)
+        for f in ("icp_error", "rgb_error", "icp_inliers", "rgb_inliers"):
+            assert getattr(x.track, f) == getattr(y.track, f) or np.isnan(getattr(x.track, f))
+    batch.close()
+
+
+def test_tracking_runs_on_concurrent_streams(gbf):
+    """Sessions driven on streams of their own, nothing waiting between them: their
+    cooperative tracking runs, each of which takes the whole chip, beside each
+    other and beside a batch's ticks give the poses that each session has alone."""
+    import torch
+    L = gbf
+    K = H.intrinsics(L, 320, 240)
+    cfg = H.small_config(L, 1, num_blocks=1 << 14, num_buckets=1 << 16)
+    nf, n = 8, 4
+    fr = [[(H.cuda(d), H.cuda(c), T) for d, c, T in H.frames(L, K, nf, seed=i)] for i in range(n)]
+
+    def make():
+        ss = [L.System(K, cfg) for _ in range(n)]
+        for i, s in enumerate(ss):
+            s.set_pose(fr[i][0][2])
+        return ss
+    alone = []
+    for i, s in enumerate(make()):
+        for d, c, _ in fr[i]:
+            s.process_images(d, c)
+            torch.cuda.synchronize()
+        alone.append(s.get_camera_pose())
+    ss, streams = make(), [torch.cuda.Stream() for _ in range(n)]
+    more = make()
+    batch = L.FusionBatch(n)
+    for i, s in enumerate(more):
+        batch.set(i, s)
+    batch.set_groups(2)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for k in range(nf):
+        for i in range(n):
+            batch.set_inputs(i, fr[i][k][0].data_ptr(), fr[i][k][1].data_ptr())
+        batch.process([True] * n, stream=side)
+        for i in range(n):
+            ss[i].process_images(fr[i][k][0], fr[i][k][1], stream=streams[i])
+    torch.cuda.synchronize()
+    for i in range(n):
+        assert np.array_equal(ss[i].get_camera_pose(), alone[i]), i
+        assert np.array_equal(more[i].get_camera_pose(), alone[i]), i
+        assert ss[i].stats().status == 0 and more[i].stats().status == 0
+    batch.close()
