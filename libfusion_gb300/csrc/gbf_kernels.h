@@ -90,8 +90,8 @@ void launch_frame_finish(const SessionView *d_sv, int nslots, cudaStream_t st);
 void launch_slot_results(const SessionView *d_sv, int nslots, gbf_slot_result *out, cudaStream_t st);
 
 // ---- meshing (mesh.cu) ------------------------------------------------------------
-// returns via device counters; the host reads C_MESH_TRIS
+// returns via device counters; the host reads C_MESH_TRIS.  counts, chunk_sums: the session's mesh_off and mesh_sums
 void launch_mesh(const SessionView *d_sv, const Extent &ex, int layout, int mode, float *vtx, void *attr,
-                 long long max_tris, int *counts, cudaStream_t st);
+                 long long max_tris, int *counts, int *chunk_sums, cudaStream_t st);
 
 }  // namespace gbf

@@ -1,18 +1,28 @@
 // mesh.cu -- marching cubes over all allocated blocks (src/voxel_hashing/
 // scene_mesh.cu:14-643, tables include/voxel_hashing/device_tables.h).
 //
-// GB300 design: two passes over the allocated-block list (ids 0..n-1 of the
-// pool; the reference instead compacts the whole hash table, scene_mesh.cu:24-52).
-//   count  one CTA (512 threads, one per voxel) per block stages the block and
-//          its +x/+y/+z halo (9x9x9 sdf + validity) in shared memory with 7
-//          neighbour lookups, classifies every voxel's cube and sums the
-//          block's triangles.
-//   scan   exclusive prefix of the per-block counts (one CTA).
-//   emit   restages, takes the in-block prefix of the voxels' triangle counts
-//          and writes every triangle at a fixed position.
+// GB300 design: passes over the allocated-block list (ids 0..n-1 of the pool;
+// the reference instead compacts the whole hash table, scene_mesh.cu:24-52).
+//   count  one 128-thread CTA per block: the signs and the validity of the block
+//          and its +x/+y/+z halo as bit rows (7 neighbour lookups, ballots), every
+//          row's eight cubes classified from four bit rows, the block's triangles
+//          summed, and those of its chunk of blocks.
+//   scan   offsets of the blocks, a CTA per chunk on top of the chunks before it.
+//   emit   restages with the values, lists the block's triangles in voxel order in
+//          shared memory, then a lane per vertex: ten triangles per warp at a time,
+//          written through shared memory as whole rows of floats.
 // Output order is deterministic (block id, voxel index, table order); the
 // reference appends with one global atomicAdd per triangle (scene_mesh.cu:231).
 // Vertex arithmetic follows make_vertex (scene_mesh.cu:119-209) exactly.
+//
+// What bounds it: latency and issue, not memory (48,000 blocks of a scanned room
+// read 98 MB of voxels and write 310 MB of triangles: 60 us at the measured
+// bandwidth).  A 512-thread CTA per block with a thread per voxel held four
+// blocks per SM through two dependent lookups, and interpolated twelve edges per
+// voxel for all lanes of a warp, with the reference's thresholds in double: 36
+// FP64 comparisons of 64 cycles each.  They are the same tests on floats (below).
+// 48,000 blocks, 4.1 M triangles with normals: 2,513 -> 541 us a call (count 0.50 ->
+// 0.11 ms, scan 50 -> 5 us, emit 1.9 -> 0.36 ms).
 #include "gbf_device.cuh"
 #include "gbf_kernels.h"
 
@@ -23,8 +33,10 @@ namespace {
 // Triangle table of classic marching cubes (the public-domain Lorensen-Cline /
 // Bourke table, identical to the reference's triangle_table so that the mesh
 // topology matches bit for bit).  Packed: low nibble = number of triangles,
-// then one nibble per edge index, three per triangle, in table order.
-__constant__ unsigned long long kTriPacked[256] = {
+// then one nibble per edge index, three per triangle, in table order.  In global
+// memory: the lanes of a warp look up different cubes, which the constant bank
+// would serve one after the other.
+__device__ const unsigned long long kTriPacked[256] = {
     0x0000000000000000ull, 0x0000000000003801ull, 0x0000000000009101ull, 0x0000000001893812ull,
     0x000000000000a211ull, 0x000000000a213802ull, 0x000000000920a292ull, 0x00000089a8a23823ull,
     0x0000000000002b31ull, 0x0000000000b82b02ull, 0x000000000b320912ull, 0x000000b89b912b13ull,
@@ -91,273 +103,371 @@ __constant__ unsigned long long kTriPacked[256] = {
     0x0000000008198312ull, 0x0000000000001901ull, 0x0000000000008301ull, 0x0000000000000000ull,
 };
 
-// Cube corners in make_vertex order (scene_mesh.cu:73-101) and the corner
-// pair of each of the 12 edges (scene_mesh.cu:147-205).
-__constant__ int kCorner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
-                                  {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
-__constant__ int kEdge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6},
-                                 {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
-
 constexpr int kHaloSide = 9;
 constexpr int kHaloCells = kHaloSide * kHaloSide * kHaloSide;
+constexpr int kHaloRows = kHaloSide * kHaloSide;
+constexpr int kHaloExtra = kHaloCells - kBlockVoxels;  // 217 cells of the neighbours
+constexpr int kMeshThreads = 128;
+constexpr int kMeshMaxTris = kBlockVoxels * 5;
 
-struct MeshSmem {
-    float sdf[kHaloCells];
-    unsigned char ok[kHaloCells];
-    unsigned char rgb[kHaloCells][3];
+// Signs and validity of a block and its halo: row z * 9 + y has x = 0..7 in the
+// low byte and x = 8 in `end`.
+struct MeshBits {
+    unsigned char ok[kHaloRows], ok_end[kHaloRows], neg[kHaloRows], neg_end[kHaloRows];
     int nb[8];
-    int tri[kBlockVoxels];
-    int warp_tot[kBlockVoxels / 32];
 };
 
-__device__ __forceinline__ int edge_mask(int ci) {
-    int m = 0;
-#pragma unroll
-    for (int e = 0; e < 12; ++e) {
-        const int a = (ci >> kEdge[e][0]) & 1, b = (ci >> kEdge[e][1]) & 1;
-        if (a != b) m |= 1 << e;
+// Halo cell i < 217: the +x, +y and +z faces (64 each), the edges (8, 8, z), (8, y, 8), (x, 8, 8), the corner.
+__device__ __forceinline__ void halo_cell(int i, int &x, int &y, int &z) {
+    const int a = i & 7, b = (i >> 3) & 7;
+    x = i < 64 ? 8 : a;
+    y = i < 64 ? a : i < 128 ? 8 : b;
+    z = i < 128 ? b : 8;
+    if (i >= 192) {
+        const int e = i - 192;
+        x = e < 16 ? 8 : e < 24 ? a : 8;
+        y = e < 8 || e >= 16 ? 8 : a;
+        z = e < 8 ? a : 8;
     }
-    return m;
 }
 
-// Stage block `id` plus its +x/+y/+z halo; validity per the mesh mode:
-// weight != 0 (scene_mesh.cu:58) or weight > 1e-3 for colour (scene_mesh.cu:397).
+// The sdf of a voxel and whether it counts: weight != 0 (scene_mesh.cu:58), or weight > 1e-3 for colour
+// (scene_mesh.cu:397; of the floats, those from 1e-3f, which lies just above 1e-3).
 template <int LAYOUT>
-__device__ void stage_block(const SessionView &sv, int id, int mode, MeshSmem &sm) {
-    const int4 bc = sv.bcoord[id];
-    if (threadIdx.x < 8) {
-        const int dx = threadIdx.x & 1, dy = (threadIdx.x >> 1) & 1, dz = (threadIdx.x >> 2) & 1;
-        sm.nb[threadIdx.x] = (threadIdx.x == 0) ? id : find_block(sv, bc.x + dx, bc.y + dy, bc.z + dz);
+__device__ __forceinline__ float mesh_sdf(const SessionView &sv, int id, int x, int y, int z, int mode, bool &ok, int &vi) {
+    ok = false;
+    vi = 0;
+    if (id < 0) return 0.f;
+    vi = id * kBlockVoxels + (z & 7) * 64 + (y & 7) * 8 + (x & 7);
+    float w;
+    const float s = load_sdf<LAYOUT>(sv, (size_t)vi, w);
+    ok = mode == GBF_MESH_COLOUR ? w >= 1e-3f : w != 0.f;
+    return s;
+}
+
+// Block `id` and its halo into the bit rows, and with VALUES the sdf (and for
+// colour the colours) of every cell.  All threads; barriers at both ends.
+template <int LAYOUT, bool VALUES>
+__device__ __forceinline__ void stage_block(const SessionView &sv, int id, int mode, MeshBits &m, float *sdf,
+                                            uchar4 *rgb) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    __syncthreads();  // the previous block's use of the shared arrays
+    if (tid < 8) {
+        const int4 bc = sv.bcoord[id];
+        m.nb[tid] = tid == 0 ? id : find_block(sv, bc.x + (tid & 1), bc.y + ((tid >> 1) & 1), bc.z + (tid >> 2));
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < kHaloCells; c += blockDim.x) {
-        const int x = c % kHaloSide, y = (c / kHaloSide) % kHaloSide, z = c / (kHaloSide * kHaloSide);
-        const int nbi = (x >> 3) | ((y >> 3) << 1) | ((z >> 3) << 2);
-        const int nid = sm.nb[nbi];
-        bool ok = false;
-        float s = 0.f;
-        uchar4 col = make_uchar4(0, 0, 0, 0);
-        if (nid >= 0) {
-            const size_t vi = (size_t)nid * kBlockVoxels + (z & 7) * 64 + (y & 7) * 8 + (x & 7);
-            float w;
-            s = load_sdf<LAYOUT>(sv, vi, w);
-            ok = (mode == GBF_MESH_COLOUR) ? ((double)w > 1e-3) : (w != 0.f);
-            if (mode == GBF_MESH_COLOUR) col = sv.vox_rgb[vi];
+    __syncwarp();
+    // the block itself: its loads go out beside the lookups
+#pragma unroll
+    for (int j = 0; j < kBlockVoxels / kMeshThreads; ++j) {
+        const int li = tid + j * kMeshThreads, x = li & 7, y = (li >> 3) & 7, z = li >> 6;
+        bool ok;
+        int vi;
+        const float s = mesh_sdf<LAYOUT>(sv, id, x, y, z, mode, ok, vi);
+        const unsigned oks = __ballot_sync(0xffffffffu, ok), negs = __ballot_sync(0xffffffffu, s < 0);
+        if (x == 0) {  // a warp covers four rows
+            m.ok[z * 9 + y] = (unsigned char)(oks >> lane);
+            m.neg[z * 9 + y] = (unsigned char)(negs >> lane);
         }
-        sm.sdf[c] = s;
-        sm.ok[c] = ok;
-        sm.rgb[c][0] = col.x; sm.rgb[c][1] = col.y; sm.rgb[c][2] = col.z;
+        if (VALUES) {
+            const int c = x + 9 * y + 81 * z;
+            sdf[c] = s;
+            if (mode == GBF_MESH_COLOUR) rgb[c] = sv.vox_rgb[vi];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = tid + j * kMeshThreads;
+        const bool in = i < kHaloExtra;
+        int x, y, z;
+        halo_cell(min(i, kHaloExtra - 1), x, y, z);
+        bool ok = false;
+        int vi = 0, id2 = -1;
+        float s = 0.f;
+        if (in) {
+            id2 = m.nb[(x >> 3) | ((y >> 3) << 1) | ((z >> 3) << 2)];
+            s = mesh_sdf<LAYOUT>(sv, id2, x, y, z, mode, ok, vi);
+        }
+        const unsigned oks = __ballot_sync(0xffffffffu, ok), negs = __ballot_sync(0xffffffffu, s < 0);
+        if (in) {
+            const int row = z * 9 + y;
+            if (x == 8) {
+                m.ok_end[row] = ok;
+                m.neg_end[row] = s < 0;
+            } else if (x == 0) {  // the faces' rows of eight lie in lanes of a multiple of eight
+                m.ok[row] = (unsigned char)(oks >> lane);
+                m.neg[row] = (unsigned char)(negs >> lane);
+            }
+            if (VALUES) {
+                const int c = x + 9 * y + 81 * z;
+                sdf[c] = s;
+                if (mode == GBF_MESH_COLOUR) rgb[c] = id2 >= 0 ? sv.vox_rgb[vi] : make_uchar4(0, 0, 0, 0);
+            }
+        }
     }
     __syncthreads();
 }
 
-__device__ __forceinline__ int cube_of(const MeshSmem &sm, int li, float s[8], int corner_cell[8]) {
-    const int x = li & 7, y = (li >> 3) & 7, z = li >> 6;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int c = (x + kCorner[k][0]) + (y + kCorner[k][1]) * kHaloSide + (z + kCorner[k][2]) * kHaloSide * kHaloSide;
-        corner_cell[k] = c;
-        if (!sm.ok[c]) return -1;
-        s[k] = sm.sdf[c];
+// The cubes of voxel row r = 8 z + y (a thread each of the first 64): which of the
+// eight have all their corners, and the four rows of signs that make them up.
+struct CubeRow {
+    unsigned valid, n00, n10, n01, n11;
+    // corner order of make_vertex (scene_mesh.cu:73-101): (0,0) (1,0) (1,1) (0,1) below, then above
+    __device__ __forceinline__ int cube(int x) const {
+        const unsigned a = n00 >> x, b = n10 >> x, c = n01 >> x, d = n11 >> x;
+        return (int)((a & 3u) | ((b & 2u) << 1) | ((b & 1u) << 3) | ((c & 3u) << 4) | ((d & 2u) << 5) | ((d & 1u) << 7));
     }
-    int ci = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-        if (s[k] < 0) ci |= 1 << k;
-    return ci;
+};
+__device__ __forceinline__ CubeRow cube_row(const MeshBits &m, int r) {
+    const int q = (r >> 3) * 9 + (r & 7);
+    auto bits = [](const unsigned char *lo, const unsigned char *end, int i) { return (unsigned)lo[i] | ((unsigned)end[i] << 8); };
+    CubeRow c;
+    const unsigned ok = bits(m.ok, m.ok_end, q) & bits(m.ok, m.ok_end, q + 1) & bits(m.ok, m.ok_end, q + 9) &
+                        bits(m.ok, m.ok_end, q + 10);
+    c.valid = ok & (ok >> 1) & 0xffu;
+    c.n00 = bits(m.neg, m.neg_end, q);
+    c.n10 = bits(m.neg, m.neg_end, q + 1);
+    c.n01 = bits(m.neg, m.neg_end, q + 9);
+    c.n11 = bits(m.neg, m.neg_end, q + 10);
+    // cubes with all corners on one side have no triangles
+    const unsigned any = c.n00 | c.n10 | c.n01 | c.n11, all = c.n00 & c.n10 & c.n01 & c.n11;
+    c.valid &= (any | (any >> 1)) & ~(all & (all >> 1));
+    return c;
+}
+
+// Blocks per chunk of the offset scan (at most kMeshChunks chunks).
+__host__ __device__ __forceinline__ int mesh_chunk(int pool) {
+    const int c = (pool + kMeshChunks - 1) / kMeshChunks;
+    return c <= 1024 ? 1024 : (c + 1023) / 1024 * 1024;
 }
 
 template <int LAYOUT>
-__global__ void __launch_bounds__(kBlockVoxels) mesh_count_kernel(const SessionView *__restrict__ svs, int mode, int *counts) {
+__global__ void __launch_bounds__(kMeshThreads, 16) mesh_count_kernel(const SessionView *__restrict__ svs, int mode, int *counts) {
     const SessionView &sv = svs[0];
-    const int n = min(sv.ctr[C_NUSED], sv.pool);
-    __shared__ MeshSmem sm;
+    const int n = min(sv.ctr[C_NUSED], sv.pool), chunk = mesh_chunk(sv.pool);
+    __shared__ MeshBits m;
+    __shared__ unsigned char tris[256];
+    __shared__ int part[2];
+    for (int i = threadIdx.x; i < 256; i += kMeshThreads) tris[i] = (unsigned char)(kTriPacked[i] & 0xf);
     for (int b = blockIdx.x; b < n; b += gridDim.x) {
-        stage_block<LAYOUT>(sv, b, mode, sm);
-        float s[8];
-        int cc[8];
-        const int ci = cube_of(sm, threadIdx.x, s, cc);
-        int t = 0;
-        if (ci > 0 && edge_mask(ci) != 0) t = (int)(kTriPacked[ci] & 0xF);
-        // block sum
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) t += __shfl_down_sync(0xffffffffu, t, off);
-        if ((threadIdx.x & 31) == 0) sm.warp_tot[threadIdx.x >> 5] = t;
+        stage_block<LAYOUT, false>(sv, b, mode, m, nullptr, nullptr);
+        if (threadIdx.x < 64) {
+            const CubeRow row = cube_row(m, threadIdx.x);
+            int t = 0;
+            for (unsigned v = row.valid; v; v &= v - 1) t += tris[row.cube(__ffs(v) - 1)];
+            __syncwarp();
+            t = __reduce_add_sync(0xffffffffu, t);
+            if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = t;
+        }
         __syncthreads();
         if (threadIdx.x == 0) {
-            int tot = 0;
-            for (int w = 0; w < kBlockVoxels / 32; ++w) tot += sm.warp_tot[w];
-            counts[b] = tot;
+            const int total = part[0] + part[1];
+            counts[b] = total;
+            if (total) atomicAdd(sv.mesh_sums + b / chunk, total);
         }
-        __syncthreads();
     }
 }
 
-// exclusive scan of counts[0..n) in place, total into C_MESH_TRIS (one CTA)
-__global__ void mesh_scan_kernel(const SessionView *__restrict__ svs, int *counts) {
+// Exclusive scan of counts[0..n) in place, the total into counts[n] and
+// C_MESH_TRIS.  A CTA per chunk: the sums of the chunks before it, then its own
+// counts, 1024 at a time.  (One CTA over all the blocks took 6.3 us for 6,000.)
+__global__ void __launch_bounds__(1024) mesh_scan_kernel(const SessionView *__restrict__ svs, int *counts) {
     const SessionView &sv = svs[0];
-    const int n = min(sv.ctr[C_NUSED], sv.pool);
-    __shared__ long long carry;
+    const int n = min(sv.ctr[C_NUSED], sv.pool), chunk = mesh_chunk(sv.pool);
+    const int first = blockIdx.x * chunk, end = min(n, first + chunk);
+    if (first >= n && blockIdx.x > 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     __shared__ int wsum[32];
-    if (threadIdx.x == 0) carry = 0;
+    __shared__ int carry;
+    const int *sums = sv.mesh_sums;
+    int before = tid < (int)blockIdx.x ? sums[tid] : 0;
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) wsum[warp] = before;
     __syncthreads();
-    for (int base = 0; base < n; base += blockDim.x) {
-        const int i = base + threadIdx.x;
-        const int v = (i < n) ? counts[i] : 0;
-        // inclusive warp scan
-        int x = v;
+    if (warp == 0) {
+        const int t = __reduce_add_sync(0xffffffffu, wsum[lane]);
+        if (lane == 0) carry = t;
+    }
+    __syncthreads();
+    for (int base = first; base < end; base += 1024) {
+        const int i = base + tid, v = i < end ? counts[i] : 0;
+        int x = v;  // inclusive warp scan
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, x, off);
-            if ((threadIdx.x & 31) >= off) x += y;
+            if (lane >= off) x += y;
         }
-        if ((threadIdx.x & 31) == 31) wsum[threadIdx.x >> 5] = x;
+        if (lane == 31) wsum[warp] = x;
         __syncthreads();
-        if (threadIdx.x < 32) {
-            int w = (threadIdx.x < (int)(blockDim.x >> 5)) ? wsum[threadIdx.x] : 0;
+        int w = wsum[lane];
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, w, off);
-                if (threadIdx.x >= off) w += y;
-            }
-            wsum[threadIdx.x] = w;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, w, off);
+            if (lane >= off) w += y;
         }
+        const int c = carry, total = __shfl_sync(0xffffffffu, w, 31);
+        const int prior = __shfl_sync(0xffffffffu, w, warp ? warp - 1 : 0);
+        if (i < end) counts[i] = c + (warp ? prior : 0) + (x - v);
         __syncthreads();
-        const int wid = threadIdx.x >> 5;
-        const long long excl = carry + (wid ? wsum[wid - 1] : 0) + (x - v);
-        if (i < n) counts[i] = (int)excl;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += wsum[(blockDim.x >> 5) - 1];
+        if (tid == 0) carry = c + total;
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        counts[n] = (int)carry;
-        sv.ctr[C_MESH_TRIS] = (int)carry;
+    if (tid == 0 && end >= n) {
+        counts[n] = carry;
+        sv.ctr[C_MESH_TRIS] = carry;
+    }
+}
+
+// interpolate_sdf (scene_mesh.cu:108-117).  The reference's thresholds compare in
+// double against 1e-6; of the floats, 1e-6f is the largest below it.
+__device__ __forceinline__ float edge_point(float v1, float v2) {
+    if (fabsf(0 - v1) <= 1e-6f) return 0.f;
+    if (fabsf(0 - v2) <= 1e-6f) return 1.f;
+    if (fabsf(v1 - v2) <= 1e-6f) return 0.f;
+    return (0 - v1) / (v2 - v1);
+}
+
+struct MeshEmit {
+    MeshBits bits;
+    float sdf[kHaloCells];
+    unsigned short tri[kMeshMaxTris];  // voxel | triangle of its cube << 9
+    unsigned char cube[kBlockVoxels];
+    int part[2];
+    float out[kMeshThreads / 32][2][90];  // a warp's ten triangles: vertices, normals
+};
+
+template <int LAYOUT, int MODE>
+__global__ void __launch_bounds__(kMeshThreads, 10) mesh_emit_kernel(const SessionView *__restrict__ svs, const int *offsets,
+                                                                     float *vtx, void *attr, long long max_tris) {
+    const SessionView &sv = svs[0];
+    const int n = min(sv.ctr[C_NUSED], sv.pool);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ MeshEmit sm;
+    __shared__ uchar4 rgb[MODE == GBF_MESH_COLOUR ? kHaloCells : 1];
+    for (int b = blockIdx.x; b < n; b += gridDim.x) {
+        const int first = offsets[b];
+        const int count = (int)min((long long)(offsets[b + 1] - first), max_tris - first);
+        if (count <= 0) continue;  // uniform per CTA
+        stage_block<LAYOUT, true>(sv, b, MODE, sm.bits, sm.sdf, rgb);
+        // the block's triangles in voxel order
+        CubeRow row;
+        int t = 0, x = 0;
+        if (tid < 64) {
+            row = cube_row(sm.bits, tid);
+            for (unsigned v = row.valid; v; v &= v - 1) {
+                const int at = __ffs(v) - 1, ci = row.cube(at);
+                sm.cube[tid * 8 + at] = (unsigned char)ci;
+                t += (int)(kTriPacked[ci] & 0xf);
+            }
+            __syncwarp();
+            x = t;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, off);
+                if (lane >= off) x += y;
+            }
+            if (lane == 31) sm.part[warp] = x;
+        }
+        __syncthreads();
+        if (tid < 64) {
+            int at = x - t + (warp ? sm.part[0] : 0);
+            for (unsigned v = row.valid; v; v &= v - 1) {
+                const int li = tid * 8 + __ffs(v) - 1, k = (int)(kTriPacked[sm.cube[li]] & 0xf);
+                for (int i = 0; i < k; ++i) sm.tri[at++] = (unsigned short)(li | (i << 9));
+            }
+        }
+        __syncthreads();
+        const int4 bc = sv.bcoord[b];
+        const float voxel = sv.voxel;
+        for (int base = warp * 10; base < count; base += 10 * (kMeshThreads / 32)) {
+            // lane 3 k + q < 30: vertex q of triangle base + k
+            const int k = lane / 3, q = lane - 3 * k, last = min(10, count - base);
+            const bool on = lane < 30 && k < last;
+            const unsigned entry = sm.tri[base + (on ? k : 0)];
+            const int li = entry & 511, lx = li & 7, ly = (li >> 3) & 7, lz = li >> 6;
+            const unsigned long long packed = kTriPacked[sm.cube[li]];
+            const int e = (int)(packed >> (4 + 12 * (entry >> 9) + 4 * (on ? q : 0))) & 0xf;
+            // edge e runs from corner c0 to c1 (scene_mesh.cu:147-205)
+            const int c0 = e < 8 ? e : e - 8, c1 = e < 8 ? (e & 4) | ((e + 1) & 3) : e - 4;
+            auto cell = [&](int c) {
+                const int dx = ((c & 3) == 1 || (c & 3) == 2) ? 1 : 0, dy = (c & 3) >> 1, dz = c >> 2;
+                return (lx + dx) + 9 * (ly + dy) + 81 * (lz + dz);
+            };
+            const int cell0 = cell(c0);
+            const float val = edge_point(sm.sdf[cell0], sm.sdf[cell(c1)]);
+            const int kind = e & 3;
+            const float far = (kind == 1 || kind == 2) ? 1.f : 0.f;  // corner x of the edges along z, and of edges 1, 2
+            float ox, oy, oz;
+            if (e < 8) {
+                ox = kind == 0 ? val : kind == 2 ? 1 - val : far;
+                oy = kind == 1 ? val : kind == 3 ? 1 - val : kind == 2 ? 1.f : 0.f;
+                oz = e < 4 ? 0.f : 1.f;
+            } else {
+                ox = far;
+                oy = kind >= 2 ? 1.f : 0.f;
+                oz = val;
+            }
+            const float px = ((float)(bc.x * 8 + lx) + ox) * voxel, py = ((float)(bc.y * 8 + ly) + oy) * voxel,
+                        pz = ((float)(bc.z * 8 + lz) + oz) * voxel;
+            float *out = sm.out[warp][0];
+            if (lane < 30) {
+                out[3 * lane] = px;
+                out[3 * lane + 1] = py;
+                out[3 * lane + 2] = pz;
+            }
+            __syncwarp();
+            const long long at = (long long)first + base;  // the warp's first triangle
+            for (int i = lane; i < 9 * last; i += 32) vtx[at * 9 + i] = out[i];
+            if (MODE == GBF_MESH_NORMAL) {
+                const float *A = out + 9 * min(k, 9);
+                const float3 u = make_float3(A[3] - A[0], A[4] - A[1], A[5] - A[2]);
+                const float3 v = make_float3(A[6] - A[0], A[7] - A[1], A[8] - A[2]);
+                const float3 nn = cross3(u, v);
+                const float l = norm3(nn.x, nn.y, nn.z);
+                // lane q divides component q, which is component q of all three vertices' normals
+                const float c = (q == 0 ? nn.x : q == 1 ? nn.y : nn.z) / l;
+                float *nrm = sm.out[warp][1];
+                if (lane < 30) nrm[9 * k + q] = nrm[9 * k + 3 + q] = nrm[9 * k + 6 + q] = c;
+                __syncwarp();
+                float *na = static_cast<float *>(attr);
+                for (int i = lane; i < 9 * last; i += 32) na[at * 9 + i] = nrm[i];
+            } else if (MODE == GBF_MESH_COLOUR && on) {
+                // edges 0-7 take corner e's colour, 8-11 corner e-8 (scene_mesh.cu:526-549)
+                const uchar4 col = rgb[cell0];
+                unsigned char *ca = static_cast<unsigned char *>(attr) + (at * 3 + lane) * 3;
+                ca[0] = col.x;
+                ca[1] = col.y;
+                ca[2] = col.z;
+            }
+            __syncwarp();
+        }
     }
 }
 
 template <int LAYOUT>
-__global__ void __launch_bounds__(kBlockVoxels) mesh_emit_kernel(const SessionView *__restrict__ svs, int mode, const int *offsets,
-                                                                 float3 *vtx, void *attr, long long max_tris) {
-    const SessionView &sv = svs[0];
-    const int n = min(sv.ctr[C_NUSED], sv.pool);
-    __shared__ MeshSmem sm;
-    for (int b = blockIdx.x; b < n; b += gridDim.x) {
-        if (offsets[b] >= max_tris || offsets[b + 1] == offsets[b]) continue;  // uniform per CTA
-        stage_block<LAYOUT>(sv, b, mode, sm);
-        float s[8];
-        int cc[8];
-        const int li = threadIdx.x;
-        const int ci = cube_of(sm, li, s, cc);
-        const int em = (ci > 0) ? edge_mask(ci) : 0;
-        const unsigned long long packed = (em != 0) ? kTriPacked[ci] : 0ull;
-        const int t = (int)(packed & 0xF);
-        // in-block exclusive prefix of t (voxel order)
-        int x = t;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, off);
-            if ((li & 31) >= off) x += y;
-        }
-        if ((li & 31) == 31) sm.warp_tot[li >> 5] = x;
-        __syncthreads();
-        if (li < 32) {
-            int w = (li < kBlockVoxels / 32) ? sm.warp_tot[li] : 0;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, w, off);
-                if (li >= off) w += y;
-            }
-            if (li < kBlockVoxels / 32) sm.warp_tot[li] = w;
-        }
-        __syncthreads();
-        const long long first = (long long)offsets[b] + ((li >> 5) ? sm.warp_tot[(li >> 5) - 1] : 0) + (x - t);
-        if (t > 0) {
-            const int4 bc = sv.bcoord[b];
-            const int px = bc.x * 8 + (li & 7), py = bc.y * 8 + ((li >> 3) & 7), pz = bc.z * 8 + (li >> 6);
-            const float fx = (float)px, fy = (float)py, fz = (float)pz;
-            // interpolate_sdf (scene_mesh.cu:108-117)
-            float3 ev[12];
-#pragma unroll
-            for (int e = 0; e < 12; ++e) {
-                if (!((em >> e) & 1)) continue;
-                const float v1 = s[kEdge[e][0]], v2 = s[kEdge[e][1]];
-                float val;
-                if ((double)fabsf(0 - v1) < 1e-6) val = 0;
-                else if ((double)fabsf(0 - v2) < 1e-6) val = 1;
-                else if ((double)fabsf(v1 - v2) < 1e-6) val = 0;
-                else val = (0 - v1) / (v2 - v1);
-                float ox, oy, oz;
-                switch (e) {
-                    case 0: ox = val; oy = 0; oz = 0; break;
-                    case 1: ox = 1; oy = val; oz = 0; break;
-                    case 2: ox = 1 - val; oy = 1; oz = 0; break;
-                    case 3: ox = 0; oy = 1 - val; oz = 0; break;
-                    case 4: ox = val; oy = 0; oz = 1; break;
-                    case 5: ox = 1; oy = val; oz = 1; break;
-                    case 6: ox = 1 - val; oy = 1; oz = 1; break;
-                    case 7: ox = 0; oy = 1 - val; oz = 1; break;
-                    case 8: ox = 0; oy = 0; oz = val; break;
-                    case 9: ox = 1; oy = 0; oz = val; break;
-                    case 10: ox = 1; oy = 1; oz = val; break;
-                    default: ox = 0; oy = 1; oz = val; break;
-                }
-                ev[e] = make_float3((fx + ox) * sv.voxel, (fy + oy) * sv.voxel, (fz + oz) * sv.voxel);
-            }
-            for (int k = 0; k < t; ++k) {
-                const long long tid = first + k;
-                if (tid >= max_tris) break;
-                const int e0 = (int)((packed >> (4 + 12 * k)) & 0xF);
-                const int e1 = (int)((packed >> (8 + 12 * k)) & 0xF);
-                const int e2 = (int)((packed >> (12 + 12 * k)) & 0xF);
-                const float3 a = ev[e0], bb = ev[e1], c = ev[e2];
-                vtx[tid * 3] = a;
-                vtx[tid * 3 + 1] = bb;
-                vtx[tid * 3 + 2] = c;
-                if (mode == GBF_MESH_NORMAL) {
-                    const float3 u = make_float3(bb.x - a.x, bb.y - a.y, bb.z - a.z);
-                    const float3 v = make_float3(c.x - a.x, c.y - a.y, c.z - a.z);
-                    const float3 nn = cross3(u, v);
-                    const float l = norm3(nn.x, nn.y, nn.z);
-                    const float3 nrm = make_float3(nn.x / l, nn.y / l, nn.z / l);
-                    float3 *na = static_cast<float3 *>(attr);
-                    na[tid * 3] = nrm;
-                    na[tid * 3 + 1] = nrm;
-                    na[tid * 3 + 2] = nrm;
-                } else if (mode == GBF_MESH_COLOUR) {
-                    // edges 0-7 take corner e's colour, 8-11 corner e-8 (scene_mesh.cu:526-549)
-                    unsigned char *ca = static_cast<unsigned char *>(attr) + tid * 9;
-                    const int es[3] = {e0, e1, e2};
-                    for (int q = 0; q < 3; ++q) {
-                        const int corner = es[q] < 8 ? es[q] : es[q] - 8;
-                        const int cell = cc[corner];
-                        ca[q * 3 + 0] = sm.rgb[cell][0];
-                        ca[q * 3 + 1] = sm.rgb[cell][1];
-                        ca[q * 3 + 2] = sm.rgb[cell][2];
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
+void launch_mesh_layout(const SessionView *d_sv, const Extent &ex, int mode, float *vtx, void *attr, long long max_tris,
+                        int *counts, cudaStream_t st) {
+    // grid-stride over the blocks, whose count only the device knows
+    const int g = min(max(ex.max_pool, 1), 152 * 16), chunks = (ex.max_pool + mesh_chunk(ex.max_pool) - 1) / mesh_chunk(ex.max_pool);
+    mesh_count_kernel<LAYOUT><<<g, kMeshThreads, 0, st>>>(d_sv, mode, counts);
+    mesh_scan_kernel<<<max(chunks, 1), 1024, 0, st>>>(d_sv, counts);
+    if (mode == GBF_MESH_VERTEX)
+        mesh_emit_kernel<LAYOUT, GBF_MESH_VERTEX><<<g, kMeshThreads, 0, st>>>(d_sv, counts, vtx, attr, max_tris);
+    else if (mode == GBF_MESH_NORMAL)
+        mesh_emit_kernel<LAYOUT, GBF_MESH_NORMAL><<<g, kMeshThreads, 0, st>>>(d_sv, counts, vtx, attr, max_tris);
+    else
+        mesh_emit_kernel<LAYOUT, GBF_MESH_COLOUR><<<g, kMeshThreads, 0, st>>>(d_sv, counts, vtx, attr, max_tris);
 }
 
 }  // namespace
 
 void launch_mesh(const SessionView *d_sv, const Extent &ex, int layout, int mode, float *vtx, void *attr,
-                 long long max_tris, int *counts, cudaStream_t st) {
-    const int g = min(max(ex.max_pool, 1), 152 * 4);
-    float3 *v3 = reinterpret_cast<float3 *>(vtx);
-    if (layout == GBF_VOXEL_REF) mesh_count_kernel<GBF_VOXEL_REF><<<g, kBlockVoxels, 0, st>>>(d_sv, mode, counts);
-    else if (layout == GBF_VOXEL_HALF) mesh_count_kernel<GBF_VOXEL_HALF><<<g, kBlockVoxels, 0, st>>>(d_sv, mode, counts);
-    else mesh_count_kernel<GBF_VOXEL_SNORM><<<g, kBlockVoxels, 0, st>>>(d_sv, mode, counts);
-    mesh_scan_kernel<<<1, 1024, 0, st>>>(d_sv, counts);
-    if (layout == GBF_VOXEL_REF)
-        mesh_emit_kernel<GBF_VOXEL_REF><<<g, kBlockVoxels, 0, st>>>(d_sv, mode, counts, v3, attr, max_tris);
-    else if (layout == GBF_VOXEL_HALF)
-        mesh_emit_kernel<GBF_VOXEL_HALF><<<g, kBlockVoxels, 0, st>>>(d_sv, mode, counts, v3, attr, max_tris);
-    else
-        mesh_emit_kernel<GBF_VOXEL_SNORM><<<g, kBlockVoxels, 0, st>>>(d_sv, mode, counts, v3, attr, max_tris);
+                 long long max_tris, int *counts, int *chunk_sums, cudaStream_t st) {
+    cudaMemsetAsync(chunk_sums, 0, kMeshChunks * sizeof(int), st);
+    if (layout == GBF_VOXEL_REF) launch_mesh_layout<GBF_VOXEL_REF>(d_sv, ex, mode, vtx, attr, max_tris, counts, st);
+    else if (layout == GBF_VOXEL_HALF) launch_mesh_layout<GBF_VOXEL_HALF>(d_sv, ex, mode, vtx, attr, max_tris, counts, st);
+    else launch_mesh_layout<GBF_VOXEL_SNORM>(d_sv, ex, mode, vtx, attr, max_tris, counts, st);
 }
 
 }  // namespace gbf

@@ -126,6 +126,7 @@ ArenaLayout plan_arena(const gbf_config &c, const gbf_intrinsics &K) {
     for (int l = 0, lw = K.width, lh = K.height; l < c.num_levels; ++l, lw /= 2, lh /= 2)
         max_ctas = std::max(max_ctas, (lw * lh + reduce_tile(l) - 1) / reduce_tile(l));
     a.partials = take((size_t)max_ctas * kPartialStride * 4);
+    a.mesh_sums = take(kMeshChunks * sizeof(int));
     a.track_rec = take((size_t)max_ctas * kPartialStride * 8);
     a.total = off;
     return a;
@@ -465,6 +466,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     v.zr_w = K->width / 8;
     v.zr_h = K->height / 8;
     v.partials = reinterpret_cast<float *>(base + a.partials);
+    v.mesh_sums = reinterpret_cast<int *>(base + a.mesh_sums);
     v.track_rec = reinterpret_cast<unsigned long long *>(base + a.track_rec);
 
     Extent &ex = s->ex;
@@ -703,7 +705,7 @@ GBF_API gbf_status gbf_extract_mesh(gbf_session *s, int32_t mode, float *vtx, vo
     if (mode != GBF_MESH_VERTEX && !attr) return set_error(GBF_ERR_INVALID_ARG, "gbf_extract_mesh: null attr");
     cudaStream_t st = (cudaStream_t)stream;
     const long long mt = (long long)std::min<uint64_t>(max_tris, (uint64_t)INT32_MAX);
-    launch_mesh(s->d_view, s->ex, s->cfg.voxel_layout, mode, vtx, attr, mt, s->view.mesh_off, st);
+    launch_mesh(s->d_view, s->ex, s->cfg.voxel_layout, mode, vtx, attr, mt, s->view.mesh_off, s->view.mesh_sums, st);
     gbf_status r = check_cuda("gbf_extract_mesh");
     if (r != GBF_OK) return r;
     int total = 0;
