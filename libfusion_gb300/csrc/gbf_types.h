@@ -112,6 +112,8 @@ struct SessionView {
     void *vox_sw;          // sdf + weight word per voxel, 512 per block: HALF uint32
                            // (fp16 sdf | fp16 weight << 16), REF uint2 (int16 sdf, f32 weight)
     uchar4 *vox_rgb;
+    int *bnext;            // per pool block: ids of the blocks at + (k & 1, k >> 1 & 1, k >> 2), k = 0..7, or -1;
+                           // of the last raycast, for the blocks its rays may meet
     int *vis;              // visible block ids
     int *ctr;              // Counter array
 
@@ -132,6 +134,7 @@ struct SessionView {
     float4 *vmap[2][kMaxLevels];
     float4 *nmap[2][kMaxLevels];
     float *zr_min, *zr_max;
+    unsigned long long *zr_slices;  // per z-range cell: depth slices that an allocated block may lie in
     int zr_w, zr_h;
 
     TrackState *ts;

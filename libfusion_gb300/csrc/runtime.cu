@@ -92,6 +92,7 @@ ArenaLayout plan_arena(const gbf_config &c, const gbf_intrinsics &K) {
     a.bcoord = take(pool * sizeof(int4));
     a.bstamp = take(pool * sizeof(int));
     a.bfresh = take(pool);
+    a.bnext = take(pool * 8 * sizeof(int));
     a.vis = take(pool * sizeof(int));
     a.mesh_off = take((pool + 1) * sizeof(int));
     a.vox_sw = take(nv * (c.voxel_layout == GBF_VOXEL_REF ? 8 : 4));
@@ -122,6 +123,7 @@ ArenaLayout plan_arena(const gbf_config &c, const gbf_intrinsics &K) {
     }
     a.zr_min = take((size_t)(K.width / 8) * (K.height / 8) * 4);
     a.zr_max = take((size_t)(K.width / 8) * (K.height / 8) * 4);
+    a.zr_slices = take((size_t)(K.width / 8) * (K.height / 8) * 8);
     int max_ctas = 1;
     for (int l = 0, lw = K.width, lh = K.height; l < c.num_levels; ++l, lw /= 2, lh /= 2)
         max_ctas = std::max(max_ctas, (lw * lh + reduce_tile(l) - 1) / reduce_tile(l));
@@ -438,6 +440,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     v.bcoord = reinterpret_cast<int4 *>(base + a.bcoord);
     v.bstamp = reinterpret_cast<int *>(base + a.bstamp);
     v.bfresh = reinterpret_cast<unsigned char *>(base + a.bfresh);
+    v.bnext = reinterpret_cast<int *>(base + a.bnext);
     v.vis = reinterpret_cast<int *>(base + a.vis);
     v.mesh_off = reinterpret_cast<int *>(base + a.mesh_off);
     v.vox_sw = base + a.vox_sw;
@@ -463,6 +466,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     }
     v.zr_min = reinterpret_cast<float *>(base + a.zr_min);
     v.zr_max = reinterpret_cast<float *>(base + a.zr_max);
+    v.zr_slices = reinterpret_cast<unsigned long long *>(base + a.zr_slices);
     v.zr_w = K->width / 8;
     v.zr_h = K->height / 8;
     v.partials = reinterpret_cast<float *>(base + a.partials);
@@ -486,6 +490,12 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     if (e != cudaSuccess) {
         gbf_session_destroy(s);
         return cuda_error(e, "gbf_session_create: upload view");
+    }
+    // neighbour lists hold block ids of the pool or -1 from the start
+    e = cudaMemset(s->view.bnext, 0xff, (size_t)cfg->num_blocks * 8 * sizeof(int));
+    if (e != cudaSuccess) {
+        gbf_session_destroy(s);
+        return cuda_error(e, "gbf_session_create: neighbour lists");
     }
     st = reset_session(s, 0);
     if (st != GBF_OK) {

@@ -93,3 +93,45 @@ def test_render_scene_matches_oracle(gbf):
     if bg.any():
         assert (g[bg][:, :3] == O.render_scene(np.full((1, 1, 4), np.nan, np.float32),
                                                np.zeros((1, 1, 4), np.float32))[0, 0, :3]).all()
+
+
+@pytest.mark.parametrize("voxel,zmin,far", [(0.01, 0.3, 0.0), (0.04, 0.05, 0.0), (0.004, 0.3, 0.0), (0.01, 0.3, 3000.0)])
+def test_raycast_skips_only_empty_space(gbf, voxel, zmin, far):
+    """Rays pass depth slices without a block unread and take neighbouring blocks
+    from lists: from poses inside, at and away from the surfaces, with blocks that
+    reach the camera plane, and with a map whose coordinates round a ray's steps
+    (3 km from the origin: 1/64 voxel per step), vertices and hit masks are the
+    oracle's bit for bit."""
+    import oracle as O
+    import torch
+    L = gbf
+    K = L.IntrinsicMatrix(168, 120, 110.0, 105.0, 80.3, 61.7)
+    cfg = H.small_config(L, 0, voxel_size=voxel, truncation=3 * voxel, zmin_raycast=zmin, zmin_update=0.3,
+                         num_blocks=1 << 16, num_buckets=1 << 18)
+    m, om = L.DenseMapping(K, cfg), O.OracleMap(O.config_from(cfg), O.intrinsics_from(K))
+    shift = np.array([far, -far, far / 2])
+    poses = []
+    for d, c, T in H.frames(L, K, 3, step=40, seed=5):
+        T = T.copy()
+        T[:3, 3] += shift
+        m.update(H.cuda(H.depth_m(d)), H.cuda(c), T)
+        om.fuse(H.depth_m(d), c, T)
+        poses.append((T, H.depth_m(d)[60, 84]))
+    rng = np.random.default_rng(2)
+    vmap = torch.empty((K.height, K.width, 4), dtype=torch.float32, device="cuda")
+    hits = 0
+    for T, z in poses:
+        for ahead in (0.0, 0.6 * z, z - 0.2, z, z + 0.05):  # up to and through the surface
+            P = T.copy()
+            a, b = rng.uniform(-0.6, 0.6, 2)
+            R = np.array([[np.cos(a), 0, np.sin(a)], [0, 1, 0], [-np.sin(a), 0, np.cos(a)]]) @ \
+                np.array([[np.cos(b), -np.sin(b), 0], [np.sin(b), np.cos(b), 0], [0, 0, 1]])
+            P[:3, 3] += ahead * T[:3, 2]
+            P[:3, :3] = T[:3, :3] @ R
+            m.raycast_check_visibility(vmap, P)
+            o = om.raycast_check_visibility(P)
+            g = vmap.cpu().numpy()
+            gh, oh = ~np.isnan(g[..., 2]), ~np.isnan(o[..., 2])
+            assert np.array_equal(gh, oh) and np.array_equal(g[gh], o[oh])
+            hits += int(gh.sum())
+    assert hits > 5000
