@@ -4,7 +4,7 @@
 //
 // GB300 design:
 //   zr_init   z-range grid (H/8 x W/8) to (100, 0), render counter to 0.
-//   zrange    one thread per visible block: the block's screen box on the 1/8
+//   zrange    eight lanes per visible block: the block's screen box on the 1/8
 //             grid and its depth interval (create_rendering_block, :63-126), then
 //             integer atomicMin / atomicMax on the float bit patterns (all values
 //             are positive) of every covered cell.  The reference's 16x16
@@ -27,7 +27,8 @@
 //             the unallocated block a ray is in (each lane its own) measured slower.
 //             640x480, march: 64 sessions 4.10 -> 2.72 ms per tick (slices 3.60,
 //             shorter sample code 3.34, neighbour lists 2.72), one 0.193 -> 0.134;
-//             the slices and lists cost 0.13 and 0.010 ms of z-range.
+//             the z-range launch, slices and lists included, takes 0.22 and 0.018 ms
+//             (0.18 and 0.018 without them and with a thread per block; 0.31 and 0.028 with).
 //   post      2x2 mean vertex pyramid, then normals of every level.
 #include "gbf_device.cuh"
 #include "gbf_kernels.h"
@@ -73,6 +74,18 @@ __device__ __forceinline__ float ray_margin(const SessionView &sv) {
     return sv.voxel * (1.f + N * (A * 0x1p-22f));
 }
 
+// The cells of a box, shared out to the eight lanes of a block.
+template <class F>
+__device__ __forceinline__ void for_cells(int x0, int y0, int x1, int y1, const F &f) {
+    const int w = x1 - x0 + 1, n = w * (y1 - y0 + 1);
+    const float inv = 1.0f / (float)w;
+    for (int i = threadIdx.x & 7; i < n; i += 8) {
+        // i / w: i + 1/2 keeps the quotient 1 / (2 w) clear of an integer, and w, n stay below 2^20
+        const int row = (int)(((float)i + 0.5f) * inv);
+        f(x0 + i - row * w, y0 + row);
+    }
+}
+
 // False when no sample of a raycast at this pose can lie in the block.
 __device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tcw, float margin, const int4 bc) {
     const LevelK &K = sv.lv[0];
@@ -101,84 +114,74 @@ __device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tc
     const int s0 = min(max((int)((z0 - sv.zmin_r) * scale), 0), kSlices - 1);
     const int s1 = min((int)((z1 - sv.zmin_r) * scale), kSlices - 1);
     const unsigned long long bits = (~0ull >> (kSlices - 1 - (s1 - s0))) << s0;
-    for (int y = cy0; y <= cy1; ++y)
-        for (int x = cx0; x <= cx1; ++x) atomicOr(sv.zr_slices + y * sv.zr_w + x, bits);
+    for_cells(cx0, cy0, cx1, cy1, [&](int x, int y) { atomicOr(sv.zr_slices + y * sv.zr_w + x, bits); });
     return true;
 }
 
-// The first half of the CTAs takes the visible blocks (z-range), the second the
-// allocated ones (slices, and the neighbour lists of the blocks that rays may
-// meet): two passes whose latencies do not add up.
+// Eight lanes to a block, a corner, a share of the cells and a neighbour each:
+// a session has some 20,000 blocks, which a thread each would leave to 600 warps
+// of long loops.  The first half of the CTAs takes the visible blocks (z-range),
+// the second the allocated ones (slices, and the neighbour lists of the blocks
+// that rays may meet).
 __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__restrict__ svs) {
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     __shared__ M34 Tcw;
     __shared__ float margin;
-    if (threadIdx.x == 0) Tcw = load_m34(sv.ts->map_tcw);
+    if (threadIdx.x < 12) Tcw.m[threadIdx.x] = sv.ts->map_tcw[threadIdx.x];
     if (threadIdx.x == 32) margin = ray_margin(sv);
     __syncthreads();
-    const int half = gridDim.x / 2;
+    const int half = gridDim.x / 2, c = threadIdx.x & 7, per_cta = blockDim.x / 8, stride = half * per_cta;
     if (blockIdx.x >= half) {
-        const int used = min(sv.ctr[C_NUSED], sv.pool), lane = threadIdx.x & 31;
-        for (int base = (blockIdx.x - half) * blockDim.x + (threadIdx.x & ~31); base < used; base += half * blockDim.x) {
-            const int b = base + lane;
-            unsigned in = __ballot_sync(0xffffffffu, b < used && mark_slices(sv, Tcw, margin, sv.bcoord[b]));
-            // eight lanes to a block
-            while (in) {
-                int pick = -1;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int j = __ffs(in) - 1;
-                    if (lane >> 3 == k) pick = j;
-                    in &= in - 1u;
-                }
-                if (pick >= 0) {
-                    const int id = base + pick, k = lane & 7;
-                    const int4 bc = sv.bcoord[id];
-                    sv.bnext[(size_t)id * 8 + k] =
-                        k == 0 ? id : find_block(sv, bc.x + (k & 1), bc.y + ((k >> 1) & 1), bc.z + (k >> 2));
-                }
-                __syncwarp();
-            }
+        const int used = min(sv.ctr[C_NUSED], sv.pool);
+        for (int id = (blockIdx.x - half) * per_cta + threadIdx.x / 8; id < used; id += stride) {
+            const int4 bc = sv.bcoord[id];
+            if (!mark_slices(sv, Tcw, margin, bc)) continue;
+            sv.bnext[(size_t)id * 8 + c] =
+                c == 0 ? id : find_block(sv, bc.x + (c & 1), bc.y + ((c >> 1) & 1), bc.z + (c >> 2));
         }
         return;
     }
     const int nvis = sv.ctr[C_NVIS];
     const LevelK &K = sv.lv[0];
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nvis; b += half * blockDim.x) {
-        const int id = sv.vis[b] & 0x7fffffff;
+    // whole warps iterate together: the corners meet by shuffles
+    for (int base = blockIdx.x * per_cta + (threadIdx.x & ~31) / 8; base < nvis; base += stride) {
+        const int b = base + ((threadIdx.x & 31) >> 3);
+        const int id = sv.vis[min(b, nvis - 1)] & 0x7fffffff;
         const int4 bc = sv.bcoord[id];
-        int ulx = sv.zr_w, uly = sv.zr_h, lrx = -1, lry = -1;
-        float zx = sv.zmax_r, zy = sv.zmin_r;
+        const int cx = bc.x + (c & 1), cy = bc.y + ((c >> 1) & 1), cz = bc.z + (c >> 2);
+        const float3 p = Tcw.apply((float)cx * sv.block_metric, (float)cy * sv.block_metric, (float)cz * sv.block_metric);
+        const float u = ((K.fx * p.x) / p.z + K.cx) / 8.0f;
+        const float v = ((K.fy * p.y) / p.z + K.cy) / 8.0f;
+        // the reference's running bounds from (zr_w, zr_h, -1, -1): a NaN coordinate changes none
+        const float fu = floorf(u), fv = floorf(v), cu = ceilf(u), cv = ceilf(v);
+        int ulx = (float)sv.zr_w > fu ? __float2int_rz(fu) : sv.zr_w, lrx = -1.f < cu ? __float2int_rz(cu) : -1;
+        int uly = (float)sv.zr_h > fv ? __float2int_rz(fv) : sv.zr_h, lry = -1.f < cv ? __float2int_rz(cv) : -1;
+        float zx = sv.zmax_r > p.z ? p.z : sv.zmax_r, zy = sv.zmin_r < p.z ? p.z : sv.zmin_r;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const int cx = bc.x + ((c & 1) ? 1 : 0), cy = bc.y + ((c & 2) ? 1 : 0), cz = bc.z + ((c & 4) ? 1 : 0);
-            const float3 p = Tcw.apply((float)cx * sv.block_metric, (float)cy * sv.block_metric,
-                                       (float)cz * sv.block_metric);
-            const float u = ((K.fx * p.x) / p.z + K.cx) / 8.0f;
-            const float v = ((K.fy * p.y) / p.z + K.cy) / 8.0f;
-            const float fu = floorf(u), fv = floorf(v), cu = ceilf(u), cv = ceilf(v);
-            if ((float)ulx > fu) ulx = __float2int_rz(fu);
-            if ((float)lrx < cu) lrx = __float2int_rz(cu);
-            if ((float)uly > fv) uly = __float2int_rz(fv);
-            if ((float)lry < cv) lry = __float2int_rz(cv);
-            if (zx > p.z) zx = p.z;
-            if (zy < p.z) zy = p.z;
+        for (int m = 1; m < 8; m <<= 1) {
+            ulx = min(ulx, __shfl_xor_sync(0xffffffffu, ulx, m));
+            uly = min(uly, __shfl_xor_sync(0xffffffffu, uly, m));
+            lrx = max(lrx, __shfl_xor_sync(0xffffffffu, lrx, m));
+            lry = max(lry, __shfl_xor_sync(0xffffffffu, lry, m));
+            const float x = __shfl_xor_sync(0xffffffffu, zx, m), y = __shfl_xor_sync(0xffffffffu, zy, m);
+            zx = fminf(zx, x);
+            zy = fmaxf(zy, y);
         }
-        if (ulx < 0) ulx = 0;
-        if (uly < 0) uly = 0;
-        if (lrx >= sv.zr_w) lrx = sv.zr_w - 1;
-        if (lry >= sv.zr_h) lry = sv.zr_h - 1;
-        if (ulx > lrx || uly > lry) continue;
-        if (zx < sv.zmin_r) zx = sv.zmin_r;
-        if (zy < sv.zmin_r) continue;
-        atomicAdd(sv.ctr + C_RENDER, 1);
+        ulx = max(ulx, 0);
+        uly = max(uly, 0);
+        lrx = min(lrx, sv.zr_w - 1);
+        lry = min(lry, sv.zr_h - 1);
+        zx = fmaxf(zx, sv.zmin_r);
+        const bool renders = b < nvis && ulx <= lrx && uly <= lry;  // (zy is never below zmin)
+        const unsigned n = __ballot_sync(0xffffffffu, renders && c == 0);
+        if ((threadIdx.x & 31) == 0 && n) atomicAdd(sv.ctr + C_RENDER, __popc(n));
+        if (!renders) continue;
         const int ix = __float_as_int(zx), iy = __float_as_int(zy);
-        for (int y = uly; y <= lry; ++y)
-            for (int x = ulx; x <= lrx; ++x) {
-                atomicMin(reinterpret_cast<int *>(sv.zr_min) + y * sv.zr_w + x, ix);
-                atomicMax(reinterpret_cast<int *>(sv.zr_max) + y * sv.zr_w + x, iy);
-            }
+        for_cells(ulx, uly, lrx, lry, [&](int x, int y) {
+            atomicMin(reinterpret_cast<int *>(sv.zr_min) + y * sv.zr_w + x, ix);
+            atomicMax(reinterpret_cast<int *>(sv.zr_max) + y * sv.zr_w + x, iy);
+        });
     }
 }
 
@@ -593,7 +596,8 @@ __global__ void nmap_all_kernel(const SessionView *__restrict__ svs) {
 void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
     const int cells = (ex.w / 8) * (ex.h / 8);
     zr_init_kernel<<<dim3((cells + 255) / 256, nslots), 256, 0, st>>>(d_sv);
-    const int gz = min(max((ex.max_pool + 255) / 256, 1), 304);
+    // two halves of up to three resident CTAs per SM each; fewer of many sessions, whose CTAs loop
+    const int gz = min(max((ex.max_pool + 31) / 32, 1), max(152, 152 * 3 / nslots));
     zrange_kernel<<<dim3(2 * gz, nslots), 256, 0, st>>>(d_sv);
 }
 
