@@ -366,4 +366,15 @@ __device__ __forceinline__ int insert_block(const SessionView &sv, unsigned long
     return -1;
 }
 
+// The z-range grid of a raycast to (100, 0) and no slices, its render counter to
+// 0; thread i of n.
+__device__ __forceinline__ void clear_zrange(const SessionView &sv, int i, int n) {
+    if (i == 0) sv.ctr[C_RENDER] = 0;
+    for (const int cells = sv.zr_w * sv.zr_h; i < cells; i += n) {
+        sv.zr_min[i] = 100.f;
+        sv.zr_max[i] = 0.f;
+        sv.zr_slices[i] = 0ull;
+    }
+}
+
 }  // namespace gbf

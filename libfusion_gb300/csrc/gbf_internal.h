@@ -25,7 +25,7 @@ gbf_status check_cuda(const char *where);
 struct ArenaLayout {
     size_t total;
     size_t table, bcoord, bstamp, bfresh, bnext, vis, mesh_off, vox_sw, vox_rgb, ctr, ts;
-    size_t in_depth, in_rgb, depth_raw, rgb4, nmap_ext, fuse_px, zr_min, zr_max, zr_slices, partials, track_rec, mesh_sums;
+    size_t in_depth, in_rgb, depth_raw, rgb4, fuse_px, zr_min, zr_max, zr_slices, partials, track_rec, mesh_sums;
     size_t depth[kMaxLevels], inten[2][kMaxLevels], gx[kMaxLevels], gy[kMaxLevels];
     size_t vmap[2][kMaxLevels], nmap[2][kMaxLevels], igd[2][kMaxLevels];
 };

@@ -40,11 +40,10 @@ struct FuseImport {
     const uint8_t *rgb; long long rgb_pitch;
     const float *nmap; long long nmap_pitch;
 };
-// mode: 0 colour update (1/d^2), 1 weighted update with the reference set's
-// level-0 normals, 2 weighted update with the imported normals.
-void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImport &in, cudaStream_t st);
-void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, int mode, const int *layouts,
-                 cudaStream_t st);
+// the caller's images and pose: colour update (1/d^2), or weighted with the imported normals
+void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImport &in, const double pose[12],
+                        cudaStream_t st);
+void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st);
 void launch_alloc_visible(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
 // visible list = allocated blocks in the frustum of the map pose (no fuse)
 void launch_visible_frustum(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
@@ -52,14 +51,18 @@ void launch_visible_frustum(const SessionView *d_sv, int nslots, const Extent &e
 void launch_render(const float4 *vmap, long long vmap_pitch, const float4 *nmap, long long nmap_pitch,
                    const uint8_t *rgb, long long rgb_pitch, int rgb_stride, int w, int h, uchar4 *out,
                    long long out_pitch, cudaStream_t st);
-void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, int mode, const int *layouts,
-                      cudaStream_t st);
+void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st);
+// the session's model prediction, shaded (textured: with the last frame's colour)
+void launch_render_session(const SessionView *d_sv, const Extent &ex, int textured, uchar4 *out, long long out_pitch,
+                           cudaStream_t st);
 
 // ---- raycast (raycast.cu) -------------------------------------------------------
+// One session's raycast at `pose`, optionally over the visible blocks of that pose.
 // rgb_ext (optional): the hits' nearest voxel colours, 3 bytes per pixel, white elsewhere
-void launch_raycast(const SessionView *d_sv, int nslots, const Extent &ex, float4 *vmap_ext, long long vmap_pitch,
-                    int post_pyramid, const int *layouts, cudaStream_t st, uint8_t *rgb_ext = nullptr,
-                    long long rgb_pitch = 0);
+void launch_raycast(const SessionView *d_sv, const Extent &ex, const double pose[12], bool check_visibility,
+                    float4 *vmap_ext, long long vmap_pitch, const int *layouts, cudaStream_t st,
+                    uint8_t *rgb_ext = nullptr, long long rgb_pitch = 0);
+// the z-range pass, its grid cleared before (launch_alloc_visible, launch_raycast)
 void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
 void launch_march(const SessionView *d_sv, int nslots, const Extent &ex, float4 *vmap_ext, long long vmap_pitch,
                   const int *layouts, cudaStream_t st, uint8_t *rgb_ext = nullptr, long long rgb_pitch = 0);

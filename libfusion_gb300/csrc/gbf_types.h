@@ -122,7 +122,6 @@ struct SessionView {
     uint8_t *in_rgb;       // staging rgb8
     float *depth_raw;      // level-0 metres, unfiltered (fused)
     uchar4 *rgb4;          // level-0 colour (fused)
-    float4 *nmap_ext;      // imported normal map (gbf_fuse)
     float2 *fuse_px;       // per pixel of the fused frame: (depth or NaN if rejected, weight)
     float *depth[kMaxLevels];
     float *inten[2][kMaxLevels];

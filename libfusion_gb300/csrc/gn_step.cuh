@@ -24,6 +24,8 @@
 
 #include <cuda_runtime.h>
 
+#include "gbf_types.h"
+
 namespace gbf {
 
 // Full-warp shuffles: every lane must reach each call (none may sit inside a
@@ -172,6 +174,27 @@ __device__ __forceinline__ double pose_mul_warp(double a, double b) {
     const double b0 = shfl_d(b, j), b1 = shfl_d(b, 4 + j), b2 = shfl_d(b, 8 + j);
     const double s = (a0 * b0 + a1 * b1) + a2 * b2;
     return j == 3 ? s + a3 : s;
+}
+
+// A pose as a kernel argument: no copy and no launch of its own.
+struct MapPose {
+    double p[12];
+};
+
+// The mapping pose and its float forms (update_map_floats), by one warp.
+__device__ __forceinline__ void store_map_pose(TrackState *ts, const MapPose &pose) {
+    const int lane = threadIdx.x & 31;
+    double v = 0.0;
+#pragma unroll
+    for (int i = 0; i < 12; ++i)
+        if (lane == i) v = pose.p[i];
+    __syncwarp();
+    const double inv = pose_inverse_warp(v);
+    if (lane < 12) {
+        ts->map_pose[lane] = v;
+        ts->map_twc[lane] = (float)v;
+        ts->map_tcw[lane] = (float)inv;
+    }
 }
 
 }  // namespace gbf

@@ -3,7 +3,8 @@
 // src/data_struct/map_struct.cu:143-389).
 //
 // GB300 design, per frame and for every session of a batch:
-//   fuse_begin  bump the session's fuse counter, clear the visible count.
+//   import      (gbf_fuse) the caller's images and pose, and each pixel's
+//               integration test and weight; a System frame has them from its ingest.
 //   alloc       one thread per level-0 pixel walks the blocks of its truncation
 //               band (3-D Bresenham, depth_fusion.cu:121-228); the CTA dedupes
 //               the keys of its 16x16 pixel tile in a shared-memory set and each
@@ -20,6 +21,7 @@
 //               of the reference's full-pool cudaMemset, map_struct.cu:90).
 #include "gbf_device.cuh"
 #include "gbf_kernels.h"
+#include "gn_step.cuh"
 
 namespace gbf {
 
@@ -28,24 +30,33 @@ namespace {
 constexpr int kAllocTile = 16;        // 16x16 pixels per CTA
 constexpr int kSetSize = 1024;        // shared-memory key set per CTA
 
-__global__ void fuse_begin_kernel(const SessionView *__restrict__ svs) {
-    const SessionView &sv = svs[blockIdx.x];
-    if (!sv.active || threadIdx.x != 0) return;
-    sv.ctr[C_FRAME] += 1;
-    sv.ctr[C_NVIS] = 0;
-}
-
-__global__ void fuse_import_kernel(const SessionView *__restrict__ svs, FuseImport in) {
+// Per-pixel part of the integration test and weight (update_map_with_colour_kernel,
+// depth_fusion.cu:317-331, without normals; update_map_weighted_kernel, :390-405, with):
+// every voxel projecting to a pixel shares them, so they are computed once per
+// pixel.  System frames get the same values from level_maps_kernel.  (1e-2f lies
+// just below the reference's double 1e-2: the floats below that are those below 1e-2f, and 1e-2f.)
+__global__ void fuse_import_kernel(const SessionView *__restrict__ svs, FuseImport in, MapPose pose) {
     const SessionView &sv = svs[0];
+    if (blockIdx.x == 0 && threadIdx.x < 32) store_map_pose(sv.ts, pose);
     const int W = sv.lv[0].w, H = sv.lv[0].h;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= W * H) return;
     const int x = i % W, y = i / W;
-    sv.depth_raw[i] = reinterpret_cast<const float *>(reinterpret_cast<const char *>(in.depth) + y * in.depth_pitch)[x];
+    const float dist = reinterpret_cast<const float *>(reinterpret_cast<const char *>(in.depth) + y * in.depth_pitch)[x];
+    sv.depth_raw[i] = dist;
     const uint8_t *px = in.rgb + y * in.rgb_pitch + (size_t)x * 3;
     sv.rgb4[i] = make_uchar4(px[0], px[1], px[2], 0);
-    if (in.nmap)
-        sv.nmap_ext[i] = reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(in.nmap) + y * in.nmap_pitch)[x];
+    bool ok;
+    float w;
+    if (!in.nmap) {
+        ok = !(isnan(dist) || dist <= 1e-2f || dist > sv.zmax_u || dist < sv.zmin_u);
+        w = 1.0f / (dist * dist);
+    } else {
+        const float4 nc = reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(in.nmap) + y * in.nmap_pitch)[x];
+        ok = !(isnan(dist) || isnan(nc.x) || dist > sv.zmax_u || dist < sv.zmin_u);
+        w = fabsf(sinf(nc.z)) / (dist * dist);
+    }
+    sv.fuse_px[i] = make_float2(ok ? dist : __int_as_float(0x7fffffff), w);
 }
 
 // Shared-memory set insert; false when the set is full (caller inserts globally).
@@ -94,7 +105,8 @@ __global__ void __launch_bounds__(kAllocTile *kAllocTile) alloc_kernel(const Ses
     for (int i = threadIdx.x; i < kSetSize; i += blockDim.x) set[i] = kEmptyKey;
     if (threadIdx.x == 0) T = load_m34(sv.ts->map_twc);
     __syncthreads();
-    const int frame = sv.ctr[C_FRAME];
+    const int frame = sv.ctr[C_FRAME] + 1;  // counted by integrate_kernel
+    if (blockIdx.x == 0 && threadIdx.x == 0) sv.ctr[C_NVIS] = 0;
 
     if (x < W && y < H) {
         const float z = sv.depth_raw[(size_t)y * W + x];
@@ -152,30 +164,6 @@ __global__ void __launch_bounds__(kAllocTile *kAllocTile) alloc_kernel(const Ses
     }
 }
 
-// Per-pixel part of the integration test and weight (update_map_with_colour_kernel,
-// depth_fusion.cu:317-331, mode 0; update_map_weighted_kernel, :390-405, mode 2):
-// every voxel projecting to a pixel shares them, so they are computed once per
-// pixel.  Mode 1 (System frames) gets the same values from level_maps_kernel.
-__global__ void fuse_prep_kernel(const SessionView *__restrict__ svs, int mode) {
-    const SessionView &sv = svs[blockIdx.y];
-    if (!sv.active) return;
-    const int n = sv.lv[0].w * sv.lv[0].h;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float dist = sv.depth_raw[i];
-    bool ok;
-    float w;
-    if (mode == 0) {
-        ok = !(isnan(dist) || (double)dist < 1e-2 || dist > sv.zmax_u || dist < sv.zmin_u);
-        w = 1.0f / (dist * dist);
-    } else {
-        const float4 nc = sv.nmap_ext[i];
-        ok = !(isnan(dist) || isnan(nc.x) || dist > sv.zmax_u || dist < sv.zmin_u);
-        w = fabsf(sinf(nc.z)) / (dist * dist);
-    }
-    sv.fuse_px[i] = make_float2(ok ? dist : __int_as_float(0x7fffffff), w);
-}
-
 // is_vertex_visible / is_block_visible (depth_fusion.cu:15-47)
 __device__ __forceinline__ bool block_in_frustum(const SessionView &sv, const M34 &Tcw, int bx, int by, int bz) {
     const LevelK &K = sv.lv[0];
@@ -192,14 +180,8 @@ __device__ __forceinline__ bool block_in_frustum(const SessionView &sv, const M3
     return false;
 }
 
-__global__ void vis_begin_kernel(const SessionView *__restrict__ svs) {
-    const SessionView &sv = svs[blockIdx.x];
-    if (!sv.active || threadIdx.x != 0) return;
-    sv.ctr[C_NVIS] = 0;
-}
-
-// touched: also count blocks stamped by this fuse (check_visibility_flag_kernel's
-// flag 2); without it, the frustum test alone (count_visible_entry,
+// TOUCHED: also count blocks stamped by this fuse (check_visibility_flag_kernel's
+// flag 2), and clear the z-range grid of the raycast that follows; without it, the frustum test alone (count_visible_entry,
 // ray_tracing.cu:778-807 with VisibleEntryEvaluateFunctor, :681-710).
 template <bool TOUCHED>
 __global__ void __launch_bounds__(256, 6) visible_kernel(const SessionView *svs) {
@@ -208,7 +190,8 @@ __global__ void __launch_bounds__(256, 6) visible_kernel(const SessionView *svs)
     __shared__ M34 Tcw;
     if (threadIdx.x == 0) Tcw = load_m34(sv.ts->map_tcw);
     __syncthreads();
-    const int frame = sv.ctr[C_FRAME];
+    if (TOUCHED) clear_zrange(sv, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    const int frame = sv.ctr[C_FRAME] + 1;
     const int n = min(sv.ctr[C_NUSED], sv.pool);
     const int stride = gridDim.x * blockDim.x;
     // whole warps iterate together so the append stays warp-uniform
@@ -229,7 +212,7 @@ __global__ void __launch_bounds__(256, 6) visible_kernel(const SessionView *svs)
 constexpr int kIntThreads = 128;  // threads per integration CTA (512 / kIntThreads voxels each), 16 CTAs per SM
 
 template <int LAYOUT>
-__global__ void __launch_bounds__(kIntThreads, 16) integrate_kernel(const SessionView *__restrict__ svs, int mode) {
+__global__ void __launch_bounds__(kIntThreads, 16) integrate_kernel(const SessionView *__restrict__ svs) {
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active || sv.layout != LAYOUT) return;
     __shared__ M34 Tcw_s;
@@ -242,7 +225,10 @@ __global__ void __launch_bounds__(kIntThreads, 16) integrate_kernel(const Sessio
     const LevelK K = sv.lv[0];
     const int W = K.w, H = K.h;
     const int nvis = sv.ctr[C_NVIS];
-    if (blockIdx.x == 0 && threadIdx.x == 0) sv.ts->integrated_blocks += nvis;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sv.ts->integrated_blocks += nvis;
+        sv.ctr[C_FRAME] += 1;  // the allocation stamp of this fuse; no kernel reads it beside this one
+    }
     const float voxel = sv.voxel, tau = sv.tau, inv_tau = sv.inv_tau;
     const int *__restrict__ vis = sv.vis;
     const int4 *__restrict__ bcoord = sv.bcoord;
@@ -322,9 +308,12 @@ __global__ void __launch_bounds__(kIntThreads, 16) integrate_kernel(const Sessio
 
 }  // namespace
 
-void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImport &in, cudaStream_t st) {
+void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImport &in, const double pose[12],
+                        cudaStream_t st) {
     const int n = ex.w * ex.h;
-    fuse_import_kernel<<<(n + 255) / 256, 256, 0, st>>>(d_sv, in);
+    MapPose p;
+    for (int i = 0; i < 12; ++i) p.p[i] = pose[i];
+    fuse_import_kernel<<<(n + 255) / 256, 256, 0, st>>>(d_sv, in, p);
 }
 
 // CTAs per session of the visible-block pass (grid-stride over the allocated
@@ -333,7 +322,6 @@ void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImp
 constexpr int kVisCtas = 152;
 
 void launch_alloc_visible(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
-    fuse_begin_kernel<<<nslots, 32, 0, st>>>(d_sv);
     const int tiles = ((ex.w + kAllocTile - 1) / kAllocTile) * ((ex.h + kAllocTile - 1) / kAllocTile);
     alloc_kernel<<<dim3(tiles, nslots), kAllocTile * kAllocTile, 0, st>>>(d_sv);
     const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
@@ -341,29 +329,25 @@ void launch_alloc_visible(const SessionView *d_sv, int nslots, const Extent &ex,
 }
 
 void launch_visible_frustum(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
-    vis_begin_kernel<<<nslots, 32, 0, st>>>(d_sv);
     const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
     visible_kernel<false><<<dim3(gv, nslots), 256, 0, st>>>(d_sv);
 }
 
-void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, int mode, const int *layouts,
-                      cudaStream_t st) {
-    if (mode != 1) fuse_prep_kernel<<<dim3((ex.w * ex.h + 255) / 256, nslots), 256, 0, st>>>(d_sv, mode);
+void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st) {
     // One CTA per visible block, grid-stride.  16 CTAs of 128 threads are resident per
     // SM; a session alone takes twice as many, so that an SM done early finds
     // more (640x480, 5 mm: 88 us with 8 per SM, 73 with 16, 68 with 32, 66 with 64).
     // Many sessions fill the chip with 8 each, and a CTA's prologue then counts
     // (64 sessions: 1.77 ms with 8, 1.80 with 16, 1.88 with 32, 2.03 with 64).
     const int gi = 152 * max(8, 32 / nslots);
-    if (layouts[GBF_VOXEL_REF]) integrate_kernel<GBF_VOXEL_REF><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv, mode);
-    if (layouts[GBF_VOXEL_HALF]) integrate_kernel<GBF_VOXEL_HALF><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv, mode);
-    if (layouts[GBF_VOXEL_SNORM]) integrate_kernel<GBF_VOXEL_SNORM><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv, mode);
+    if (layouts[GBF_VOXEL_REF]) integrate_kernel<GBF_VOXEL_REF><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv);
+    if (layouts[GBF_VOXEL_HALF]) integrate_kernel<GBF_VOXEL_HALF><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv);
+    if (layouts[GBF_VOXEL_SNORM]) integrate_kernel<GBF_VOXEL_SNORM><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv);
 }
 
-void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, int mode, const int *layouts,
-                 cudaStream_t st) {
+void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st) {
     launch_alloc_visible(d_sv, nslots, ex, st);
-    launch_integrate(d_sv, nslots, ex, mode, layouts, st);
+    launch_integrate(d_sv, nslots, ex, layouts, st);
 }
 
 }  // namespace gbf

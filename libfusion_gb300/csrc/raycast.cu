@@ -3,7 +3,9 @@
 // resize_device_map, src/tracking/device_image.cpp:188-199).
 //
 // GB300 design:
-//   zr_init   z-range grid (H/8 x W/8) to (100, 0), render counter to 0.
+//   begin     (raycast calls) the pose, the z-range grid (H/8 x W/8) to (100, 0); a
+//             System frame has its pose from tracking and the grid cleared by the
+//             visible-block pass.
 //   zrange    eight lanes per visible block: the block's screen box on the 1/8
 //             grid and its depth interval (create_rendering_block, :63-126), then
 //             integer atomicMin / atomicMax on the float bit patterns (all values
@@ -32,21 +34,17 @@
 //   post      2x2 mean vertex pyramid, then normals of every level.
 #include "gbf_device.cuh"
 #include "gbf_kernels.h"
+#include "gn_step.cuh"
 
 namespace gbf {
 
 namespace {
 
-__global__ void zr_init_kernel(const SessionView *__restrict__ svs) {
-    const SessionView &sv = svs[blockIdx.y];
-    if (!sv.active) return;
-    const int n = sv.zr_w * sv.zr_h;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        sv.zr_min[i] = 100.f;
-        sv.zr_max[i] = 0.f;
-        sv.zr_slices[i] = 0ull;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) sv.ctr[C_RENDER] = 0;
+__global__ void ray_begin_kernel(const SessionView *__restrict__ svs, MapPose pose, int check_visibility) {
+    const SessionView &sv = svs[0];
+    if (blockIdx.x == 0 && threadIdx.x < 32) store_map_pose(sv.ts, pose);
+    if (check_visibility && blockIdx.x == 0 && threadIdx.x == 32) sv.ctr[C_NVIS] = 0;  // counted again by visible_kernel
+    clear_zrange(sv, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // The depth slices of a cell that an allocated block may lie in: 64 slices of the
@@ -594,8 +592,6 @@ __global__ void nmap_all_kernel(const SessionView *__restrict__ svs) {
 }  // namespace
 
 void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
-    const int cells = (ex.w / 8) * (ex.h / 8);
-    zr_init_kernel<<<dim3((cells + 255) / 256, nslots), 256, 0, st>>>(d_sv);
     // two halves of up to three resident CTAs per SM each; fewer of many sessions, whose CTAs loop
     const int gz = min(max((ex.max_pool + 31) / 32, 1), max(152, 152 * 3 / nslots));
     zrange_kernel<<<dim3(2 * gz, nslots), 256, 0, st>>>(d_sv);
@@ -648,11 +644,16 @@ void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, cudaStre
     nmap_all_kernel<<<dim3(total, nslots), 256, 0, st>>>(d_sv);
 }
 
-void launch_raycast(const SessionView *d_sv, int nslots, const Extent &ex, float4 *vmap_ext, long long vmap_pitch,
-                    int post_pyramid, const int *layouts, cudaStream_t st, uint8_t *rgb_ext, long long rgb_pitch) {
-    launch_zrange(d_sv, nslots, ex, st);
-    launch_march(d_sv, nslots, ex, vmap_ext, vmap_pitch, layouts, st, rgb_ext, rgb_pitch);
-    if (post_pyramid) launch_post(d_sv, nslots, ex, st);
+void launch_raycast(const SessionView *d_sv, const Extent &ex, const double pose[12], bool check_visibility,
+                    float4 *vmap_ext, long long vmap_pitch, const int *layouts, cudaStream_t st, uint8_t *rgb_ext,
+                    long long rgb_pitch) {
+    MapPose p;
+    for (int i = 0; i < 12; ++i) p.p[i] = pose[i];
+    const int cells = (ex.w / 8) * (ex.h / 8);
+    ray_begin_kernel<<<(cells + 255) / 256, 256, 0, st>>>(d_sv, p, check_visibility ? 1 : 0);
+    if (check_visibility) launch_visible_frustum(d_sv, 1, ex, st);
+    launch_zrange(d_sv, 1, ex, st);
+    launch_march(d_sv, 1, ex, vmap_ext, vmap_pitch, layouts, st, rgb_ext, rgb_pitch);
 }
 
 }  // namespace gbf

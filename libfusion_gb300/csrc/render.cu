@@ -54,7 +54,28 @@ __global__ void render_kernel(const float4 *vmap, long long vmap_pitch, const fl
         render_point(make_float3(v.x, v.y, v.z), make_float3(n.x, n.y, n.z), img);
 }
 
+// The session's model prediction, whose image set only the device knows.
+__global__ void render_session_kernel(const SessionView *__restrict__ svs, int textured, uchar4 *out, long long out_pitch) {
+    const SessionView &sv = svs[0];
+    const int w = sv.lv[0].w, x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+    if (x >= w) return;
+    const int set = sv.ts->idx, i = y * w + x;
+    const float4 v = sv.vmap[set][0][i], n = sv.nmap[set][0][i];
+    float3 img = make_float3(1.f, 1.f, 1.f);
+    if (textured) {
+        const uchar4 c = sv.rgb4[i];
+        img = make_float3((float)c.x / 255.f, (float)c.y / 255.f, (float)c.z / 255.f);
+    }
+    reinterpret_cast<uchar4 *>(reinterpret_cast<char *>(out) + y * out_pitch)[x] =
+        render_point(make_float3(v.x, v.y, v.z), make_float3(n.x, n.y, n.z), img);
+}
+
 }  // namespace
+
+void launch_render_session(const SessionView *d_sv, const Extent &ex, int textured, uchar4 *out, long long out_pitch,
+                           cudaStream_t st) {
+    render_session_kernel<<<dim3((ex.w + 127) / 128, ex.h), 128, 0, st>>>(d_sv, textured, out, out_pitch);
+}
 
 void launch_render(const float4 *vmap, long long vmap_pitch, const float4 *nmap, long long nmap_pitch,
                    const uint8_t *rgb, long long rgb_pitch, int rgb_stride, int w, int h, uchar4 *out,

@@ -104,7 +104,6 @@ ArenaLayout plan_arena(const gbf_config &c, const gbf_intrinsics &K) {
     a.in_rgb = take(P * 3);
     a.depth_raw = take(P * 4);
     a.rgb4 = take(P * 4);
-    a.nmap_ext = take(P * 16);
     a.fuse_px = take(P * 8);
     size_t w = K.width, h = K.height;
     for (int l = 0; l < c.num_levels; ++l) {
@@ -257,16 +256,6 @@ void to44(const double o[12], double T[16]) {
 
 __global__ void map_pose_kernel(TrackState *ts) { update_map_floats(ts); }
 
-gbf_status set_map_pose(gbf_session *s, const double T[16], cudaStream_t st) {
-    double p[12];
-    to34(T, p);
-    // pageable source: the copy is staged before the call returns
-    cudaError_t e = cudaMemcpyAsync(s->view.ts->map_pose, p, sizeof(p), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return cuda_error(e, "set pose");
-    map_pose_kernel<<<1, 1, 0, st>>>(s->view.ts);
-    return check_cuda("set pose");
-}
-
 // One frame for `nslots` slots.  With `ev` (kPhases + 1 events) the phase
 // boundaries are recorded: ingest, track, alloc+visible, integrate, z-range,
 // march, post.
@@ -307,7 +296,7 @@ void enqueue_second_half(const SessionView *d_sv, int nslots, const Extent &ex, 
     PhaseMarks mark(ev, st);
     launch_alloc_visible(d_sv, nslots, ex, st);
     mark(3, st);
-    launch_integrate(d_sv, nslots, ex, 1, layouts, st);
+    launch_integrate(d_sv, nslots, ex, layouts, st);
     mark(4, st);
     launch_zrange(d_sv, nslots, ex, st);
     mark(5, st);
@@ -327,7 +316,7 @@ void enqueue_frame(const SessionView *d_sv, int nslots, const Extent &ex, const 
 int kernels_per_frame(const Extent &ex, const int *layouts, int nslots, bool alone) {
     int nl = 0;
     for (int l = 0; l < kNumLayouts; ++l) nl += layouts[l];
-    return (1 + (ex.levels - 1) + 1) + track_launches(nslots, ex, alone) + 3 + nl + 2 + nl + post_launches(ex);
+    return (1 + (ex.levels - 1) + 1) + track_launches(nslots, ex, alone) + 2 + nl + 1 + nl + post_launches(ex);
 }
 
 }  // namespace
@@ -451,7 +440,6 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     v.in_rgb = reinterpret_cast<uint8_t *>(base + a.in_rgb);
     v.depth_raw = reinterpret_cast<float *>(base + a.depth_raw);
     v.rgb4 = reinterpret_cast<uchar4 *>(base + a.rgb4);
-    v.nmap_ext = reinterpret_cast<float4 *>(base + a.nmap_ext);
     v.fuse_px = reinterpret_cast<float2 *>(base + a.fuse_px);
     for (int l = 0; l < cfg->num_levels; ++l) {
         v.depth[l] = reinterpret_cast<float *>(base + a.depth[l]);
@@ -619,11 +607,9 @@ GBF_API gbf_status gbf_fuse(gbf_session *s, const float *depth, int64_t depth_pi
     if (!rows_aligned(depth, depth_pitch, 4) || (nmap && !rows_aligned(nmap, nmap_pitch, 16)))
         return set_error(GBF_ERR_INVALID_ARG, "gbf_fuse: depth rows must be 4-byte and normal rows 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    gbf_status r = set_map_pose(s, T, st);
-    if (r != GBF_OK) return r;
     FuseImport in{depth, depth_pitch, rgb, rgb_pitch, nmap, nmap_pitch};
-    launch_fuse_import(s->d_view, s->ex, in, st);
-    launch_fuse(s->d_view, 1, s->ex, nmap ? 2 : 0, s->layouts, st);
+    launch_fuse_import(s->d_view, s->ex, in, T, st);
+    launch_fuse(s->d_view, 1, s->ex, s->layouts, st);
     return check_cuda("gbf_fuse");
 }
 
@@ -633,9 +619,7 @@ GBF_API gbf_status gbf_raycast(gbf_session *s, const double T[16], float *vmap, 
     if (!rows_aligned(vmap, vmap_pitch, 16))
         return set_error(GBF_ERR_INVALID_ARG, "gbf_raycast: vertex-map rows must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    gbf_status r = set_map_pose(s, T, st);
-    if (r != GBF_OK) return r;
-    launch_raycast(s->d_view, 1, s->ex, reinterpret_cast<float4 *>(vmap), vmap_pitch, 0, s->layouts, st);
+    launch_raycast(s->d_view, s->ex, T, false, reinterpret_cast<float4 *>(vmap), vmap_pitch, s->layouts, st);
     return check_cuda("gbf_raycast");
 }
 
@@ -648,9 +632,7 @@ GBF_API gbf_status gbf_raycast_maps(gbf_session *s, const double T[16], float *v
     if (!rows_aligned(vmap, vmap_pitch, 16) || (nmap && !rows_aligned(nmap, nmap_pitch, 16)))
         return set_error(GBF_ERR_INVALID_ARG, "gbf_raycast_maps: vertex and normal rows must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    gbf_status r = set_map_pose(s, T, st);
-    if (r != GBF_OK) return r;
-    launch_raycast(s->d_view, 1, s->ex, reinterpret_cast<float4 *>(vmap), vmap_pitch, 0, s->layouts, st, rgb,
+    launch_raycast(s->d_view, s->ex, T, false, reinterpret_cast<float4 *>(vmap), vmap_pitch, s->layouts, st, rgb,
                    rgb_pitch);
     if (nmap)
         launch_nmap_of(reinterpret_cast<const float4 *>(vmap), vmap_pitch, reinterpret_cast<float4 *>(nmap),
@@ -666,10 +648,7 @@ GBF_API gbf_status gbf_raycast_check_visibility(gbf_session *s, const double T[1
     if (!rows_aligned(vmap, vmap_pitch, 16))
         return set_error(GBF_ERR_INVALID_ARG, "gbf_raycast_check_visibility: vertex-map rows must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    gbf_status r = set_map_pose(s, T, st);
-    if (r != GBF_OK) return r;
-    launch_visible_frustum(s->d_view, 1, s->ex, st);
-    launch_raycast(s->d_view, 1, s->ex, reinterpret_cast<float4 *>(vmap), vmap_pitch, 0, s->layouts, st);
+    launch_raycast(s->d_view, s->ex, T, true, reinterpret_cast<float4 *>(vmap), vmap_pitch, s->layouts, st);
     return check_cuda("gbf_raycast_check_visibility");
 }
 
@@ -697,14 +676,7 @@ GBF_API gbf_status gbf_session_render(gbf_session *s, int32_t textured, uint8_t 
     if (!rows_aligned(out, out_pitch, 4))
         return set_error(GBF_ERR_INVALID_ARG, "gbf_session_render: output rows must be 4-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    // the reference frame's maps: the model prediction of the last raycast
-    int idx = 0;
-    cudaError_t e = cudaMemcpyAsync(&idx, &s->view.ts->idx, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_error(e, "gbf_session_render");
-    launch_render(s->view.vmap[idx][0], W * 16LL, s->view.nmap[idx][0], W * 16LL,
-                  textured ? reinterpret_cast<const uint8_t *>(s->view.rgb4) : nullptr, W * 4LL, 4, W, H,
-                  reinterpret_cast<uchar4 *>(out), out_pitch, st);
+    launch_render_session(s->d_view, s->ex, textured ? 1 : 0, reinterpret_cast<uchar4 *>(out), out_pitch, st);
     return check_cuda("gbf_session_render");
 }
 
