@@ -137,14 +137,18 @@ __device__ __forceinline__ bool icp_row(const LevelIn &K, const M34 &T, const fl
 // divide at the same place (1e-4f and 1e-5f lie just below 1e-4 and 1e-5), and
 // one thread of a CTA makes the product (photo_huber).
 struct PhotoConst {
-    float stddev, huber, inv;
+    float stddev, huber;
+    float div, inv;  // res / stddev as div_rn_by(res, div, inv)
     bool normalise, robust;
 };
 __device__ __forceinline__ float photo_huber(float stddev) { return (float)(1.345 * (double)stddev); }
 __device__ __forceinline__ PhotoConst photo_const(float stddev, float huber) {
     PhotoConst c;
     c.stddev = stddev;
+    // six rows leave stddev infinite and the residuals zero: 0 * res, remainder res,
+    // where an infinite div would make the remainder NaN
     c.inv = __frcp_rn(stddev);
+    c.div = isinf(stddev) ? 0.f : stddev;
     c.normalise = stddev > 1e-4f;
     c.robust = stddev > 1e-5f;
     c.huber = huber;
@@ -809,7 +813,7 @@ __device__ __forceinline__ void pixel_rows(const LevelIn &K, const M34 &T, const
         const float lx = (dx * K.fx) * zi, ly = (dy * K.fy) * zi;
         const float lz = (-(lx * p.x + ly * p.y)) * zi;
         float res = ic - il;
-        if (pc.normalise) res = div_rn_by(res, pc.stddev, pc.inv);
+        if (pc.normalise) res = div_rn_by(res, pc.div, pc.inv);
         float wt = 1.f;
         if (fabsf(res) > pc.huber && pc.robust) wt = sqrtf(pc.huber / fabsf(res));
         const float3 x = cross3(p, make_float3(lx, ly, lz));

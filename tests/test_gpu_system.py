@@ -800,6 +800,46 @@ def test_tracking_run_matches_launches_per_iteration(gbf, w, h, levels, iters, p
     batch.close()
 
 
+def test_tracking_run_with_six_photometric_rows(gbf):
+    """Six photometric rows leave no degree of freedom: the residuals' deviation is
+    infinite, the next iteration's residuals are zero (x / inf).  The run of a session
+    alone gives what the launches per iteration give."""
+    import torch
+    L = gbf
+    w, h = 320, 240
+    K = H.intrinsics(L, w, h)
+    d, _, T = H.frames(L, K, 1, seed=4)[0]
+    c = np.full((h, w, 3), 100, np.uint8)
+    for x, y in ((140, 110), (160, 120), (180, 130)):
+        c[y, x] = 120  # a gradient above 2 at (x - 1, y) and (x, y - 1) only
+
+    def run(iters, n):
+        cfg = H.small_config(L, 2, num_levels=1, max_iterations=[iters, 0, 0, 0, 0], num_blocks=1 << 14,
+                             num_buckets=1 << 16)
+        ss = [L.System(K, cfg) for _ in range(n)]
+        batch = L.FusionBatch(n)
+        batch.set_groups(n)
+        for i, s in enumerate(ss):
+            s.set_pose(T)
+            batch.set(i, s)
+        for k in range(2):
+            for s in ss:
+                s.stage(H.cuda(d), H.cuda(c + np.uint8(5 * k)))
+            torch.cuda.synchronize()
+            batch.process([True] * n)
+            torch.cuda.synchronize()
+        out = ss[0].get_camera_pose(), ss[0].stats()
+        batch.close()
+        return out
+    assert run(1, 1)[1].track.rgb_inliers == 6  # the case is what it says
+    for iters in (2, 4):
+        (p, x), (q, y) = run(iters, 1), run(iters, 2)
+        assert np.isfinite(p).all() and np.array_equal(p, q)
+        assert (x.track.success, x.track.iterations) == (y.track.success, y.track.iterations)
+        for f in ("icp_error", "rgb_error", "icp_inliers", "rgb_inliers"):
+            assert np.array_equal(getattr(x.track, f), getattr(y.track, f), equal_nan=True), f
+
+
 def test_tracking_runs_on_concurrent_streams(gbf):
     """Sessions driven on streams of their own, nothing waiting between them: their
     cooperative tracking runs, each of which takes the whole chip, beside each
