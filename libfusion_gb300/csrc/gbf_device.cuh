@@ -106,8 +106,10 @@ __device__ __forceinline__ M34 load_m34(const float *m) {
 // 510, 0 < b <= 510, nonzero |a / b| far above the subnormal range; a is never
 // -0 there, which would need both products -0, so a zero quotient keeps its
 // sign; tests/test_arith_proofs.py checks the steps in exact arithmetic on these
-// ranges).  For two quotients sharing b (the voxel and photometric
-// projections) it measured slower than two divisions.
+// ranges), and for the photometric projection, whose reciprocal the row needs anyway
+// (quotients too small for the steps to be exact fall on the image's principal point
+// either way).  For the voxel projection's two quotients it measured slower than two
+// divisions.
 __device__ __forceinline__ float div_rn_by(float a, float b, float y) {
     const float q0 = __fmul_rn(a, y);
     const float q1 = __fmaf_rn(__fmaf_rn(-q0, b, a), y, q0);
@@ -115,9 +117,8 @@ __device__ __forceinline__ float div_rn_by(float a, float b, float y) {
 }
 
 // Vector3 helpers in the reference's order (include/math/vector_type.h)
-__device__ __forceinline__ float norm3(float x, float y, float z) {
-    return sqrtf((x * x + y * y) + z * z);
-}
+__device__ __forceinline__ float norm3_sq(float x, float y, float z) { return (x * x + y * y) + z * z; }
+__device__ __forceinline__ float norm3(float x, float y, float z) { return sqrtf(norm3_sq(x, y, z)); }
 __device__ __forceinline__ float3 cross3(float3 a, float3 b) {
     return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }

@@ -5,6 +5,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include "../../include/gbfusion.h"
@@ -72,6 +73,21 @@ void launch_nmap_of(const float4 *vmap, long long vmap_pitch, float4 *nmap, long
 // kernel launches of one launch_post
 int post_launches(const Extent &ex);
 void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
+
+// The ICP gates sine < angle and length <= dist (pose_estimator.cu:200) as bounds on
+// the squares whose rounded roots they compare: the root rounded to nearest is
+// monotonic, so exactly the squares below angle2, and those up to dist2, pass.  The
+// two roots per pixel and iteration cost 2.5% of a 64-session tracking phase.
+inline void square_gates(SessionView &v, float dist, float angle) {
+    float a = angle > 0.f ? angle * angle : 0.f;  // the least float whose root is not below angle
+    while (a > 0.f && sqrtf(nextafterf(a, 0.f)) >= angle) a = nextafterf(a, 0.f);
+    while (a < INFINITY && sqrtf(a) < angle) a = nextafterf(a, INFINITY);
+    float d = dist >= 0.f ? dist * dist : -1.f;  // the greatest float whose root is not above dist
+    while (d > 0.f && sqrtf(d) > dist) d = nextafterf(d, 0.f);
+    while (d >= 0.f && d < INFINITY && sqrtf(nextafterf(d, INFINITY)) <= dist) d = nextafterf(d, INFINITY);
+    v.icp_angle2 = a;
+    v.icp_dist2 = d;
+}
 
 // ---- tracking (tracking.cu) -----------------------------------------------------
 // mode 0: full Gauss-Newton (gbf_track / process frame), stops at the schedule end

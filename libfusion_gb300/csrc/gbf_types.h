@@ -96,7 +96,8 @@ struct SessionView {
     int cap_mask;          // cap - 1 when cap is a power of two, else -1
     float voxel, inv_voxel, tau, inv_tau, step_scale;
     float zmin_u, zmax_u, zmin_r, zmax_r, block_metric;
-    float w_icp, w_rgb, icp_dist, icp_angle;
+    float w_icp, w_rgb;
+    float icp_dist2, icp_angle2;  // the gates on squared lengths (square_gates)
     int bilateral;
     int levels;
     int max_iter[kMaxLevels];

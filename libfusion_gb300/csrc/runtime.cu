@@ -420,8 +420,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     v.block_metric = (float)kBlockSide * cfg->voxel_size;        // MapState::block_size_metric
     v.w_icp = cfg->w_icp;
     v.w_rgb = cfg->w_rgb;
-    v.icp_dist = cfg->icp_dist_thresh;
-    v.icp_angle = cfg->icp_angle_thresh;
+    square_gates(v, cfg->icp_dist_thresh, cfg->icp_angle_thresh);
     v.bilateral = cfg->bilateral;
     v.levels = cfg->num_levels;
     fill_levels(*cfg, *K, v);

@@ -1,5 +1,6 @@
 """The Gauss-Newton step's solve, exponential and composition (csrc/gn_step.cuh)
 against exact rational arithmetic."""
+import ctypes as C
 import subprocess
 from fractions import Fraction as F
 from pathlib import Path
@@ -105,3 +106,40 @@ def test_step_with_infinities_ends(step):
     assert np.array_equal(x[0], np.ones(6))
     assert np.array_equal(x[1], [1, 1, 0, 1, 1, 1])  # b / infinity
     assert np.isnan(x[2]).any()
+
+
+@pytest.mark.parametrize("gate", ["dist", "angle"])
+def test_icp_gates_at_their_thresholds(gbf, gate):
+    """sine < angle and dist <= dist_max hold for the rounded square roots: thresholds
+    at, next below and next above the roots of pixels, zero, negative, tiny, huge,
+    infinite and NaN ones count the pixels that the comparison of the roots counts."""
+    import torch
+    L = gbf
+    w, h = 64, 16
+    f = np.float32
+    rng = np.random.default_rng(3)
+    py, px = np.mgrid[0:h, 0:w].astype(f)
+    ref = np.stack([px, py, np.ones_like(px), np.ones_like(px)], -1)  # fx = z = 1: pixel (x, y)
+    cur, nr, nc = ref.copy(), np.zeros_like(ref), np.zeros_like(ref)
+    cur[..., :3] += rng.normal(0, 10.0 ** rng.uniform(-4, 3, (h, w, 1)), (h, w, 3)).astype(f)
+    nr[..., :3], nc[..., :3] = rng.normal(size=(2, h, w, 3)).astype(f) * f(0.6)
+    cur[0, :8], nc[0, :8] = ref[0, :8], nr[0, :8]  # roots of zero
+    a, b = nc, nr
+    cr = [a[..., i] * b[..., j] - a[..., j] * b[..., i] for i, j in ((1, 2), (2, 0), (0, 1))]
+    dd = [ref[..., i] - cur[..., i] for i in range(3)]
+    dist, sine = (np.sqrt((v[0] * v[0] + v[1] * v[1]) + v[2] * v[2]).ravel() for v in (dd, cr))
+    assert dist.dtype == f and sine.dtype == f
+    grey = np.full((h, w), 50, f)
+    imgs = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (ref, nr, grey, cur, nc, grey, 0 * grey, 0 * grey)]
+    roots = dist if gate == "dist" else sine
+    picks = roots[rng.integers(0, roots.size, 24)]
+    tests = np.concatenate([picks, np.nextafter(picks, f(0)), np.nextafter(picks, f(np.inf)),
+                            np.array([0, -0.0, -1, 1e-45, 1e-30, 1e-20, 1e30, np.inf, np.nan], f)])
+    out = torch.empty(58, dtype=torch.float64, device="cuda")
+    for t in tests:
+        d_max, angle = (t, f(np.inf)) if gate == "dist" else (f(np.inf), t)
+        inp = L._lib.ReduceInputs(w, h, 1.0, 1.0, 0.0, 0.0, *[x.data_ptr() for x in imgs], float(d_max), float(angle))
+        L._lib.call("gbf_reduce_noalloc", C.byref(inp), L._lib.mat16(np.eye(4)), 0.0, out.data_ptr(),
+                    torch.cuda.current_stream().cuda_stream)
+        want = np.count_nonzero((sine < angle) & (dist <= d_max))
+        assert int(out.cpu()[28]) == want, (gate, t)
