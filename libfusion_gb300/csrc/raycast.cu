@@ -238,13 +238,27 @@ __device__ __noinline__ float interp_spanning(const SV sv, int i000, int x0, int
     return trilinear(fx, fy, fz, c000, c100, c010, c110, c001, c101, c011, c111);
 }
 
+// True when `p` holds on every lane that runs this together (one asm: nothing can part
+// the lanes between the two).  Which lanes do is up to the scheduler, so a result must
+// not depend on it.
+__device__ __forceinline__ bool all_converged(bool p) {
+    unsigned all;
+    asm volatile("{\n .reg .pred a, b;\n .reg .b32 m;\n setp.ne.u32 a, %1, 0;\n activemask.b32 m;\n"
+                 " vote.sync.all.pred b, a, m;\n selp.u32 %0, 1, 0, b;\n}\n"
+                 : "=r"(all)
+                 : "r"((unsigned)p));
+    return all != 0;
+}
+
 // read_sdf_interped (ray_tracing.cu:307-339) at a point whose floor (x0, y0, z0)
 // and its block id are at hand; c000: the corner there, observed.  The reference reads the
 // corners at pt + (0|1, 0|1, 0|1) and floors each sum: floor(p + 1) is floor(p) + 1
 // unless p + 1 rounds up to the next integer, which a comparison tells.  When the
 // eight corners lie in one block (about 2/3 of the samples) they are read by
-// offset from it, all loads issued together.  NaN unless all corners are observed
-// (the reference's sum over NaN corners).
+// offset from it, all loads issued together -- unless a lane beside needs the spanning
+// read, which then serves them all (the same eight voxels; a warp with both paid for both:
+// march of 64 VGA sessions 2.73 -> 2.58 ms, the spanning read alone for all 2.70).  NaN
+// unless all corners are observed (the reference's sum over NaN corners).
 template <int LAYOUT, class SV>
 __device__ __forceinline__ float read_sdf_interped(const SV &sv, int id, int li, float px, float py, float pz, int x0,
                                                    int y0, int z0, float c000, bool &valid) {
@@ -254,7 +268,7 @@ __device__ __forceinline__ float read_sdf_interped(const SV &sv, int id, int li,
     // li + 73 carries out of a 3-bit field where that coordinate is 7
     const bool inside = (((li + 73) ^ li ^ 73) & 0x248) == 0;
     float v;
-    if (plain && inside) {
+    if (all_converged(plain && inside)) {
         const int i = id * kBlockVoxels + li;
         bool v1, v2, v3, v4, v5, v6, v7;
         const float c100 = sdf_raw<LAYOUT>(sv, i + 1, v1), c010 = sdf_raw<LAYOUT>(sv, i + 8, v2);
