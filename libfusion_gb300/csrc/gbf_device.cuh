@@ -116,6 +116,15 @@ __device__ __forceinline__ float div_rn_by(float a, float b, float y) {
     return __fmaf_rn(__fmaf_rn(-q1, b, a), y, q1);
 }
 
+// First statement of every kernel that launch_kernel may chain: lets the next launch of
+// the stream start its CTAs once all of this one's run, and waits until the launches
+// before have ended and their writes are seen (which implies that those before them
+// have).  Nothing above it may touch memory that a kernel writes.  Without a chained
+// launch both do nothing.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;\n" ::: "memory");
+}
+
 // Vector3 helpers in the reference's order (include/math/vector_type.h)
 __device__ __forceinline__ float norm3_sq(float x, float y, float z) { return (x * x + y * y) + z * z; }
 __device__ __forceinline__ float norm3(float x, float y, float z) { return sqrtf(norm3_sq(x, y, z)); }

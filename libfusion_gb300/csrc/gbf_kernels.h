@@ -20,7 +20,28 @@ struct Extent {
     int levels;      // largest level count
     int max_iter[kMaxLevels];
     int ray_tw;      // raycast tile width (4, 8, 16 or 32 of a 64-pixel tile); 0 = 8
+    int chain;       // 1: a session's own launches, one after the other on a stream (launch_kernel)
 };
+
+// A launch that, when chained, is set up while the launch before it in the stream
+// still runs (programmatic dependent launch; the kernel waits in chain_begin).  A frame
+// of one session is a chain of a dozen launches of 4 to 150 us, with 2.0 to 2.5 us between two
+// plain ones and 0.4 between chained ones.  A batch's ticks launch plainly: captured,
+// their launches are 0.5 us apart, and the CTAs that wait early would take the places of the
+// other branch's.
+template <class... P, class... A>
+inline void launch_kernel(void (*kernel)(P...), dim3 grid, int threads, bool chain, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = chain ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
 
 inline int ray_tile_width(const Extent &ex) {
     return (ex.ray_tw == 4 || ex.ray_tw == 16 || ex.ray_tw == 32) ? ex.ray_tw : 8;

@@ -38,6 +38,7 @@ __device__ __forceinline__ int set_index(const SessionView &sv, int sel) {
 }
 
 __global__ void __launch_bounds__(kTileW *kTileH) ingest_l0_kernel(const SessionView *__restrict__ svs, IngestArgs a) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     const int W = sv.lv[0].w, H = sv.lv[0].h;
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(kTileW *kTileH) ingest_l0_kernel(const Session
 }
 
 __global__ void pyr_down_kernel(const SessionView *__restrict__ svs, int set_sel, int level) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active || level >= sv.levels) return;
     const int w = sv.lv[level].w, h = sv.lv[level].h;
@@ -165,6 +167,7 @@ __device__ __forceinline__ void fuse_weight(const SessionView &sv, int i, float4
 }
 
 __global__ void __launch_bounds__(256, 8) level_maps_kernel(const SessionView *__restrict__ svs, int set_sel, int tiles_per_level0) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     // flatten the levels: level l owns ceil(P_l / blockDim) CTAs
@@ -213,11 +216,11 @@ __global__ void __launch_bounds__(256, 8) level_maps_kernel(const SessionView *_
 
 void launch_ingest(const SessionView *d_sv, int nslots, const Extent &ex, const IngestArgs &a, cudaStream_t st) {
     const int tiles = ((ex.w + kTileW - 1) / kTileW) * ((ex.h + kTileH - 1) / kTileH);
-    ingest_l0_kernel<<<dim3(tiles, nslots), kTileW * kTileH, 0, st>>>(d_sv, a);
+    launch_kernel(ingest_l0_kernel, dim3(tiles, nslots), kTileW * kTileH, ex.chain, st, d_sv, a);
     int w = ex.w, h = ex.h;
     for (int l = 1; l < ex.levels; ++l) {
         w /= 2; h /= 2;
-        pyr_down_kernel<<<dim3((w * h + 255) / 256, nslots), 256, 0, st>>>(d_sv, a.set_sel, l);
+        launch_kernel(pyr_down_kernel, dim3((w * h + 255) / 256, nslots), 256, ex.chain, st, d_sv, a.set_sel, l);
     }
     int total = 0;
     w = ex.w; h = ex.h;
@@ -225,7 +228,7 @@ void launch_ingest(const SessionView *d_sv, int nslots, const Extent &ex, const 
         total += (w * h + 255) / 256;
         w /= 2; h /= 2;
     }
-    level_maps_kernel<<<dim3(total, nslots), 256, 0, st>>>(d_sv, a.set_sel, 0);
+    launch_kernel(level_maps_kernel, dim3(total, nslots), 256, ex.chain, st, d_sv, a.set_sel, 0);
 }
 
 }  // namespace gbf

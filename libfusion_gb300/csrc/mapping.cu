@@ -36,6 +36,7 @@ constexpr int kSetSize = 1024;        // shared-memory key set per CTA
 // pixel.  System frames get the same values from level_maps_kernel.  (1e-2f lies
 // just below the reference's double 1e-2: the floats below that are those below 1e-2f, and 1e-2f.)
 __global__ void fuse_import_kernel(const SessionView *__restrict__ svs, FuseImport in, MapPose pose) {
+    chain_begin();
     const SessionView &sv = svs[0];
     if (blockIdx.x == 0 && threadIdx.x < 32) store_map_pose(sv.ts, pose);
     const int W = sv.lv[0].w, H = sv.lv[0].h;
@@ -92,6 +93,7 @@ __device__ __forceinline__ int3 pixel_block(const SessionView &sv, const M34 &T,
 }
 
 __global__ void __launch_bounds__(kAllocTile *kAllocTile) alloc_kernel(const SessionView *svs) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     const int W = sv.lv[0].w, H = sv.lv[0].h;
@@ -185,6 +187,7 @@ __device__ __forceinline__ bool block_in_frustum(const SessionView &sv, const M3
 // ray_tracing.cu:778-807 with VisibleEntryEvaluateFunctor, :681-710).
 template <bool TOUCHED>
 __global__ void __launch_bounds__(256, 6) visible_kernel(const SessionView *svs) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     __shared__ M34 Tcw;
@@ -213,6 +216,7 @@ constexpr int kIntThreads = 128;  // threads per integration CTA (512 / kIntThre
 
 template <int LAYOUT>
 __global__ void __launch_bounds__(kIntThreads, 16) integrate_kernel(const SessionView *__restrict__ svs) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active || sv.layout != LAYOUT) return;
     __shared__ M34 Tcw_s;
@@ -313,7 +317,7 @@ void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImp
     const int n = ex.w * ex.h;
     MapPose p;
     for (int i = 0; i < 12; ++i) p.p[i] = pose[i];
-    fuse_import_kernel<<<(n + 255) / 256, 256, 0, st>>>(d_sv, in, p);
+    launch_kernel(fuse_import_kernel, (n + 255) / 256, 256, ex.chain, st, d_sv, in, p);
 }
 
 // CTAs per session of the visible-block pass (grid-stride over the allocated
@@ -323,14 +327,14 @@ constexpr int kVisCtas = 152;
 
 void launch_alloc_visible(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
     const int tiles = ((ex.w + kAllocTile - 1) / kAllocTile) * ((ex.h + kAllocTile - 1) / kAllocTile);
-    alloc_kernel<<<dim3(tiles, nslots), kAllocTile * kAllocTile, 0, st>>>(d_sv);
+    launch_kernel(alloc_kernel, dim3(tiles, nslots), kAllocTile * kAllocTile, ex.chain, st, d_sv);
     const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
-    visible_kernel<true><<<dim3(gv, nslots), 256, 0, st>>>(d_sv);
+    launch_kernel(visible_kernel<true>, dim3(gv, nslots), 256, ex.chain, st, d_sv);
 }
 
 void launch_visible_frustum(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
     const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
-    visible_kernel<false><<<dim3(gv, nslots), 256, 0, st>>>(d_sv);
+    launch_kernel(visible_kernel<false>, dim3(gv, nslots), 256, ex.chain, st, d_sv);
 }
 
 void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st) {
@@ -340,9 +344,10 @@ void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, con
     // Many sessions fill the chip with 8 each, and a CTA's prologue then counts
     // (64 sessions: 1.77 ms with 8, 1.80 with 16, 1.88 with 32, 2.03 with 64).
     const int gi = 152 * max(8, 32 / nslots);
-    if (layouts[GBF_VOXEL_REF]) integrate_kernel<GBF_VOXEL_REF><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv);
-    if (layouts[GBF_VOXEL_HALF]) integrate_kernel<GBF_VOXEL_HALF><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv);
-    if (layouts[GBF_VOXEL_SNORM]) integrate_kernel<GBF_VOXEL_SNORM><<<dim3(gi, nslots), kIntThreads, 0, st>>>(d_sv);
+    const dim3 g(gi, nslots);
+    if (layouts[GBF_VOXEL_REF]) launch_kernel(integrate_kernel<GBF_VOXEL_REF>, g, kIntThreads, ex.chain, st, d_sv);
+    if (layouts[GBF_VOXEL_HALF]) launch_kernel(integrate_kernel<GBF_VOXEL_HALF>, g, kIntThreads, ex.chain, st, d_sv);
+    if (layouts[GBF_VOXEL_SNORM]) launch_kernel(integrate_kernel<GBF_VOXEL_SNORM>, g, kIntThreads, ex.chain, st, d_sv);
 }
 
 void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st) {

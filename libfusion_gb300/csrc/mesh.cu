@@ -244,6 +244,7 @@ __host__ __device__ __forceinline__ int mesh_chunk(int pool) {
 
 template <int LAYOUT>
 __global__ void __launch_bounds__(kMeshThreads, 16) mesh_count_kernel(const SessionView *__restrict__ svs, int mode, int *counts) {
+    chain_begin();
     const SessionView &sv = svs[0];
     const int n = min(sv.ctr[C_NUSED], sv.pool), chunk = mesh_chunk(sv.pool);
     __shared__ MeshBits m;
@@ -273,6 +274,7 @@ __global__ void __launch_bounds__(kMeshThreads, 16) mesh_count_kernel(const Sess
 // C_MESH_TRIS.  A CTA per chunk: the sums of the chunks before it, then its own
 // counts, 1024 at a time.  (One CTA over all the blocks took 6.3 us for 6,000.)
 __global__ void __launch_bounds__(1024) mesh_scan_kernel(const SessionView *__restrict__ svs, int *counts) {
+    chain_begin();
     const SessionView &sv = svs[0];
     const int n = min(sv.ctr[C_NUSED], sv.pool), chunk = mesh_chunk(sv.pool);
     const int first = blockIdx.x * chunk, end = min(n, first + chunk);
@@ -340,6 +342,7 @@ struct MeshEmit {
 template <int LAYOUT, int MODE>
 __global__ void __launch_bounds__(kMeshThreads, 10) mesh_emit_kernel(const SessionView *__restrict__ svs, const int *offsets,
                                                                      float *vtx, void *attr, long long max_tris) {
+    chain_begin();
     const SessionView &sv = svs[0];
     const int n = min(sv.ctr[C_NUSED], sv.pool);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -450,14 +453,17 @@ void launch_mesh_layout(const SessionView *d_sv, const Extent &ex, int mode, flo
                         int *counts, cudaStream_t st) {
     // grid-stride over the blocks, whose count only the device knows
     const int g = min(max(ex.max_pool, 1), 152 * 16), chunks = (ex.max_pool + mesh_chunk(ex.max_pool) - 1) / mesh_chunk(ex.max_pool);
-    mesh_count_kernel<LAYOUT><<<g, kMeshThreads, 0, st>>>(d_sv, mode, counts);
-    mesh_scan_kernel<<<max(chunks, 1), 1024, 0, st>>>(d_sv, counts);
+    launch_kernel(mesh_count_kernel<LAYOUT>, g, kMeshThreads, ex.chain, st, d_sv, mode, counts);
+    launch_kernel(mesh_scan_kernel, max(chunks, 1), 1024, ex.chain, st, d_sv, counts);
     if (mode == GBF_MESH_VERTEX)
-        mesh_emit_kernel<LAYOUT, GBF_MESH_VERTEX><<<g, kMeshThreads, 0, st>>>(d_sv, counts, vtx, attr, max_tris);
+        launch_kernel(mesh_emit_kernel<LAYOUT, GBF_MESH_VERTEX>, g, kMeshThreads, ex.chain, st, d_sv, counts, vtx, attr,
+                      max_tris);
     else if (mode == GBF_MESH_NORMAL)
-        mesh_emit_kernel<LAYOUT, GBF_MESH_NORMAL><<<g, kMeshThreads, 0, st>>>(d_sv, counts, vtx, attr, max_tris);
+        launch_kernel(mesh_emit_kernel<LAYOUT, GBF_MESH_NORMAL>, g, kMeshThreads, ex.chain, st, d_sv, counts, vtx, attr,
+                      max_tris);
     else
-        mesh_emit_kernel<LAYOUT, GBF_MESH_COLOUR><<<g, kMeshThreads, 0, st>>>(d_sv, counts, vtx, attr, max_tris);
+        launch_kernel(mesh_emit_kernel<LAYOUT, GBF_MESH_COLOUR>, g, kMeshThreads, ex.chain, st, d_sv, counts, vtx, attr,
+                      max_tris);
 }
 
 }  // namespace

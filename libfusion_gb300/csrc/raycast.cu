@@ -41,6 +41,7 @@ namespace gbf {
 namespace {
 
 __global__ void ray_begin_kernel(const SessionView *__restrict__ svs, MapPose pose, int check_visibility) {
+    chain_begin();
     const SessionView &sv = svs[0];
     if (blockIdx.x == 0 && threadIdx.x < 32) store_map_pose(sv.ts, pose);
     if (check_visibility && blockIdx.x == 0 && threadIdx.x == 32) sv.ctr[C_NVIS] = 0;  // counted again by visible_kernel
@@ -122,6 +123,7 @@ __device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tc
 // the second the allocated ones (slices, and the neighbour lists of the blocks
 // that rays may meet).
 __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__restrict__ svs) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     __shared__ M34 Tcw;
@@ -306,6 +308,7 @@ template <int LAYOUT, bool RGB>
 __global__ void __launch_bounds__(kRayThreads, 24) raycast_kernel(const SessionView *__restrict__ svs, float4 *vmap_ext,
                                                                   long long vmap_pitch, int tw, uint8_t *rgb_ext,
                                                                   long long rgb_pitch) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active || sv.layout != LAYOUT) return;
     // the reference skips the raycast when nothing was visible or renderable
@@ -449,6 +452,7 @@ __global__ void __launch_bounds__(kRayThreads, 24) raycast_kernel(const SessionV
 
 // cv::cuda::resize(vmap, 0.5): 2x2 mean of every channel
 __global__ void vmap_down_kernel(const SessionView *__restrict__ svs, int level) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active || level >= sv.levels) return;
     const int w = sv.lv[level].w, h = sv.lv[level].h, pw = sv.lv[level - 1].w;
@@ -500,6 +504,7 @@ __device__ __forceinline__ float4 mean4(const float4 a, const float4 b, const fl
 // writing and re-reading every level.
 constexpr int kPostTile = 32;
 __global__ void __launch_bounds__(256) post_pyramid_kernel(const SessionView *__restrict__ svs) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     const int w0 = sv.lv[0].w, h0 = sv.lv[0].h;
@@ -578,6 +583,7 @@ __global__ void __launch_bounds__(256) post_pyramid_kernel(const SessionView *__
 
 __global__ void nmap_of_kernel(const float4 *vmap, long long vmap_pitch, float4 *nmap, long long nmap_pitch, int w,
                                int h) {
+    chain_begin();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= w || y >= h) return;
     // the pitches are multiples of 16 bytes (checked by the caller)
@@ -586,6 +592,7 @@ __global__ void nmap_of_kernel(const float4 *vmap, long long vmap_pitch, float4 
 }
 
 __global__ void nmap_all_kernel(const SessionView *__restrict__ svs) {
+    chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     int b = blockIdx.x, level = 0;
@@ -608,7 +615,7 @@ __global__ void nmap_all_kernel(const SessionView *__restrict__ svs) {
 void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
     // two halves of up to three resident CTAs per SM each; fewer of many sessions, whose CTAs loop
     const int gz = min(max((ex.max_pool + 31) / 32, 1), max(152, 152 * 3 / nslots));
-    zrange_kernel<<<dim3(2 * gz, nslots), 256, 0, st>>>(d_sv);
+    launch_kernel(zrange_kernel, dim3(2 * gz, nslots), 256, ex.chain, st, d_sv);
 }
 
 void launch_march(const SessionView *d_sv, int nslots, const Extent &ex, float4 *vmap_ext, long long vmap_pitch,
@@ -616,29 +623,23 @@ void launch_march(const SessionView *d_sv, int nslots, const Extent &ex, float4 
     const int tw = ray_tile_width(ex), th = kRayThreads / tw;
     // every slot's tiles fit: a smaller frame has fewer tiles per row and per column
     const dim3 g(((ex.w + tw - 1) / tw) * ((ex.h + th - 1) / th), nslots);
+    const auto march = [&](auto *kernel) {
+        launch_kernel(kernel, g, kRayThreads, ex.chain, st, d_sv, vmap_ext, vmap_pitch, tw, rgb_ext, rgb_pitch);
+    };
     if (rgb_ext) {
-        if (layouts[GBF_VOXEL_REF])
-            raycast_kernel<GBF_VOXEL_REF, true><<<g, kRayThreads, 0, st>>>(d_sv, vmap_ext, vmap_pitch, tw, rgb_ext,
-                                                                           rgb_pitch);
-        if (layouts[GBF_VOXEL_HALF])
-            raycast_kernel<GBF_VOXEL_HALF, true><<<g, kRayThreads, 0, st>>>(d_sv, vmap_ext, vmap_pitch, tw, rgb_ext,
-                                                                            rgb_pitch);
-        if (layouts[GBF_VOXEL_SNORM])
-            raycast_kernel<GBF_VOXEL_SNORM, true><<<g, kRayThreads, 0, st>>>(d_sv, vmap_ext, vmap_pitch, tw, rgb_ext,
-                                                                             rgb_pitch);
+        if (layouts[GBF_VOXEL_REF]) march(raycast_kernel<GBF_VOXEL_REF, true>);
+        if (layouts[GBF_VOXEL_HALF]) march(raycast_kernel<GBF_VOXEL_HALF, true>);
+        if (layouts[GBF_VOXEL_SNORM]) march(raycast_kernel<GBF_VOXEL_SNORM, true>);
         return;
     }
-    if (layouts[GBF_VOXEL_REF])
-        raycast_kernel<GBF_VOXEL_REF, false><<<g, kRayThreads, 0, st>>>(d_sv, vmap_ext, vmap_pitch, tw, nullptr, 0);
-    if (layouts[GBF_VOXEL_HALF])
-        raycast_kernel<GBF_VOXEL_HALF, false><<<g, kRayThreads, 0, st>>>(d_sv, vmap_ext, vmap_pitch, tw, nullptr, 0);
-    if (layouts[GBF_VOXEL_SNORM])
-        raycast_kernel<GBF_VOXEL_SNORM, false><<<g, kRayThreads, 0, st>>>(d_sv, vmap_ext, vmap_pitch, tw, nullptr, 0);
+    if (layouts[GBF_VOXEL_REF]) march(raycast_kernel<GBF_VOXEL_REF, false>);
+    if (layouts[GBF_VOXEL_HALF]) march(raycast_kernel<GBF_VOXEL_HALF, false>);
+    if (layouts[GBF_VOXEL_SNORM]) march(raycast_kernel<GBF_VOXEL_SNORM, false>);
 }
 
 void launch_nmap_of(const float4 *vmap, long long vmap_pitch, float4 *nmap, long long nmap_pitch, int w, int h,
                     cudaStream_t st) {
-    nmap_of_kernel<<<dim3((w + 127) / 128, h), 128, 0, st>>>(vmap, vmap_pitch, nmap, nmap_pitch, w, h);
+    launch_kernel(nmap_of_kernel, dim3((w + 127) / 128, h), 128, true, st, vmap, vmap_pitch, nmap, nmap_pitch, w, h);
 }
 
 int post_launches(const Extent &ex) { return ex.levels <= 3 ? 1 : ex.levels; }
@@ -646,16 +647,16 @@ int post_launches(const Extent &ex) { return ex.levels <= 3 ? 1 : ex.levels; }
 void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
     if (ex.levels <= 3) {
         const int tiles = ((ex.w + kPostTile - 1) / kPostTile) * ((ex.h + kPostTile - 1) / kPostTile);
-        post_pyramid_kernel<<<dim3(tiles, nslots), 256, 0, st>>>(d_sv);
+        launch_kernel(post_pyramid_kernel, dim3(tiles, nslots), 256, ex.chain, st, d_sv);
         return;
     }
     int w = ex.w, h = ex.h, total = (w * h + 255) / 256;
     for (int l = 1; l < ex.levels; ++l) {
         w /= 2; h /= 2;
-        vmap_down_kernel<<<dim3((w * h + 255) / 256, nslots), 256, 0, st>>>(d_sv, l);
+        launch_kernel(vmap_down_kernel, dim3((w * h + 255) / 256, nslots), 256, ex.chain, st, d_sv, l);
         total += (w * h + 255) / 256;
     }
-    nmap_all_kernel<<<dim3(total, nslots), 256, 0, st>>>(d_sv);
+    launch_kernel(nmap_all_kernel, dim3(total, nslots), 256, ex.chain, st, d_sv);
 }
 
 void launch_raycast(const SessionView *d_sv, const Extent &ex, const double pose[12], bool check_visibility,
@@ -664,7 +665,7 @@ void launch_raycast(const SessionView *d_sv, const Extent &ex, const double pose
     MapPose p;
     for (int i = 0; i < 12; ++i) p.p[i] = pose[i];
     const int cells = (ex.w / 8) * (ex.h / 8);
-    ray_begin_kernel<<<(cells + 255) / 256, 256, 0, st>>>(d_sv, p, check_visibility ? 1 : 0);
+    launch_kernel(ray_begin_kernel, (cells + 255) / 256, 256, ex.chain, st, d_sv, p, check_visibility ? 1 : 0);
     if (check_visibility) launch_visible_frustum(d_sv, 1, ex, st);
     launch_zrange(d_sv, 1, ex, st);
     launch_march(d_sv, 1, ex, vmap_ext, vmap_pitch, layouts, st, rgb_ext, rgb_pitch);

@@ -41,6 +41,7 @@ __device__ __forceinline__ uchar4 render_point(float3 p, float3 n, float3 img) {
 __global__ void render_kernel(const float4 *vmap, long long vmap_pitch, const float4 *nmap, long long nmap_pitch,
                               const uint8_t *rgb, long long rgb_pitch, int rgb_stride, int w, int h, uchar4 *out,
                               long long out_pitch) {
+    chain_begin();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= w || y >= h) return;
     const float4 v = reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(vmap) + y * vmap_pitch)[x];
@@ -56,6 +57,7 @@ __global__ void render_kernel(const float4 *vmap, long long vmap_pitch, const fl
 
 // The session's model prediction, whose image set only the device knows.
 __global__ void render_session_kernel(const SessionView *__restrict__ svs, int textured, uchar4 *out, long long out_pitch) {
+    chain_begin();
     const SessionView &sv = svs[0];
     const int w = sv.lv[0].w, x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= w) return;
@@ -74,14 +76,15 @@ __global__ void render_session_kernel(const SessionView *__restrict__ svs, int t
 
 void launch_render_session(const SessionView *d_sv, const Extent &ex, int textured, uchar4 *out, long long out_pitch,
                            cudaStream_t st) {
-    render_session_kernel<<<dim3((ex.w + 127) / 128, ex.h), 128, 0, st>>>(d_sv, textured, out, out_pitch);
+    launch_kernel(render_session_kernel, dim3((ex.w + 127) / 128, ex.h), 128, ex.chain, st, d_sv, textured, out,
+                  out_pitch);
 }
 
 void launch_render(const float4 *vmap, long long vmap_pitch, const float4 *nmap, long long nmap_pitch,
                    const uint8_t *rgb, long long rgb_pitch, int rgb_stride, int w, int h, uchar4 *out,
                    long long out_pitch, cudaStream_t st) {
-    render_kernel<<<dim3((w + 127) / 128, h), 128, 0, st>>>(vmap, vmap_pitch, nmap, nmap_pitch, rgb, rgb_pitch,
-                                                           rgb_stride, w, h, out, out_pitch);
+    launch_kernel(render_kernel, dim3((w + 127) / 128, h), 128, true, st, vmap, vmap_pitch, nmap, nmap_pitch, rgb,
+                  rgb_pitch, rgb_stride, w, h, out, out_pitch);
 }
 
 }  // namespace gbf

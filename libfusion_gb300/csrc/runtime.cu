@@ -466,6 +466,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     ex.h = K->height;
     ex.max_pool = cfg->num_blocks;
     ex.levels = cfg->num_levels;
+    ex.chain = 1;
     for (int l = 0; l < cfg->num_levels; ++l) {
         ex.max_red[l] = v.red_ctas[l];
         ex.max_iter[l] = cfg->max_iterations[l];

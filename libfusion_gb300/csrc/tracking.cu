@@ -1142,6 +1142,7 @@ __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv
 
 __global__ void __launch_bounds__(kTrackThreads, 1)
     gn_track_kernel(const SessionView *__restrict__ svs, int frame_mode) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char track_smem[];
     TrackSmem &sm = *reinterpret_cast<TrackSmem *>(track_smem);
     const SessionView &sv = svs[blockIdx.y];

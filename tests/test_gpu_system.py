@@ -840,6 +840,63 @@ def test_tracking_run_with_six_photometric_rows(gbf):
             assert np.array_equal(getattr(x.track, f), getattr(y.track, f), equal_nan=True), f
 
 
+def test_session_launches_captured_in_a_graph(gbf):
+    """A session's launches are chained (each set up while the one before runs); captured
+    in a caller's graph and replayed they do what they do when launched: a frame with its
+    cooperative tracking run, and an update with the raycast behind it."""
+    import torch
+    L = gbf
+    K = H.intrinsics(L, 320, 240)
+    cfg = H.small_config(L, 2, num_blocks=1 << 14, num_buckets=1 << 16)
+    fr = [(H.cuda(d), H.cuda(c), T) for d, c, T in H.frames(L, K, 6, seed=8)]
+    side = torch.cuda.Stream()
+
+    def frames(captured):
+        s, g, out = L.System(K, cfg), torch.cuda.CUDAGraph(), []
+        s.set_pose(fr[0][2])
+        for k, (d, c, _) in enumerate(fr):
+            s.stage(d, c, stream=side)
+            side.synchronize()
+            if captured and k == 2:
+                with torch.cuda.graph(g, stream=side):
+                    s.process_staged(stream=side)
+            if captured and k >= 2:
+                with torch.cuda.stream(side):
+                    g.replay()
+            else:
+                s.process_staged(stream=side)
+            side.synchronize()
+            out.append(s.get_camera_pose())
+        return np.stack(out), s.stats().allocated_blocks, s.get_rendered_image().cpu().numpy()
+    for a, b in zip(frames(False), frames(True)):
+        assert np.array_equal(a, b)
+
+    def maps(captured):
+        m, g = L.DenseMapping(K, cfg), torch.cuda.CUDAGraph()
+        v = torch.empty((K.height, K.width, 4), dtype=torch.float32, device="cuda")
+        d, c, T = torch.zeros((K.height, K.width), device="cuda"), fr[0][1].clone(), fr[0][2]
+
+        def step():
+            m.update(d, c, T, stream=side)
+            m.raycast(v, T, stream=side)
+        for k, f in enumerate(fr[:4]):
+            d.copy_(f[0].to(torch.int32).to(torch.float32) * 0.001)
+            c.copy_(f[1])
+            torch.cuda.synchronize()
+            if captured and k == 1:
+                with torch.cuda.graph(g, stream=side):
+                    step()
+            if captured and k >= 1:
+                with torch.cuda.stream(side):
+                    g.replay()
+            else:
+                step()
+            side.synchronize()
+        return v.cpu().numpy(), m.stats().allocated_blocks
+    for a, b in zip(maps(False), maps(True)):
+        assert np.array_equal(a, b, equal_nan=True)
+
+
 def test_tracking_runs_on_concurrent_streams(gbf):
     """Sessions driven on streams of their own, nothing waiting between them: their
     cooperative tracking runs, each of which takes the whole chip, beside each
