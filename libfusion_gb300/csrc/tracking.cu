@@ -745,9 +745,11 @@ __global__ void track_finish_kernel(const SessionView *__restrict__ svs, int fra
 // CTA per SM stays for the run, its code and the maps it gathers from in its
 // caches.  512 threads make the two rows of two pixels each of a 1024-pixel tile,
 // every gather of the tile in flight at once, into shared memory (zeros for a
-// rejected row); then two threads sum the 29 products of each eight-pixel chain,
-// where holding 29 sums while gathering leaves registers for two pixels in
-// flight.  CTA 0 makes no rows: it sums the tiles' records as they arrive, takes
+// rejected row); then half of the threads sum the 29 products of an eight-pixel chain
+// each, where holding 29 sums while gathering leaves registers for two pixels in
+// flight (all threads, two to a chain with half of the products each, read the rows
+// twice and took 3% longer over a 1280x720 frame's run: the rows' way through shared
+// memory weighs as much as the arithmetic).  CTA 0 makes no rows: it sums the tiles' records as they arrive, takes
 // the step on the tracking state in its shared memory and publishes the next
 // pose, so that the step's code stays in one SM's instruction cache.
 // An iteration then takes 10 us at 160x120 and 320x240 and 15 us at 640x480
@@ -825,65 +827,18 @@ __device__ __forceinline__ void pixel_rows(const LevelIn &K, const M34 &T, const
     }
 }
 
-// The products of PART of the eight rows of a chain, summed: the 29 sums of the
-// packed upper triangle by the words they multiply, PART 0 the ten products
-// within row[0..3] (lo) and the six within row[4..6] (hi), PART 1 the twelve
-// across and the count.
-template <int PART>
-__device__ __forceinline__ void chain_sums(const float4 *lo, const float4 *hi, int t, float (&acc)[16]) {
+// The 29 sums of chain t's eight rows (t, t + 128, ... of the tile).
+__device__ __forceinline__ void chain_sums(const float4 *lo, const float4 *hi, int t, float (&acc)[29]) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) acc[k] = 0.f;
+    for (int k = 0; k < 29; ++k) acc[k] = 0.f;
 #pragma unroll
     for (int i = 0; i < kCtaPixels / kHalfThreads; ++i) {
         const float4 a = lo[t + i * kHalfThreads], b = hi[t + i * kHalfThreads];
-        const float x[4] = {a.x, a.y, a.z, a.w}, y[3] = {b.x, b.y, b.z};
-        int k = 0;
-        if (PART == 0) {
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-#pragma unroll
-                for (int q = p; q < 4; ++q, ++k) acc[k] = __fmaf_rn(x[p], x[q], acc[k]);
-#pragma unroll
-            for (int p = 0; p < 3; ++p)
-#pragma unroll
-                for (int q = p; q < 3; ++q, ++k) acc[k] = __fmaf_rn(y[p], y[q], acc[k]);
-        } else {
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-#pragma unroll
-                for (int q = 0; q < 3; ++q, ++k) acc[k] = __fmaf_rn(x[p], y[q], acc[k]);
-            acc[12] += b.w;
-        }
+        const float row[7] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z};
+        const float count = acc[28] + b.w;  // a rejected pixel's row is all zeros
+        accumulate(acc, row);
+        acc[28] = count;
     }
-}
-// the packed index of sum k of a part (29 and above: none)
-__device__ __forceinline__ int packed_index(int part, int k) {
-    if (part == 0) {
-        const int p = (k >= 4) + (k >= 7) + (k >= 9), q = p + k - (p == 0 ? 0 : p == 1 ? 4 : p == 2 ? 7 : 9);
-        return k < 10 ? 7 * p - p * (p - 1) / 2 + (q - p) : 12 + k;  // then (4,4) (4,5) (4,6) (5,5) (5,6) (6,6): 22 ..
-    }
-    const int p = k / 3, q = 4 + k % 3;
-    return k < 12 ? 7 * p - p * (p - 1) / 2 + (q - p) : k == 12 ? 28 : 32;
-}
-
-// Warp sums of 16 values: after xor 16, 8, 4, 2 a lane holds one of them,
-// completed by xor 1; lane bits 4..1, most significant first, are its index.
-template <int N>
-__device__ __forceinline__ void part_step(float (&v)[16], int lane, int mask) {
-    const bool upper = (lane & mask) != 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const float send = upper ? v[i] : v[i + N];
-        const float keep = upper ? v[i + N] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
-    }
-}
-__device__ __forceinline__ float part_sum(float (&v)[16], int lane) {
-    part_step<8>(v, lane, 16);
-    part_step<4>(v, lane, 8);
-    part_step<2>(v, lane, 4);
-    part_step<1>(v, lane, 2);
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
 // A CTA of the run waits for another at most this long.  Every CTA is resident
@@ -1100,15 +1055,12 @@ __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv
                 load(tile + ctas < tiles ? tile + ctas : cta);
                 __syncwarp();
                 __syncthreads();
-                {
-                    // a warp per half (ICP, photometric), part of the products and chain warp
-                    const int half = warp & 1, part = (warp >> 1) & 1, cw = warp >> 2;
-                    float acc[16];
-                    if (part == 0) chain_sums<0>(sm.lo[half], sm.hi[half], 32 * cw + lane, acc);
-                    else chain_sums<1>(sm.lo[half], sm.hi[half], 32 * cw + lane, acc);
-                    const float s = part_sum(acc, lane);
-                    const int k = packed_index(part, lane >> 1);
-                    if (!(lane & 1) && k < 29) sm.warp_sums[cw][half * 29 + k] = s;
+                if (warp < 8) {  // ICP chains, then photometric ones
+                    const int half = warp >> 2, cw = warp & 3;
+                    float acc[29];
+                    chain_sums(sm.lo[half], sm.hi[half], 32 * cw + lane, acc);
+                    const float s = warp_sum29(acc);
+                    if (lane < 29) sm.warp_sums[cw][half * 29 + lane] = s;
                 }
                 __syncwarp();
                 __syncthreads();
