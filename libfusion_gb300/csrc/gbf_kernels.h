@@ -117,8 +117,8 @@ inline void square_gates(SessionView &v, float dist, float angle) {
 // kernel launches of one launch_track over nslots sessions
 int track_launches(int nslots, const Extent &ex, bool alone);
 void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, bool alone, cudaStream_t st);
-// sessions up to which a launch alone on the chip tracks in one cooperative kernel
-int track_run_sessions();
+// whether a launch of these sessions alone on the chip tracks in one cooperative kernel
+bool track_run_fits(int nslots, const Extent &ex);
 // what launch_track needs of the current device, asked once (before any stream capture)
 void prepare_track();
 // single reduction for gbf_reduce: pose given as float 3x4 in the kernel args

@@ -1117,11 +1117,10 @@ static void batch_results(gbf_batch *b, int k, cudaStream_t st) {
 
 // Branches of a tick.  Where the caller or the tuner has not set a number, few
 // sessions run as one: they then track in one launch that takes the chip
-// (launch_track), 0.73 against 0.83 ms per tick for two 640x480 sessions, 0.87
-// against 0.92 for three, 1.01 against 1.03 for four; from six on two branches
-// are faster (1.42 against 1.45 ms).
+// (track_run_fits), 0.61 against 0.83 ms per tick for two 640x480 sessions, 0.73
+// against 0.92 for three, 0.85 against 1.03 for four.
 static int tick_groups(const gbf_batch *b) {
-    if (!b->groups_set && !b->stagger && b->nslots <= track_run_sessions()) return 1;
+    if (!b->groups_set && !b->stagger && track_run_fits(b->nslots, b->ex)) return 1;
     return std::max(1, std::min(b->groups, b->nslots));
 }
 static int effective_groups(const gbf_batch *b) { return b->timing ? 1 : tick_groups(b); }

@@ -749,9 +749,9 @@ __global__ void track_finish_kernel(const SessionView *__restrict__ svs, int fra
 // each, where holding 29 sums while gathering leaves registers for two pixels in
 // flight (all threads, two to a chain with half of the products each, read the rows
 // twice and took 3% longer over a 1280x720 frame's run: the rows' way through shared
-// memory weighs as much as the arithmetic).  CTA 0 makes no rows: it sums the tiles' records as they arrive, takes
-// the step on the tracking state in its shared memory and publishes the next
-// pose, so that the step's code stays in one SM's instruction cache.
+// memory weighs as much as the arithmetic).  CTA 0 makes no rows: it sums the tiles'
+// records as they arrive, takes the step on the tracking state in its shared memory and
+// publishes the next pose, so that the step's code stays in one SM's instruction cache.
 // An iteration then takes 10 us at 160x120 and 320x240 and 15 us at 640x480
 // (two tiles per CTA: 7 us; step 3.7; each hop between CTAs 0.7), the run of a
 // 640x480 frame 0.25 -> 0.16 ms.  1024 threads of 64 registers spilled (0.25 ms);
@@ -1147,13 +1147,18 @@ constexpr int kTrackSubgroup = 64;
 constexpr int kDeferStepSessions = 32;
 static bool defer_step(int sessions) { return sessions >= kDeferStepSessions; }
 
-// Sessions up to which a launch that has the chip to itself takes the tracking
-// run in one cooperative kernel: track 0.25 -> 0.16 ms for one 640x480 session,
-// 0.28 -> 0.19 for two, 0.34 -> 0.26 for three, 0.39 -> 0.33 for four.  With more
-// the CTAs are busy with their tiles most of the time, and what is left to gain
-// (0.49 -> 0.43 ms for six) is less than concurrent groups give.
-constexpr int kTrackRunSessions = 4;
-int track_run_sessions() { return kTrackRunSessions; }
+// Whether a launch that has the chip to itself takes the tracking run in one
+// cooperative kernel: track 0.25 -> 0.154 ms for one 640x480 session, 0.28 -> 0.18 for
+// two, 0.34 -> 0.23 for three, 0.39 -> 0.29 for four.  More sessions share the CTAs, which
+// are then busy with their tiles most of the time; small images leave the run ahead of
+// two concurrent groups of launches (ticks of 6 sessions at 320x240, 450 level-0 tiles, 0.80
+// -> 0.76 ms; 12, 900 tiles, 1.14 -> 1.11; 16 at 256x192, 768 tiles, 1.39 -> 1.34), larger
+// ones do not (8 at 448x336, 1176 tiles, 1.02 both; 16 at 320x240, 1200 tiles, 1.42 -> 1.47;
+// 5 at 896x672, 2940 tiles, 1.50 -> 1.55).
+constexpr int kTrackRunFew = 4, kTrackRunSessions = 16, kTrackRunTiles = 1000;
+bool track_run_fits(int nslots, const Extent &ex) {
+    return nslots <= kTrackRunFew || (nslots <= kTrackRunSessions && nslots * ex.max_red[0] <= kTrackRunTiles);
+}
 
 // CTAs of one cooperative launch of gn_track_kernel on the current device (one
 // per SM), or 0 where it cannot be launched.
@@ -1178,12 +1183,12 @@ static int track_run_ctas() {
     return c - 1;
 }
 
-static bool takes_run(int nslots, bool alone) {
-    return alone && nslots <= kTrackRunSessions && track_run_ctas() >= 2 * nslots;
+static bool takes_run(int nslots, const Extent &ex, bool alone) {
+    return alone && track_run_fits(nslots, ex) && track_run_ctas() >= 2 * nslots;
 }
 
 int track_launches(int nslots, const Extent &ex, bool alone) {
-    if (takes_run(nslots, alone)) return 1;
+    if (takes_run(nslots, ex, alone)) return 1;
     int it = 0;
     for (int l = 0; l < ex.levels; ++l) it += ex.max_iter[l];
     int n = 0;
@@ -1195,7 +1200,7 @@ int track_launches(int nslots, const Extent &ex, bool alone) {
 void prepare_track() { track_run_ctas(); }
 
 void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, bool alone, cudaStream_t st) {
-    if (takes_run(nslots, alone)) {
+    if (takes_run(nslots, ex, alone)) {
         void *args[] = {(void *)&d_sv, (void *)&frame_mode};
         cudaLaunchCooperativeKernel((const void *)gn_track_kernel, dim3(track_run_ctas() / nslots, nslots),
                                     dim3(kTrackThreads), args, sizeof(TrackSmem), st);

@@ -800,6 +800,42 @@ def test_tracking_run_matches_launches_per_iteration(gbf, w, h, levels, iters, p
     batch.close()
 
 
+@pytest.mark.parametrize("n,groups", [(5, 0), (16, 0), (16, 1), (17, 0), (5, 3)])
+def test_many_small_sessions_track_as_alone(gbf, n, groups):
+    """Up to sixteen sessions of small images share one cooperative tracking run, more
+    or those of explicit groups take launches per iteration: every session's poses
+    are those it has alone."""
+    import torch
+    L = gbf
+    sizes = [(168, 120), (128, 96), (160, 128)]
+    alone, batch, todo = [], L.FusionBatch(n), []
+    if groups:
+        batch.set_groups(groups)
+    for i in range(n):
+        K = H.intrinsics(L, *sizes[i % 3])
+        cfg = H.small_config(L, 2, num_blocks=1 << 13, num_buckets=1 << 15, max_iterations=[4, 3, 2, 0, 0])
+        fr = [(H.cuda(d), H.cuda(c), T) for d, c, T in H.frames(L, K, 4, seed=i)]
+        a, b = L.System(K, cfg), L.System(K, cfg)
+        for s in (a, b):
+            s.set_pose(fr[0][2])
+        for d, c, _ in fr:
+            a.process_images(d, c)
+        batch.set(i, b)
+        alone.append(a)
+        todo.append((b, fr))
+    for k in range(4):
+        for b, fr in todo:
+            b.stage(fr[k][0], fr[k][1])
+        torch.cuda.synchronize()
+        batch.process([True] * n)
+        torch.cuda.synchronize()
+    for a, (b, _) in zip(alone, todo):
+        assert np.array_equal(a.get_camera_pose(), b.get_camera_pose())
+        x, y = a.stats(), b.stats()
+        assert list(x.level_iterations) == list(y.level_iterations) and x.track.iterations == y.track.iterations
+    batch.close()
+
+
 def test_tracking_run_with_six_photometric_rows(gbf):
     """Six photometric rows leave no degree of freedom: the residuals' deviation is
     infinite, the next iteration's residuals are zero (x / inf).  The run of a session
