@@ -54,6 +54,8 @@ struct IngestArgs {
     const void *depth; long long depth_pitch;
     const uint8_t *rgb; long long rgb_pitch;
 };
+// kernel launches of one launch_ingest
+inline int ingest_launches(const Extent &ex) { return 2 + (ex.levels > 3 ? ex.levels - 3 : 0); }
 void launch_ingest(const SessionView *d_sv, int nslots, const Extent &ex, const IngestArgs &a, cudaStream_t st);
 
 // ---- mapping (mapping.cu) ------------------------------------------------------

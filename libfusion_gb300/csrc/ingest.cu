@@ -1,15 +1,15 @@
 // ingest.cu -- frame ingest and tracking pyramids (DeviceImage::upload,
 // src/tracking/device_image.cpp:146-181; kernels of src/tracking/cuda_imgproc.cu).
 //
-// Three launches per frame for all sessions of a batch:
-//   1. ingest_l0:  u16 mm -> metres (System::process_images, src/system.cpp:43),
+// Two launches per frame for all sessions of a batch:
+//   1. ingest:     u16 mm -> metres (System::process_images, src/system.cpp:43),
 //                  rgb8 -> uchar4 + grey (device_image.cpp:161-162), bilateral
-//                  filter of the tracking depth (cuda_imgproc.cu:197-200) from a
-//                  shared-memory tile with a 2-pixel halo.
-//   2. pyr_down:   per level, 2x2 mean of depth (cv::cuda::resize 0.5,
+//                  filter of the tracking depth (cuda_imgproc.cu:197-200), and
+//                  levels 1 and 2: 2x2 mean of depth (cv::cuda::resize 0.5,
 //                  cuda_imgproc.cu:202-205) and 5x5 binomial pyrDown of the
-//                  intensity (cuda_imgproc.cu:207-210).  One launch per level.
-//   3. level_maps: every level in one launch: dI/dx, dI/dy (computeDerivativeK,
+//                  intensity (cuda_imgproc.cu:207-210), from shared-memory tiles.
+//                  Levels 3 and 4, where configured, are a launch each (pyr_down).
+//   2. level_maps: every level in one launch: dI/dx, dI/dy (computeDerivativeK,
 //                  cuda_imgproc.cu:217-234), vertex map (backProjectDepthK,
 //                  :249-263) and normal map (computeNMapK, :276-294), the normal
 //                  computed from back-projected neighbours so no second pass.
@@ -24,91 +24,229 @@ namespace gbf {
 
 namespace {
 
-constexpr int kTileW = 32, kTileH = 8, kHalo = 2;
-
 __device__ __forceinline__ int reflect101(int i, int n) {
     if (i < 0) i = -i;
     if (i >= n) i = 2 * n - 2 - i;
     return i;
 }
 
+__device__ __forceinline__ int clamp_index(int i, int n) { return min(max(i, 0), n - 1); }
+
 __device__ __forceinline__ int set_index(const SessionView &sv, int sel) {
     const int idx = sv.ts->idx;
     return sel ? idx : 1 - idx;
 }
 
-__global__ void __launch_bounds__(kTileW *kTileH) ingest_l0_kernel(const SessionView *__restrict__ svs, IngestArgs a) {
+// The frame's images and its pyramid down to level 2, a CTA per 32x32 tile of level 0.
+// Level 1 needs the grey image two pixels around the tile and level 2 level 1 two around
+// its part, six pixels of level 0 together, which every CTA converts for itself
+// (1.9 times the tile); the depth means stay within the tile.
+// What bounds it: issue, most of it the bilateral filter's thirteen exponentials.
+// A thread filters four rows of a column, whose windows share 28 of 52 samples, and the
+// binomial runs along rows and then columns, a lane per column whose reflected indices it
+// keeps.  As launches of their own (a pixel per thread, a window each; then a launch per
+// level) the three levels took, and take here: 8 sessions of 640x480 53 -> 45 us, one of
+// 1280x720 27 -> 21, of 320x240 12.4 -> 7.6.  40 or 48 registers instead of 64: 2% and 1% slower.
+constexpr int kTile = 32, kTileRows = 4, kTileThreads = kTile * kTile / kTileRows, kTileWarps = kTileThreads / 32;
+constexpr int kWin = 2, kGrey = 6;                                        // halos of the depth and the grey image
+constexpr int kZ = kTile + 2 * kWin, kG = kTile + 2 * kGrey, kG1 = kTile / 2 + 4;
+struct TileSmem {
+    float z[kZ][kZ];               // depth
+    float g[kG][kG];               // grey; read only where the image is
+    float h[kG][kG1];              // its rows, filtered for level 1
+    float g1[kG1][kG1];            // level 1, two pixels around the tile's part
+    float f[kTile][kTile];         // filtered depth
+    float d1[kTile / 2][kTile / 2];
+};
+
+__device__ __forceinline__ float binomial5(float a, float b, float c, float d, float e) {
+    return (((a + 4.f * b) + 6.f * c) + 4.f * d) + e;
+}
+
+__global__ void __launch_bounds__(kTileThreads, 4) ingest_kernel(const SessionView *__restrict__ svs, IngestArgs a) {
     chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
-    const int W = sv.lv[0].w, H = sv.lv[0].h;
-    const int tiles_x = (W + kTileW - 1) / kTileW;
-    const int tx0 = (blockIdx.x % tiles_x) * kTileW;
-    const int ty0 = (blockIdx.x / tiles_x) * kTileH;
-    if (ty0 >= H) return;  // uniform per CTA
+    const int W = sv.lv[0].w, H = sv.lv[0].h, levels = sv.levels;
+    const int tiles_x = (W + kTile - 1) / kTile;
+    const int x0 = (blockIdx.x % tiles_x) * kTile, y0 = (blockIdx.x / tiles_x) * kTile;
+    if (y0 >= H) return;  // uniform per CTA
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, set = set_index(sv, a.set_sel);
+    __shared__ TileSmem sm;
 
-    __shared__ float tile[kTileH + 2 * kHalo][kTileW + 2 * kHalo];
-    const int nt = (kTileH + 2 * kHalo) * (kTileW + 2 * kHalo);
-    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
-        const int ly = i / (kTileW + 2 * kHalo), lx = i % (kTileW + 2 * kHalo);
-        const int gx = reflect101(tx0 + lx - kHalo, W), gy = reflect101(ty0 + ly - kHalo, H);
-        float z;
-        if (a.src == 0) {
-            z = (float)sv.in_depth[(size_t)gy * W + gx] * 0.001f;
-        } else if (a.src == 1) {
-            const uint16_t *row = reinterpret_cast<const uint16_t *>(static_cast<const char *>(a.depth) + gy * a.depth_pitch);
-            z = (float)row[gx] * 0.001f;
-        } else {
-            const float *row = reinterpret_cast<const float *>(static_cast<const char *>(a.depth) + gy * a.depth_pitch);
-            z = row[gx];
+    // the tile's depth and colour, all loads before the first store: a warp per row,
+    // columns 0..31 of it, then what the halo adds
+    constexpr int kZRows = (kZ + kTileWarps - 1) / kTileWarps, kGRows = (kG + kTileWarps - 1) / kTileWarps;
+    float za[kZRows], zb[kZRows];
+    {
+        // (past the image's far border a tile holds samples that no pixel reads)
+        const int xa = clamp_index(reflect101(x0 + lane - kWin, W), W);
+        const int xb = clamp_index(reflect101(x0 + 32 + lane - kWin, W), W);
+        const char *rows = a.src == 0 ? reinterpret_cast<const char *>(sv.in_depth) : static_cast<const char *>(a.depth);
+        const long long pitch = a.src == 0 ? (long long)W * 2 : a.depth_pitch;
+        const auto load = [&](const auto &at) {
+#pragma unroll
+            for (int k = 0; k < kZRows; ++k) {
+                const int r = warp + k * kTileWarps;
+                const char *row = rows + clamp_index(reflect101(y0 + r - kWin, H), H) * pitch;
+                za[k] = zb[k] = 0.f;
+                if (r < kZ) {
+                    za[k] = at(row, xa);
+                    if (lane < 2 * kWin) zb[k] = at(row, xb);
+                }
+            }
+        };
+        if (a.src == 2) load([](const char *row, int x) { return __ldg(reinterpret_cast<const float *>(row) + x); });
+        else load([](const char *row, int x) { return (float)__ldg(reinterpret_cast<const uint16_t *>(row) + x) * 0.001f; });
+    }
+    {
+        const uint8_t *rgb = a.src == 0 ? sv.in_rgb : a.rgb;
+        const long long pitch = a.src == 0 ? (long long)W * 3 : a.rgb_pitch;
+        const int hx = lane < kGrey ? x0 - kGrey + lane : x0 + kTile + lane - kGrey;  // halo columns, lanes 0..11
+        uchar4 ca[kGRows], cb[kGRows];
+#pragma unroll
+        for (int k = 0; k < kGRows; ++k) {
+            const int r = warp + k * kTileWarps, y = y0 + r - kGrey;
+            const bool in = r < kG && y >= 0 && y < H && (levels > 1 || (r >= kGrey && r < kGrey + kTile));
+            const auto load = [&](int x) {
+                const uint8_t *px = rgb + y * pitch + (long long)x * 3;
+                return make_uchar4(__ldg(px), __ldg(px + 1), __ldg(px + 2), 0);
+            };
+            ca[k] = cb[k] = make_uchar4(0, 0, 0, 0);
+            if (in && x0 + lane < W) ca[k] = load(x0 + lane);
+            if (in && levels > 1 && lane < 2 * kGrey && hx >= 0 && hx < W) cb[k] = load(hx);
         }
-        tile[ly][lx] = z;
+#pragma unroll
+        for (int k = 0; k < kZRows; ++k) {
+            const int r = warp + k * kTileWarps;
+            if (r < kZ) {
+                sm.z[r][lane] = za[k];
+                if (lane < 2 * kWin) sm.z[r][32 + lane] = zb[k];
+            }
+        }
+        // cv::COLOR_RGB2GRAY on CV_32FC3: 0.299 R + 0.587 G + 0.114 B
+        const auto grey = [](uchar4 c) { return (0.299f * (float)c.x + 0.587f * (float)c.y) + 0.114f * (float)c.z; };
+#pragma unroll
+        for (int k = 0; k < kGRows; ++k) {
+            const int r = warp + k * kTileWarps, y = y0 + r - kGrey;
+            if (r >= kG) continue;
+            const float v = grey(ca[k]);
+            sm.g[r][kGrey + lane] = v;
+            if (lane < 2 * kGrey) sm.g[r][lane < kGrey ? lane : kTile + lane] = grey(cb[k]);
+            if (r >= kGrey && r < kGrey + kTile && y < H && x0 + lane < W) {
+                const size_t p = (size_t)y * W + x0 + lane;
+                sv.rgb4[p] = ca[k];
+                sv.inten[set][0][p] = v;
+            }
+        }
     }
     __syncthreads();
 
-    const int lx = threadIdx.x % kTileW, ly = threadIdx.x / kTileW;
-    const int x = tx0 + lx, y = ty0 + ly;
-    if (x >= W || y >= H) return;
-    const size_t p = (size_t)y * W + x;
-    const float c = tile[ly + kHalo][lx + kHalo];
-    sv.depth_raw[p] = c;
-
-    float filt = c;
-    if (sv.bilateral) {
-        // circular window of radius 2 (cv::cuda::bilateralFilter(src, dst, 5, 1, 1))
-        const float ks = -0.5f, kc = -0.5f;  // -1/(2 sigma^2), sigma_space = sigma_colour = 1
-        float s1 = 0.f, s2 = 0.f;
+    // depth: rows 4 warp .. + 3 of column lane
+    {
+        const int r0 = kTileRows * warp;
+        float m[kTileRows + 4], l1[kTileRows + 2], r1[kTileRows + 2], l2[kTileRows], r2[kTileRows];
 #pragma unroll
-        for (int dy = -2; dy <= 2; ++dy) {
+        for (int k = 0; k < kTileRows + 4; ++k) m[k] = sm.z[r0 + k][lane + 2];
 #pragma unroll
-            for (int dx = -2; dx <= 2; ++dx) {
-                const int sp = dx * dx + dy * dy;
-                if (sp > 4) continue;
-                const float v = tile[ly + kHalo + dy][lx + kHalo + dx];
-                const float d = v - c;
-                const float w = expf((float)sp * ks + (d * d) * kc);
-                s1 += w * v;
-                s2 += w;
+        for (int k = 0; k < kTileRows + 2; ++k) {
+            l1[k] = sm.z[r0 + k + 1][lane + 1];
+            r1[k] = sm.z[r0 + k + 1][lane + 3];
+        }
+#pragma unroll
+        for (int k = 0; k < kTileRows; ++k) {
+            l2[k] = sm.z[r0 + k + 2][lane];
+            r2[k] = sm.z[r0 + k + 2][lane + 4];
+        }
+#pragma unroll
+        for (int k = 0; k < kTileRows; ++k) {
+            const float c = m[k + 2];
+            float filt = c;
+            if (sv.bilateral) {
+                // circular window of radius 2 (cv::cuda::bilateralFilter(src, dst, 5, 1, 1))
+                const float ks = -0.5f, kc = -0.5f;  // -1/(2 sigma^2), sigma_space = sigma_colour = 1
+                float s1 = 0.f, s2 = 0.f;
+                const auto tap = [&](float v, int sp) {
+                    const float d = v - c;
+                    const float w = expf((float)sp * ks + (d * d) * kc);
+                    s1 += w * v;
+                    s2 += w;
+                };
+                tap(m[k], 4);
+                tap(l1[k], 2); tap(m[k + 1], 1); tap(r1[k], 2);
+                tap(l2[k], 4); tap(l1[k + 1], 1); tap(c, 0); tap(r1[k + 1], 1); tap(r2[k], 4);
+                tap(l1[k + 2], 2); tap(m[k + 3], 1); tap(r1[k + 2], 2);
+                tap(m[k + 4], 4);
+                filt = s1 / s2;
+            }
+            sm.f[r0 + k][lane] = filt;
+            const int y = y0 + r0 + k, x = x0 + lane;
+            if (y < H && x < W) {
+                const size_t p = (size_t)y * W + x;
+                sv.depth_raw[p] = c;
+                sv.depth[0][p] = filt;
             }
         }
-        filt = s1 / s2;
     }
-    sv.depth[0][p] = filt;
-
-    uint8_t r, g, b;
-    if (a.src == 0) {
-        const uint8_t *px = sv.in_rgb + p * 3;
-        r = px[0]; g = px[1]; b = px[2];
-    } else {
-        const uint8_t *px = a.rgb + y * a.rgb_pitch + (size_t)x * 3;
-        r = px[0]; g = px[1]; b = px[2];
+    if (levels < 2) return;
+    const int w1 = sv.lv[1].w, h1 = sv.lv[1].h, X1 = x0 / 2, Y1 = y0 / 2;
+    // intensity: 5x5 binomial, reflect-101, sample at (2x, 2y); its rows first, a warp
+    // per row and a lane per column of level 1
+    const int x1 = X1 - 2 + lane;
+    const bool in1 = lane < kG1 && x1 >= 0 && x1 < w1;
+    {
+        const int at = 2 * x1, o = kGrey - x0;
+        const int c0 = abs(at - 2) + o, c1 = abs(at - 1) + o, c3 = reflect101(at + 1, W) + o, c4 = reflect101(at + 2, W) + o;
+        if (in1) {
+#pragma unroll 2
+            for (int r = warp; r < kG; r += kTileWarps) {
+                const float *row = sm.g[r];
+                sm.h[r][lane] = binomial5(row[c0], row[c1], row[at + o], row[c3], row[c4]);
+            }
+        }
     }
-    sv.rgb4[p] = make_uchar4(r, g, b, 0);
-    // cv::COLOR_RGB2GRAY on CV_32FC3: 0.299 R + 0.587 G + 0.114 B
-    const float grey = (0.299f * (float)r + 0.587f * (float)g) + 0.114f * (float)b;
-    sv.inten[set_index(sv, a.set_sel)][0][p] = grey;
+    __syncthreads();
+    for (int r = warp; r < kG1; r += kTileWarps) {
+        const int y = Y1 - 2 + r, at = 2 * y, o = kGrey - y0;
+        if (!in1 || y < 0 || y >= h1) continue;
+        const float v = binomial5(sm.h[abs(at - 2) + o][lane], sm.h[abs(at - 1) + o][lane], sm.h[at + o][lane],
+                                  sm.h[reflect101(at + 1, H) + o][lane], sm.h[reflect101(at + 2, H) + o][lane]) *
+                        (1.f / 256.f);
+        sm.g1[r][lane] = v;
+        if (r >= 2 && r < 2 + kTile / 2 && lane >= 2 && lane < 2 + kTile / 2) sv.inten[set][1][(size_t)y * w1 + x1] = v;
+    }
+    // depth: 2x2 mean (resize by 0.5, pixel-centre bilinear)
+    const auto mean = [](float a0, float a1, float a2, float a3) { return (((a0 + a1) + a2) + a3) * 0.25f; };
+    {
+        const int lx = tid & 15, ly = tid >> 4, x = X1 + lx, y = Y1 + ly;
+        if (x < w1 && y < h1) {
+            const float v = mean(sm.f[2 * ly][2 * lx], sm.f[2 * ly][2 * lx + 1], sm.f[2 * ly + 1][2 * lx],
+                                 sm.f[2 * ly + 1][2 * lx + 1]);
+            sm.d1[ly][lx] = v;
+            sv.depth[1][(size_t)y * w1 + x] = v;
+        }
+    }
+    if (levels < 3) return;
+    __syncthreads();
+    const int w2 = sv.lv[2].w, h2 = sv.lv[2].h, lx = tid & 7, ly = (tid >> 3) & 7, x = x0 / 4 + lx, y = y0 / 4 + ly;
+    if (x >= w2 || y >= h2) return;
+    if (tid < 64) {
+        float hrow[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const float *row = sm.g1[reflect101(2 * y + j - 2, h1) - (Y1 - 2)] + (2 - X1);
+            const int at = 2 * x;
+            hrow[j] = binomial5(row[abs(at - 2)], row[abs(at - 1)], row[at], row[reflect101(at + 1, w1)],
+                                row[reflect101(at + 2, w1)]);
+        }
+        sv.inten[set][2][(size_t)y * w2 + x] = binomial5(hrow[0], hrow[1], hrow[2], hrow[3], hrow[4]) * (1.f / 256.f);
+    } else if (tid < 128) {
+        sv.depth[2][(size_t)y * w2 + x] =
+            mean(sm.d1[2 * ly][2 * lx], sm.d1[2 * ly][2 * lx + 1], sm.d1[2 * ly + 1][2 * lx], sm.d1[2 * ly + 1][2 * lx + 1]);
+    }
 }
 
+// Levels 3 and up, a launch each.
 __global__ void pyr_down_kernel(const SessionView *__restrict__ svs, int set_sel, int level) {
     chain_begin();
     const SessionView &sv = svs[blockIdx.y];
@@ -245,10 +383,10 @@ __global__ void __launch_bounds__(kMapThreads, 3) level_maps_kernel(const Sessio
 }  // namespace
 
 void launch_ingest(const SessionView *d_sv, int nslots, const Extent &ex, const IngestArgs &a, cudaStream_t st) {
-    const int tiles = ((ex.w + kTileW - 1) / kTileW) * ((ex.h + kTileH - 1) / kTileH);
-    launch_kernel(ingest_l0_kernel, dim3(tiles, nslots), kTileW * kTileH, ex.chain, st, d_sv, a);
-    int w = ex.w, h = ex.h;
-    for (int l = 1; l < ex.levels; ++l) {
+    const int tiles = ((ex.w + kTile - 1) / kTile) * ((ex.h + kTile - 1) / kTile);
+    launch_kernel(ingest_kernel, dim3(tiles, nslots), kTileThreads, ex.chain, st, d_sv, a);
+    int w = ex.w / 4, h = ex.h / 4;
+    for (int l = 3; l < ex.levels; ++l) {
         w /= 2; h /= 2;
         launch_kernel(pyr_down_kernel, dim3((w * h + 255) / 256, nslots), 256, ex.chain, st, d_sv, a.set_sel, l);
     }

@@ -435,6 +435,49 @@ def test_raycast_maps_bit_exact(gbf, layout):
     assert np.array_equal(np.nan_to_num(vm2.cpu().numpy(), nan=7.0), np.nan_to_num(g, nan=7.0))
 
 
+@pytest.mark.parametrize("w,h,levels", [(64, 64, 3), (72, 80, 2), (96, 64, 1), (104, 72, 3), (176, 144, 4), (328, 248, 3)])
+def test_pyramid_tiles(gbf, w, h, levels):
+    """The fused pyramid's tiles at their edges: images of whole and of ragged 32x32 tiles
+    and of one to four levels, of noise with invalid depths, every image bit for bit the
+    oracle's from float depth; and the same images from pitched and from staged u16 depth."""
+    import oracle as O
+    import torch
+    L = gbf
+    K = L.IntrinsicMatrix(w, h, 0.8 * w, 0.8 * w, w / 2 - 0.3, h / 2 + 0.2)
+    rng = np.random.default_rng(w)
+    mm = rng.integers(250, 5100, (h, w)).astype(np.uint16)
+    mm[rng.random((h, w)) < 0.1] = 0
+    mm[:4, :4] = mm[-4:, -4:] = 1500
+    c = rng.integers(0, 256, (h, w, 3)).astype(np.uint8)
+    dm = H.depth_m(mm)
+    for bil in (0, 1):
+        cfg = H.small_config(L, 0, bilateral=bil, num_levels=levels, num_blocks=1 << 12, num_buckets=1 << 14)
+        t = L.DenseTracking(K, cfg)
+        t.set_reference(H.cuda(dm), H.cuda(c))
+
+        def oracle_run():
+            fr = O.OracleFrame(O.config_from(cfg), O.intrinsics_from(K))
+            fr.build(dm, c)
+            return [[fr.get(kind, lvl) for kind in range(6)] for lvl in range(levels)]
+        want, _, misses = O.with_device_transcendentals(oracle_run, {O.TRANS_EXP: _device_exp})
+        assert misses[O.TRANS_EXP] == 0
+        for lvl in range(levels):
+            for kind in range(6):
+                assert np.array_equal(t.get_image(1, kind, lvl).cpu().numpy(), want[lvl][kind], equal_nan=True), (bil, lvl, kind)
+        wide_d = torch.zeros((h, w + 6), dtype=torch.uint16, device="cuda")
+        wide_c = torch.zeros((h, w + 6, 3), dtype=torch.uint8, device="cuda")
+        wide_d[:, :w], wide_c[:, :w] = H.cuda(mm), H.cuda(c)
+        pitched, staged = L.System(K, cfg), L.System(K, cfg)
+        L._lib.call("gbf_process_frame", pitched._h, wide_d.data_ptr(), 2 * (w + 6), wide_c.data_ptr(), 3 * (w + 6),
+                    torch.cuda.current_stream().cuda_stream)
+        staged.stage(H.cuda(mm), H.cuda(c))
+        staged.process_staged()
+        for s in (pitched, staged):
+            for lvl in range(levels):
+                assert np.array_equal(s.get_image(1, 2, lvl).cpu().numpy(), want[lvl][2]), lvl
+                assert np.array_equal(s.get_image(1, 5, lvl).cpu().numpy(), want[lvl][5], equal_nan=True), lvl
+
+
 @pytest.mark.parametrize("w,h", [(320, 240), (328, 248), (1280, 720)])
 def test_post_raycast_pyramid_bit_exact(gbf, w, h):
     """DeviceImage::resize_device_map (src/tracking/device_image.cpp:188-199):
