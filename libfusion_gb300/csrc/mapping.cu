@@ -27,8 +27,8 @@ namespace gbf {
 
 namespace {
 
-constexpr int kAllocTile = 16;        // 16x16 pixels per CTA
-constexpr int kSetSize = 1024;        // shared-memory key set per CTA
+constexpr int kAllocThreads = 256;      // 32 pixels wide, 8 rows at a time
+constexpr int kSetBits = 10, kSetSize = 1 << kSetBits;  // shared-memory key set per CTA
 
 // Per-pixel part of the integration test and weight (update_map_with_colour_kernel,
 // depth_fusion.cu:317-331, without normals; update_map_weighted_kernel, :390-405, with):
@@ -60,20 +60,38 @@ __global__ void fuse_import_kernel(const SessionView *__restrict__ svs, FuseImpo
     sv.fuse_px[i] = make_float2(ok ? dist : __int_as_float(0x7fffffff), w);
 }
 
-// Shared-memory set insert; false when the set is full (caller inserts globally).
-__device__ __forceinline__ bool set_insert(unsigned long long *set, unsigned long long key) {
+// The blocks a CTA's pixels pass, each once: an open-addressed key set and the list of
+// its entries.
+struct BlockSet {
+    __align__(16) unsigned long long key[kSetSize];
+    unsigned long long list[kSetSize];
+    int count;
+};
+
+// False when the set is full where the key belongs (caller inserts globally).  The entry
+// is read before it is claimed: the pixels of a warp pass the same few blocks, whose keys
+// are there already and are read at once, where a compare-and-swap takes one lane
+// after the other.
+__device__ __forceinline__ bool set_insert(BlockSet &set, unsigned long long key) {
     unsigned h = (unsigned)(key ^ (key >> 29) ^ (key >> 43)) * 0x9E3779B1u;
-    unsigned s = h >> (32 - 10);  // kSetSize = 1024
+    unsigned s = h >> (32 - kSetBits);
     for (int p = 0; p < 64; ++p) {
-        const unsigned long long old = atomicCAS(set + s, kEmptyKey, key);
-        if (old == kEmptyKey || old == key) return true;
+        unsigned long long old = *static_cast<volatile unsigned long long *>(set.key + s);
+        if (old == key) return true;
+        if (old == kEmptyKey) {
+            old = atomicCAS(set.key + s, kEmptyKey, key);
+            if (old == key) return true;
+            if (old == kEmptyKey) {
+                set.list[atomicAdd(&set.count, 1)] = key;
+                return true;
+            }
+        }
         s = (s + 1) & (kSetSize - 1);
     }
     return false;
 }
 
-__device__ __forceinline__ void visit_block(const SessionView &sv, unsigned long long *set, int bx, int by, int bz,
-                                            int frame) {
+__device__ __forceinline__ void visit_block(const SessionView &sv, BlockSet &set, int bx, int by, int bz, int frame) {
     if (!coord_ok(bx, by, bz)) {
         raise_flag(sv, GBF_FLAG_COORD_RANGE);
         return;
@@ -92,26 +110,46 @@ __device__ __forceinline__ int3 pixel_block(const SessionView &sv, const M34 &T,
                      voxel_to_block(floor_ref(w.z / sv.voxel)));
 }
 
-__global__ void __launch_bounds__(kAllocTile *kAllocTile) alloc_kernel(const SessionView *svs) {
+// The blocks within half the truncation of each valid pixel's depth, gathered per tile of
+// 32 x 8 ROWS pixels and then looked up or created, a thread per block.  What bounded it
+// was the way into the shared set, a 64-bit compare-and-swap per pixel and block with
+// up to 32 lanes on one entry, and the set's own 8 KB cleared and scanned per 256 pixels;
+// now it is the pixels' own arithmetic (64 sessions of 640x480, with the visible pass: 489
+// -> 408 us entry read first, 353 two rows a thread, 302 four, 276 with the list).
+template <int ROWS>
+__global__ void __launch_bounds__(kAllocThreads) alloc_kernel(const SessionView *svs) {
     chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     const int W = sv.lv[0].w, H = sv.lv[0].h;
-    const int tiles_x = (W + kAllocTile - 1) / kAllocTile;
-    const int x = (blockIdx.x % tiles_x) * kAllocTile + (threadIdx.x % kAllocTile);
-    const int y = (blockIdx.x / tiles_x) * kAllocTile + (threadIdx.x / kAllocTile);
-    if ((blockIdx.x / tiles_x) * kAllocTile >= H) return;  // uniform per CTA
+    const int tiles_x = (W + 31) / 32;
+    const int x = (blockIdx.x % tiles_x) * 32 + (threadIdx.x & 31), y0 = (blockIdx.x / tiles_x) * (8 * ROWS);
+    if (y0 >= H) return;  // uniform per CTA
 
-    __shared__ unsigned long long set[kSetSize];
+    __shared__ BlockSet set;
     __shared__ M34 T;
-    for (int i = threadIdx.x; i < kSetSize; i += blockDim.x) set[i] = kEmptyKey;
-    if (threadIdx.x == 0) T = load_m34(sv.ts->map_twc);
+    float zs[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+        const int y = y0 + 8 * k + (threadIdx.x >> 5);
+        zs[k] = x < W && y < H ? sv.depth_raw[(size_t)y * W + x] : __int_as_float(0x7fffffff);
+    }
+    for (int i = threadIdx.x; i < kSetSize / 2; i += kAllocThreads)
+        reinterpret_cast<ulonglong2 *>(set.key)[i] = make_ulonglong2(kEmptyKey, kEmptyKey);
+    if (threadIdx.x == 0) {
+        T = load_m34(sv.ts->map_twc);
+        set.count = 0;
+    }
     __syncthreads();
     const int frame = sv.ctr[C_FRAME] + 1;  // counted by integrate_kernel
     if (blockIdx.x == 0 && threadIdx.x == 0) sv.ctr[C_NVIS] = 0;
 
-    if (x < W && y < H) {
-        const float z = sv.depth_raw[(size_t)y * W + x];
+#pragma unroll 1
+    for (int k = 0; k < ROWS; ++k) {
+        const int y = y0 + 8 * k + (threadIdx.x >> 5);
+        float z = zs[0];
+#pragma unroll
+        for (int q = 1; q < ROWS; ++q) z = k == q ? zs[q] : z;
         // create_blocks_kernel (depth_fusion.cu:130-141)
         if (!(isnan(z) || z < sv.zmin_u || z > sv.zmax_u)) {
             const float z_thresh = sv.tau * 0.5f;
@@ -155,9 +193,8 @@ __global__ void __launch_bounds__(kAllocTile *kAllocTile) alloc_kernel(const Ses
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kSetSize; i += blockDim.x) {
-        const unsigned long long key = set[i];
-        if (key == kEmptyKey) continue;
+    for (int i = threadIdx.x; i < set.count; i += kAllocThreads) {
+        const unsigned long long key = set.list[i];
         // unpack the 21-bit fields (sign-extend)
         const int bx = (int)((long long)(key << (64 - 3 * kCoordBits)) >> (64 - kCoordBits));
         const int by = (int)((long long)(key << (64 - 2 * kCoordBits)) >> (64 - kCoordBits));
@@ -326,8 +363,18 @@ void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImp
 constexpr int kVisCtas = 152;
 
 void launch_alloc_visible(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
-    const int tiles = ((ex.w + kAllocTile - 1) / kAllocTile) * ((ex.h + kAllocTile - 1) / kAllocTile);
-    launch_kernel(alloc_kernel, dim3(tiles, nslots), kAllocTile * kAllocTile, ex.chain, st, d_sv);
+    // Rows of a thread: one where the image's CTAs then still start at once (8 per SM),
+    // two up to four rounds of them, four beyond, where a block that several tiles see
+    // costs more than the length of a CTA.  Allocation and visible pass in us with 1, 2, 4
+    // rows: one 640x480 session 19.8, 20.4, 24.4; four 34.6, 32.8, 34.7; 64: 338, 300, 276.
+    const auto alloc = [&](auto *kernel, int rows) {
+        const dim3 g(((ex.w + 31) / 32) * ((ex.h + 8 * rows - 1) / (8 * rows)), nslots);
+        launch_kernel(kernel, g, kAllocThreads, ex.chain, st, d_sv);
+    };
+    const long long ctas = (long long)ex.w * ex.h / kAllocThreads * nslots;
+    if (ctas <= 8 * 152) alloc(alloc_kernel<1>, 1);
+    else if (ctas <= 4 * 8 * 152) alloc(alloc_kernel<2>, 2);
+    else alloc(alloc_kernel<4>, 4);
     const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
     launch_kernel(visible_kernel<true>, dim3(gv, nslots), 256, ex.chain, st, d_sv);
 }
