@@ -870,11 +870,13 @@ __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long lon
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-// two words at once from L2; each carries its own number, so they need not arrive together
-__device__ __forceinline__ uint4 ld_l2(const unsigned long long *p) {
-    uint4 v;
-    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+// Two words from L2; each carries its own number, so they need not arrive together.  The
+// plain load moves five times the bytes of relaxed ones, but only those are sure to see
+// a store in the end: whoever reads again reads relaxed.
+__device__ __forceinline__ ulonglong2 ld_l2(const unsigned long long *p, bool again) {
+    if (again) return make_ulonglong2(ld_relaxed(p), ld_relaxed(p + 1));
+    ulonglong2 v;
+    asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ void st_relaxed(unsigned long long *p, unsigned long long v) {
@@ -906,9 +908,8 @@ __device__ __forceinline__ unsigned long long *record_word(const SessionView &sv
 // The sums of the item numbered `number`, by all threads of CTA 0: warp g waits
 // for records g, g + 16, ... (a lane per record looks at its first word), then
 // lane q adds columns 2 q and 2 q + 1 of them in turn; the 16 groups follow in
-// order (the sums and the order of sum_partials).  The words are read by plain
-// L2 loads, ten in flight, which moved five times the bytes of relaxed ones, and checked by their
-// numbers.  Records past the last count as zeros, which add nothing.
+// order (the sums and the order of sum_partials).  The words are read ten in
+// flight (ld_l2) and checked by their numbers.  Records past the last count as zeros, which add nothing.
 static_assert(kTrackThreads == 32 * kSumGroups, "a warp per record group");
 __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv, int n, int number) {
     const int g = threadIdx.x >> 5, lane = threadIdx.x & 31, q = min(2 * lane, kReduceWidth - 2);
@@ -920,22 +921,23 @@ __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv
         while (!__all_sync(0xffffffffu, r >= end || (int)(ld_relaxed(record_word(sv, r, 0)) >> 32) == number) &&
                !__any_sync(0xffffffffu, limit.over())) {}
         for (int c = first; c < end; c += kBatch * kSumGroups) {
-            uint4 w[kBatch];
-            bool all;
+            ulonglong2 w[kBatch];
+            bool all, again = false;
             do {
                 all = true;
 #pragma unroll
                 for (int i = 0; i < kBatch; ++i) {
-                    w[i] = make_uint4(0u, (unsigned)number, 0u, (unsigned)number);
-                    if (c + i * kSumGroups < end) w[i] = ld_l2(record_word(sv, c + i * kSumGroups, q));
+                    w[i] = make_ulonglong2(tagged(number, 0u), tagged(number, 0u));
+                    if (c + i * kSumGroups < end) w[i] = ld_l2(record_word(sv, c + i * kSumGroups, q), again);
                 }
 #pragma unroll
-                for (int i = 0; i < kBatch; ++i) all = all && (int)w[i].y == number && (int)w[i].w == number;
+                for (int i = 0; i < kBatch; ++i) all = all && (int)(w[i].x >> 32) == number && (int)(w[i].y >> 32) == number;
+                again = true;
             } while (!__all_sync(0xffffffffu, all) && !__any_sync(0xffffffffu, limit.over()));
 #pragma unroll
             for (int i = 0; i < kBatch; ++i) {
-                s0.add(__uint_as_float(w[i].x));
-                s1.add(__uint_as_float(w[i].z));
+                s0.add(__uint_as_float((unsigned)w[i].x));
+                s1.add(__uint_as_float((unsigned)w[i].y));
             }
         }
     }
@@ -999,7 +1001,12 @@ __device__ __forceinline__ void track_steps(TrackSmem &sm, const SessionView &sv
     }
     __syncthreads();
     if (tid < 32) {
-        if (lost) ts->invalid = 1;  // a wait ran out: the frame counts as not tracked
+        if (lost) {
+            // a wait ran out: the frame counts as not tracked, the other CTAs end, and the
+            // numbers go on behind that of the records that may still come
+            ts->invalid = 1;
+            if (lane < kPubWords) st_relaxed(pub + lane, tagged(seen + 1, 0u));
+        }
         __syncwarp();
         track_finish(sv, ts, frame_mode);
     }
@@ -1071,6 +1078,8 @@ __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv
                     st_relaxed(record_word(sv, tile, tid), tagged(seen + 1, __float_as_uint(s)));
                 }
             }
+        } else {
+            __syncthreads();  // every warp has the item before the next one takes its place
         }
         if (warp == 0) {
             unsigned value = 0;
