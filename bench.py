@@ -1036,15 +1036,14 @@ def phase_bytes(phase: str, P: int, levels: int, s_v: int, d: dict) -> float | N
         return 5 * P + 8 * P + sum(8 * (Pl[l - 1] + Pl[l]) for l in range(1, levels)) + sum(48 * x for x in Pl)
     if phase == "track":    # reference vmap+nmap+I, current vmap+nmap+I+gradients per pixel-iteration
         return 80.0 * d["pixel_iterations"]
-    if phase == "alloc_visible":  # depth in; per allocated block its record; the visible list out (lower bound)
-        return 4 * P + 20.0 * d["allocated_blocks"] + 4.0 * d["visible_blocks"]
+    if phase == "alloc_visible":  # depth in; per allocated block its record; the visible list and the z-range grid out
+        return 4 * P + 20.0 * d["allocated_blocks"] + 4.0 * d["visible_blocks"] + 8 * (P // 64)
     if phase == "integrate":  # voxel read-modify-write of every visible block + depth, normal, colour per pixel
         return 2.0 * s_v * 512 * d["integrated_blocks"] + 23 * P
-    if phase == "zrange":
-        return 20.0 * d["visible_blocks"] + 8 * (P // 64)
     if phase == "post":     # vertex maps halved per level, normals recomputed per level
         return sum(16 * (Pl[l - 1] + Pl[l]) for l in range(1, levels)) + sum(32 * x for x in Pl)
-    return None             # the march: bound by instruction issue, its voxel fetches depend on the rays
+    return None             # the march: bound by instruction issue, its voxel fetches depend on the rays;
+                            # the z-range: made with the visible list
 
 
 def run_scale(args):

@@ -484,7 +484,8 @@ GBF_API gbf_status gbf_autotune_forget(void);
  * the slots, groups, stagger or timing, and destroying the batch, flush too. */
 GBF_API gbf_status gbf_batch_flush(gbf_batch *b, void *stream);
 /* Record CUDA events at the phase boundaries of every tick (captured into the
- * graph): ingest, track, alloc+visible, integrate, z-range, march, post. */
+ * graph): ingest, track, alloc+visible (with the z-range, made in the same pass),
+ * integrate, z-range (no launch of its own: about 2 us), march, post. */
 GBF_API gbf_status gbf_batch_set_timing(gbf_batch *b, int32_t enable);
 /* Mean durations (ms) of the 7 phases over the ticks since timing was enabled
  * (waits for the outstanding ticks); ms[7], when n > 7, receives the tick count. */

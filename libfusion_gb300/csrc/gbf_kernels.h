@@ -68,9 +68,8 @@ struct FuseImport {
 void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImport &in, const double pose[12],
                         cudaStream_t st);
 void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st);
-void launch_alloc_visible(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
-// visible list = allocated blocks in the frustum of the map pose (no fuse)
-void launch_visible_frustum(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
+// the blocks of the frame's surface; also clears the visible count and the z-range grid
+void launch_alloc(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
 // Phong shading of camera-frame vertex / normal maps into RGBA8 (rgb NULL = untextured)
 void launch_render(const float4 *vmap, long long vmap_pitch, const float4 *nmap, long long nmap_pitch,
                    const uint8_t *rgb, long long rgb_pitch, int rgb_stride, int w, int h, uchar4 *out,
@@ -86,8 +85,11 @@ void launch_render_session(const SessionView *d_sv, const Extent &ex, int textur
 void launch_raycast(const SessionView *d_sv, const Extent &ex, const double pose[12], bool check_visibility,
                     float4 *vmap_ext, long long vmap_pitch, const int *layouts, cudaStream_t st,
                     uint8_t *rgb_ext = nullptr, long long rgb_pitch = 0);
-// the z-range pass, its grid cleared before (launch_alloc_visible, launch_raycast)
-void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
+// The z-range pass, its grid cleared before (launch_alloc, launch_raycast): of the visible
+// list, or making the list on its way -- the blocks in the frustum of the map pose, or
+// those and the ones that this fuse touched.
+enum class ZrangeOf { list, frustum, fuse };
+void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, ZrangeOf of, cudaStream_t st);
 void launch_march(const SessionView *d_sv, int nslots, const Extent &ex, float4 *vmap_ext, long long vmap_pitch,
                   const int *layouts, cudaStream_t st, uint8_t *rgb_ext = nullptr, long long rgb_pitch = 0);
 // computeNMapK (cuda_imgproc.cu:276-305) of a pitched vertex map into a pitched normal map

@@ -7,13 +7,14 @@
 //               integration test and weight; a System frame has them from its ingest.
 //   alloc       one thread per level-0 pixel walks the blocks of its truncation
 //               band (3-D Bresenham, depth_fusion.cu:121-228); the CTA dedupes
-//               the keys of its 16x16 pixel tile in a shared-memory set and each
+//               the keys of its pixel tile in a shared-memory set and each
 //               unique key is inserted once into the session's open-addressing
 //               table with a 64-bit CAS (lock-free, no dropped blocks), stamping
 //               the block with the fuse counter.
-//   visible     one thread per ALLOCATED block (not per table slot): visible =
-//               stamped this fuse OR a block corner projects into the image
-//               within [zmin, zmax] (is_block_visible, depth_fusion.cu:15-47);
+//   visible     (gbf_fuse; a frame has the list from its z-range pass) one thread
+//               per ALLOCATED block (not per table slot): visible = stamped this
+//               fuse OR a block corner projects into the image within
+//               [zmin, zmax] (is_block_visible, depth_fusion.cu:15-47);
 //               warp-aggregated append to the visible list.
 //   integrate   one CTA per visible block (grid-stride), 4 voxels per thread,
 //               coalesced SoA voxel read-modify-write; blocks allocated this
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(kAllocThreads) alloc_kernel(const SessionView 
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     const int W = sv.lv[0].w, H = sv.lv[0].h;
+    clear_zrange(sv, blockIdx.x * kAllocThreads + threadIdx.x, gridDim.x * kAllocThreads);
     const int tiles_x = (W + 31) / 32;
     const int x = (blockIdx.x % tiles_x) * 32 + (threadIdx.x & 31), y0 = (blockIdx.x / tiles_x) * (8 * ROWS);
     if (y0 >= H) return;  // uniform per CTA
@@ -219,10 +221,8 @@ __device__ __forceinline__ bool block_in_frustum(const SessionView &sv, const M3
     return false;
 }
 
-// TOUCHED: also count blocks stamped by this fuse (check_visibility_flag_kernel's
-// flag 2), and clear the z-range grid of the raycast that follows; without it, the frustum test alone (count_visible_entry,
-// ray_tracing.cu:778-807 with VisibleEntryEvaluateFunctor, :681-710).
-template <bool TOUCHED>
+// The visible blocks of a fuse without a raycast behind it (a frame makes its list with
+// the raycast's z-range, zrange_kernel).
 __global__ void __launch_bounds__(256, 6) visible_kernel(const SessionView *svs) {
     chain_begin();
     const SessionView &sv = svs[blockIdx.y];
@@ -230,7 +230,6 @@ __global__ void __launch_bounds__(256, 6) visible_kernel(const SessionView *svs)
     __shared__ M34 Tcw;
     if (threadIdx.x == 0) Tcw = load_m34(sv.ts->map_tcw);
     __syncthreads();
-    if (TOUCHED) clear_zrange(sv, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     const int frame = sv.ctr[C_FRAME] + 1;
     const int n = min(sv.ctr[C_NUSED], sv.pool);
     const int stride = gridDim.x * blockDim.x;
@@ -241,7 +240,7 @@ __global__ void __launch_bounds__(256, 6) visible_kernel(const SessionView *svs)
         int tag = 0;
         if (id < n) {
             const int4 c = sv.bcoord[id];
-            vis = (TOUCHED && sv.bstamp[id] == frame) || block_in_frustum(sv, Tcw, c.x, c.y, c.z);
+            vis = sv.bstamp[id] == frame || block_in_frustum(sv, Tcw, c.x, c.y, c.z);
             tag = sv.bfresh[id] ? (int)0x80000000 : 0;
         }
         const int pos = warp_append(sv.ctr + C_NVIS, vis);
@@ -362,7 +361,7 @@ void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImp
 // without launching a CTA per 256 pool slots
 constexpr int kVisCtas = 152;
 
-void launch_alloc_visible(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
+void launch_alloc(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
     // Rows of a thread: one where the image's CTAs then still start at once (8 per SM),
     // two up to four rounds of them, four beyond, where a block that several tiles see
     // costs more than the length of a CTA.  Allocation and visible pass in us with 1, 2, 4
@@ -375,13 +374,6 @@ void launch_alloc_visible(const SessionView *d_sv, int nslots, const Extent &ex,
     if (ctas <= 8 * 152) alloc(alloc_kernel<1>, 1);
     else if (ctas <= 4 * 8 * 152) alloc(alloc_kernel<2>, 2);
     else alloc(alloc_kernel<4>, 4);
-    const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
-    launch_kernel(visible_kernel<true>, dim3(gv, nslots), 256, ex.chain, st, d_sv);
-}
-
-void launch_visible_frustum(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
-    const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
-    launch_kernel(visible_kernel<false>, dim3(gv, nslots), 256, ex.chain, st, d_sv);
 }
 
 void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st) {
@@ -398,7 +390,9 @@ void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, con
 }
 
 void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st) {
-    launch_alloc_visible(d_sv, nslots, ex, st);
+    launch_alloc(d_sv, nslots, ex, st);
+    const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
+    launch_kernel(visible_kernel, dim3(gv, nslots), 256, ex.chain, st, d_sv);
     launch_integrate(d_sv, nslots, ex, layouts, st);
 }
 

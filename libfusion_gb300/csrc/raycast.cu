@@ -5,8 +5,8 @@
 // GB300 design:
 //   begin     (raycast calls) the pose, the z-range grid (H/8 x W/8) to (100, 0); a
 //             System frame has its pose from tracking and the grid cleared by the
-//             visible-block pass.
-//   zrange    eight lanes per visible block: the block's screen box on the 1/8
+//             allocation.
+//   zrange    eight lanes per block: a visible block's screen box on the 1/8
 //             grid and its depth interval (create_rendering_block, :63-126), then
 //             integer atomicMin / atomicMax on the float bit patterns (all values
 //             are positive) of every covered cell.  The reference's 16x16
@@ -14,7 +14,8 @@
 //             (:223-277) are gone; the union of its tiles is exactly the box.
 //             In the same launch every allocated block marks the depth slices of
 //             the cells that rays may meet it in, and gets the ids of its
-//             neighbours at +x, +y, +z.
+//             neighbours at +x, +y, +z; a frame, and a raycast with visibility of
+//             its own, make the visible list there too, before the integration.
 //   raycast   one thread per pixel, 64-pixel CTAs (8x8 by default: a warp is
 //             an 8x4 patch of one z-range cell);
 //             the march of MapRenderingDelegate::operator() (:346-425), passing
@@ -27,10 +28,10 @@
 //             rays, some 250 steps of 0.5 us.  The slices are the same for all lanes of a
 //             warp, so skipping them keeps the warp together, where skipping by
 //             the unallocated block a ray is in (each lane its own) measured slower.
-//             640x480, march: 64 sessions 4.10 -> 2.72 ms per tick (slices 3.60,
-//             shorter sample code 3.34, neighbour lists 2.72), one 0.193 -> 0.134;
-//             the z-range launch, slices and lists included, takes 0.22 and 0.018 ms
-//             (0.18 and 0.018 without them and with a thread per block; 0.31 and 0.028 with).
+//             640x480, march: 64 sessions 4.10 -> 2.57 ms per tick (slices 3.60,
+//             shorter sample code 3.34, neighbour lists 2.72, one interpolation path
+//             per warp 2.57), one 0.193 -> 0.130; allocation, visible list, z-range,
+//             slices and neighbours together 0.61 -> 0.47 and 0.040 -> 0.028 ms.
 //   post      2x2 mean vertex pyramid, then normals of every level.
 #include "gbf_device.cuh"
 #include "gbf_kernels.h"
@@ -44,7 +45,7 @@ __global__ void ray_begin_kernel(const SessionView *__restrict__ svs, MapPose po
     chain_begin();
     const SessionView &sv = svs[0];
     if (blockIdx.x == 0 && threadIdx.x < 32) store_map_pose(sv.ts, pose);
-    if (check_visibility && blockIdx.x == 0 && threadIdx.x == 32) sv.ctr[C_NVIS] = 0;  // counted again by visible_kernel
+    if (check_visibility && blockIdx.x == 0 && threadIdx.x == 32) sv.ctr[C_NVIS] = 0;  // counted again by zrange_kernel
     clear_zrange(sv, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
@@ -117,11 +118,78 @@ __device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tc
     return true;
 }
 
+// A block's corner `c` in the camera frame and where it projects.
+struct Corner {
+    float3 p;
+    float u, v;
+};
+__device__ __forceinline__ Corner block_corner(const SessionView &sv, const M34 &Tcw, const int4 bc, int c) {
+    const LevelK &K = sv.lv[0];
+    const int cx = bc.x + (c & 1), cy = bc.y + ((c >> 1) & 1), cz = bc.z + (c >> 2);
+    Corner k;
+    k.p = Tcw.apply((float)cx * sv.block_metric, (float)cy * sv.block_metric, (float)cz * sv.block_metric);
+    k.u = (K.fx * k.p.x) / k.p.z + K.cx;
+    k.v = (K.fy * k.p.y) / k.p.z + K.cy;
+    return k;
+}
+
+// create_rendering_block (ray_tracing.cu:63-126) by eight lanes with a corner each, four
+// blocks a warp (all lanes call): the block's screen box and depth interval into the grid.
+__device__ __forceinline__ void mark_zrange(const SessionView &sv, const Corner &k, bool visible) {
+    const float u = k.u / 8.0f, v = k.v / 8.0f;
+    // the reference's running bounds from (zr_w, zr_h, -1, -1): a NaN coordinate changes none
+    const float fu = floorf(u), fv = floorf(v), cu = ceilf(u), cv = ceilf(v);
+    int ulx = (float)sv.zr_w > fu ? __float2int_rz(fu) : sv.zr_w, lrx = -1.f < cu ? __float2int_rz(cu) : -1;
+    int uly = (float)sv.zr_h > fv ? __float2int_rz(fv) : sv.zr_h, lry = -1.f < cv ? __float2int_rz(cv) : -1;
+    float zx = sv.zmax_r > k.p.z ? k.p.z : sv.zmax_r, zy = sv.zmin_r < k.p.z ? k.p.z : sv.zmin_r;
+#pragma unroll
+    for (int m = 1; m < 8; m <<= 1) {
+        ulx = min(ulx, __shfl_xor_sync(0xffffffffu, ulx, m));
+        uly = min(uly, __shfl_xor_sync(0xffffffffu, uly, m));
+        lrx = max(lrx, __shfl_xor_sync(0xffffffffu, lrx, m));
+        lry = max(lry, __shfl_xor_sync(0xffffffffu, lry, m));
+        const float x = __shfl_xor_sync(0xffffffffu, zx, m), y = __shfl_xor_sync(0xffffffffu, zy, m);
+        zx = fminf(zx, x);
+        zy = fmaxf(zy, y);
+    }
+    ulx = max(ulx, 0);
+    uly = max(uly, 0);
+    lrx = min(lrx, sv.zr_w - 1);
+    lry = min(lry, sv.zr_h - 1);
+    zx = fmaxf(zx, sv.zmin_r);
+    const bool renders = visible && ulx <= lrx && uly <= lry;  // (zy is never below zmin)
+    const unsigned n = __ballot_sync(0xffffffffu, renders && (threadIdx.x & 7) == 0);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(sv.ctr + C_RENDER, __popc(n));
+    if (renders) {
+        const int ix = __float_as_int(zx), iy = __float_as_int(zy);
+        for_cells(ulx, uly, lrx, lry, [&](int x, int y) {
+            atomicMin(reinterpret_cast<int *>(sv.zr_min) + y * sv.zr_w + x, ix);
+            atomicMax(reinterpret_cast<int *>(sv.zr_max) + y * sv.zr_w + x, iy);
+        });
+    }
+    __syncwarp();
+}
+
+// The slices of an allocated block and, where rays may meet it, its neighbours' ids.
+__device__ __forceinline__ void mark_block(const SessionView &sv, const M34 &Tcw, float margin, const int4 bc, int id) {
+    const int c = threadIdx.x & 7;
+    if (mark_slices(sv, Tcw, margin, bc))
+        sv.bnext[(size_t)id * 8 + c] =
+            c == 0 ? id : find_block(sv, bc.x + (c & 1), bc.y + ((c >> 1) & 1), bc.z + (c >> 2));
+}
+
 // Eight lanes to a block, a corner, a share of the cells and a neighbour each:
 // a session has some 20,000 blocks, which a thread each would leave to 600 warps
-// of long loops.  The first half of the CTAs takes the visible blocks (z-range),
-// the second the allocated ones (slices, and the neighbour lists of the blocks
-// that rays may meet).
+// of long loops.  LIST: the visible blocks are those of the list (a raycast after a
+// fuse, from a pose of its own); the first half of the CTAs takes them, the second the
+// allocated ones.  Otherwise the pass makes the list on its way, from every allocated
+// block's corners, which are the ones the z-range projects (a visible pass ahead of
+// this one took 7 us per 640x480 frame and 14 in a large map, a thread per block
+// projecting its eight corners one after the other): visible = a corner in the image
+// within [zmin, zmax] (is_block_visible, depth_fusion.cu:15-47; a raycast's own
+// visibility, ray_tracing.cu:681-807) or, with TOUCHED, stamped by this fuse
+// (check_visibility_flag_kernel's flag 2).
+template <bool LIST, bool TOUCHED>
 __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__restrict__ svs) {
     chain_begin();
     const SessionView &sv = svs[blockIdx.y];
@@ -131,57 +199,38 @@ __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__res
     if (threadIdx.x < 12) Tcw.m[threadIdx.x] = sv.ts->map_tcw[threadIdx.x];
     if (threadIdx.x == 32) margin = ray_margin(sv);
     __syncthreads();
-    const int half = gridDim.x / 2, c = threadIdx.x & 7, per_cta = blockDim.x / 8, stride = half * per_cta;
-    if (blockIdx.x >= half) {
-        const int used = min(sv.ctr[C_NUSED], sv.pool);
-        for (int id = (blockIdx.x - half) * per_cta + threadIdx.x / 8; id < used; id += stride) {
-            const int4 bc = sv.bcoord[id];
-            if (!mark_slices(sv, Tcw, margin, bc)) continue;
-            sv.bnext[(size_t)id * 8 + c] =
-                c == 0 ? id : find_block(sv, bc.x + (c & 1), bc.y + ((c >> 1) & 1), bc.z + (c >> 2));
+    const int c = threadIdx.x & 7, per_cta = blockDim.x / 8, lists = LIST ? gridDim.x / 2 : 0;
+    const int used = min(sv.ctr[C_NUSED], sv.pool);
+    if (LIST && blockIdx.x < lists) {
+        const int nvis = sv.ctr[C_NVIS];
+        // whole warps iterate together: the corners meet by shuffles
+        for (int base = blockIdx.x * per_cta + (threadIdx.x & ~31) / 8; base < nvis; base += lists * per_cta) {
+            const int b = base + ((threadIdx.x & 31) >> 3);
+            const int4 bc = sv.bcoord[sv.vis[min(b, nvis - 1)] & 0x7fffffff];
+            mark_zrange(sv, block_corner(sv, Tcw, bc, c), b < nvis);
         }
         return;
     }
-    const int nvis = sv.ctr[C_NVIS];
-    const LevelK &K = sv.lv[0];
-    // whole warps iterate together: the corners meet by shuffles
-    for (int base = blockIdx.x * per_cta + (threadIdx.x & ~31) / 8; base < nvis; base += stride) {
-        const int b = base + ((threadIdx.x & 31) >> 3);
-        const int id = sv.vis[min(b, nvis - 1)] & 0x7fffffff;
+    const int first = (blockIdx.x - lists) * per_cta, stride = (gridDim.x - lists) * per_cta;
+    if (LIST) {
+        for (int id = first + threadIdx.x / 8; id < used; id += stride) mark_block(sv, Tcw, margin, sv.bcoord[id], id);
+        return;
+    }
+    const int frame = sv.ctr[C_FRAME] + 1;
+    const float umax = (float)(sv.lv[0].w - 1), vmax = (float)(sv.lv[0].h - 1);
+    for (int base = first + (threadIdx.x & ~31) / 8; base < used; base += stride) {
+        const int b = base + ((threadIdx.x & 31) >> 3), id = min(b, used - 1);
         const int4 bc = sv.bcoord[id];
-        const int cx = bc.x + (c & 1), cy = bc.y + ((c >> 1) & 1), cz = bc.z + (c >> 2);
-        const float3 p = Tcw.apply((float)cx * sv.block_metric, (float)cy * sv.block_metric, (float)cz * sv.block_metric);
-        const float u = ((K.fx * p.x) / p.z + K.cx) / 8.0f;
-        const float v = ((K.fy * p.y) / p.z + K.cy) / 8.0f;
-        // the reference's running bounds from (zr_w, zr_h, -1, -1): a NaN coordinate changes none
-        const float fu = floorf(u), fv = floorf(v), cu = ceilf(u), cv = ceilf(v);
-        int ulx = (float)sv.zr_w > fu ? __float2int_rz(fu) : sv.zr_w, lrx = -1.f < cu ? __float2int_rz(cu) : -1;
-        int uly = (float)sv.zr_h > fv ? __float2int_rz(fv) : sv.zr_h, lry = -1.f < cv ? __float2int_rz(cv) : -1;
-        float zx = sv.zmax_r > p.z ? p.z : sv.zmax_r, zy = sv.zmin_r < p.z ? p.z : sv.zmin_r;
-#pragma unroll
-        for (int m = 1; m < 8; m <<= 1) {
-            ulx = min(ulx, __shfl_xor_sync(0xffffffffu, ulx, m));
-            uly = min(uly, __shfl_xor_sync(0xffffffffu, uly, m));
-            lrx = max(lrx, __shfl_xor_sync(0xffffffffu, lrx, m));
-            lry = max(lry, __shfl_xor_sync(0xffffffffu, lry, m));
-            const float x = __shfl_xor_sync(0xffffffffu, zx, m), y = __shfl_xor_sync(0xffffffffu, zy, m);
-            zx = fminf(zx, x);
-            zy = fmaxf(zy, y);
-        }
-        ulx = max(ulx, 0);
-        uly = max(uly, 0);
-        lrx = min(lrx, sv.zr_w - 1);
-        lry = min(lry, sv.zr_h - 1);
-        zx = fmaxf(zx, sv.zmin_r);
-        const bool renders = b < nvis && ulx <= lrx && uly <= lry;  // (zy is never below zmin)
-        const unsigned n = __ballot_sync(0xffffffffu, renders && c == 0);
-        if ((threadIdx.x & 31) == 0 && n) atomicAdd(sv.ctr + C_RENDER, __popc(n));
-        if (!renders) continue;
-        const int ix = __float_as_int(zx), iy = __float_as_int(zy);
-        for_cells(ulx, uly, lrx, lry, [&](int x, int y) {
-            atomicMin(reinterpret_cast<int *>(sv.zr_min) + y * sv.zr_w + x, ix);
-            atomicMax(reinterpret_cast<int *>(sv.zr_max) + y * sv.zr_w + x, iy);
-        });
+        const Corner k = block_corner(sv, Tcw, bc, c);
+        // is_vertex_visible: false comparisons (NaN) leave the corner in
+        const bool in = !(k.u < 0 || k.v < 0 || k.u > umax || k.v > vmax || k.p.z < sv.zmin_u || k.p.z > sv.zmax_u);
+        const unsigned corners = __ballot_sync(0xffffffffu, in) >> (threadIdx.x & 24) & 0xffu;
+        const bool visible = b < used && (corners || (TOUCHED && sv.bstamp[id] == frame));
+        const int pos = warp_append(sv.ctr + C_NVIS, visible && c == 0);
+        if (visible && c == 0) sv.vis[pos] = id | (sv.bfresh[id] ? (int)0x80000000 : 0);
+        mark_zrange(sv, k, visible);
+        if (b < used) mark_block(sv, Tcw, margin, bc, id);
+        __syncwarp();
     }
 }
 
@@ -612,10 +661,18 @@ __global__ void nmap_all_kernel(const SessionView *__restrict__ svs) {
 
 }  // namespace
 
-void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
-    // two halves of up to three resident CTAs per SM each; fewer of many sessions, whose CTAs loop
-    const int gz = min(max((ex.max_pool + 31) / 32, 1), max(152, 152 * 3 / nslots));
-    launch_kernel(zrange_kernel, dim3(2 * gz, nslots), 256, ex.chain, st, d_sv);
+// CTAs per session: up to three resident ones per SM, fewer of many sessions, whose CTAs loop
+static int zrange_ctas(const Extent &ex, int nslots) {
+    return min(max((ex.max_pool + 31) / 32, 1), max(152, 152 * 3 / nslots));
+}
+void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, ZrangeOf of, cudaStream_t st) {
+    const int n = zrange_ctas(ex, nslots);
+    const auto go = [&](auto *kernel, int halves) {
+        launch_kernel(kernel, dim3(n * halves, nslots), 256, ex.chain, st, d_sv);
+    };
+    if (of == ZrangeOf::list) go(zrange_kernel<true, false>, 2);
+    else if (of == ZrangeOf::frustum) go(zrange_kernel<false, false>, 2);
+    else go(zrange_kernel<false, true>, 2);
 }
 
 void launch_march(const SessionView *d_sv, int nslots, const Extent &ex, float4 *vmap_ext, long long vmap_pitch,
@@ -666,8 +723,7 @@ void launch_raycast(const SessionView *d_sv, const Extent &ex, const double pose
     for (int i = 0; i < 12; ++i) p.p[i] = pose[i];
     const int cells = (ex.w / 8) * (ex.h / 8);
     launch_kernel(ray_begin_kernel, (cells + 255) / 256, 256, ex.chain, st, d_sv, p, check_visibility ? 1 : 0);
-    if (check_visibility) launch_visible_frustum(d_sv, 1, ex, st);
-    launch_zrange(d_sv, 1, ex, st);
+    launch_zrange(d_sv, 1, ex, check_visibility ? ZrangeOf::frustum : ZrangeOf::list, st);
     launch_march(d_sv, 1, ex, vmap_ext, vmap_pitch, layouts, st, rgb_ext, rgb_pitch);
 }
 

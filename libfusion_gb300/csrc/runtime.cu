@@ -289,17 +289,17 @@ void enqueue_first_half(const SessionView *d_sv, int nslots, const Extent &ex, c
     mark(2, st);
 }
 
-// Second half: allocation, visibility, integration and the raycast that makes
-// the next frame's reference maps.
+// Second half: allocation, visibility (with the z-range of the raycast, at the same
+// pose), integration and the raycast that makes the next frame's reference maps.
 void enqueue_second_half(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st,
                          cudaEvent_t *ev = nullptr) {
     PhaseMarks mark(ev, st);
-    launch_alloc_visible(d_sv, nslots, ex, st);
+    launch_alloc(d_sv, nslots, ex, st);
+    launch_zrange(d_sv, nslots, ex, ZrangeOf::fuse, st);
     mark(3, st);
     launch_integrate(d_sv, nslots, ex, layouts, st);
     mark(4, st);
-    launch_zrange(d_sv, nslots, ex, st);
-    mark(5, st);
+    mark(5, st);  // (no launch of its own any more)
     launch_march(d_sv, nslots, ex, nullptr, 0, layouts, st);
     mark(6, st);
     launch_post(d_sv, nslots, ex, st);
@@ -316,7 +316,7 @@ void enqueue_frame(const SessionView *d_sv, int nslots, const Extent &ex, const 
 int kernels_per_frame(const Extent &ex, const int *layouts, int nslots, bool alone) {
     int nl = 0;
     for (int l = 0; l < kNumLayouts; ++l) nl += layouts[l];
-    return ingest_launches(ex) + track_launches(nslots, ex, alone) + 2 + nl + 1 + nl + post_launches(ex);
+    return ingest_launches(ex) + track_launches(nslots, ex, alone) + 2 + nl + nl + post_launches(ex);
 }
 
 }  // namespace
