@@ -29,6 +29,7 @@ constexpr int kCoarseReduceTile = 1024;
 constexpr int kReduceWidth = 58;        // 29 ICP + 29 RGB sums
 constexpr int kPartialStride = 64;      // floats per CTA partial record
 constexpr int kMeshChunks = 256;        // chunks of blocks of a mesh's offset scan, at most
+constexpr int kMeshWords = kMeshChunks + 1;  // their sums and the block counter of the emission
 
 // Open-addressing hash slot.  key packs the block position (21 bits per axis,
 // two's complement), ptr is the pool block id (-1 while unassigned).  The home
@@ -141,7 +142,7 @@ struct SessionView {
     float *partials;       // [red_ctas][kPartialStride]
     unsigned long long *track_rec;  // [red_ctas][kPartialStride] (gn_track_kernel)
     int *mesh_off;         // per-block triangle counts / offsets (pool + 1)
-    int *mesh_sums;        // triangles per chunk of blocks [kMeshChunks]
+    int *mesh_sums;        // triangles per chunk of blocks, block counter [kMeshWords]
 };
 
 }  // namespace gbf

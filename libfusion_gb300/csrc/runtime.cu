@@ -127,7 +127,7 @@ ArenaLayout plan_arena(const gbf_config &c, const gbf_intrinsics &K) {
     for (int l = 0, lw = K.width, lh = K.height; l < c.num_levels; ++l, lw /= 2, lh /= 2)
         max_ctas = std::max(max_ctas, (lw * lh + reduce_tile(l) - 1) / reduce_tile(l));
     a.partials = take((size_t)max_ctas * kPartialStride * 4);
-    a.mesh_sums = take(kMeshChunks * sizeof(int));
+    a.mesh_sums = take(kMeshWords * sizeof(int));
     a.track_rec = take((size_t)max_ctas * kPartialStride * 8);
     a.total = off;
     return a;
