@@ -906,39 +906,41 @@ __device__ __forceinline__ unsigned long long *record_word(const SessionView &sv
 }
 
 // The sums of the item numbered `number`, by all threads of CTA 0: warp g waits
-// for records g, g + 16, ... (a lane per record looks at its first word), then
-// lane q adds columns 2 q and 2 q + 1 of them in turn; the 16 groups follow in
+// for ten of the records g, g + 16, ... at a time (a lane per record looks at its first
+// word), then lane q adds columns 2 q and 2 q + 1 of them in turn; the 16 groups follow in
 // order (the sums and the order of sum_partials).  The words are read ten in
-// flight (ld_l2) and checked by their numbers.  Records past the last count as zeros, which add nothing.
+// flight (ld_l2) and checked by their numbers.  Only the records that come last are
+// then left to read when the last tile is done (waiting for thirty at a time, as many as fit
+// the lanes, left a 1280x720 image's whole second half).  Records past the last
+// count as zeros, which add nothing.
 static_assert(kTrackThreads == 32 * kSumGroups, "a warp per record group");
 __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv, int n, int number) {
     const int g = threadIdx.x >> 5, lane = threadIdx.x & 31, q = min(2 * lane, kReduceWidth - 2);
     WaitLimit limit;
     FSum s0, s1;
-    constexpr int kBatch = 10, kChunk = 3 * kBatch * kSumGroups;  // at most a record per lane
-    for (int first = g; first < n; first += kChunk) {
-        const int r = first + lane * kSumGroups, end = min(n, first + kChunk);
-        while (!__all_sync(0xffffffffu, r >= end || (int)(ld_relaxed(record_word(sv, r, 0)) >> 32) == number) &&
+    constexpr int kBatch = 10;  // at most a record per lane
+    for (int c = g; c < n; c += kBatch * kSumGroups) {
+        const int r = c + lane * kSumGroups;
+        const bool mine = lane < kBatch && r < n;
+        while (!__all_sync(0xffffffffu, !mine || (int)(ld_relaxed(record_word(sv, r, 0)) >> 32) == number) &&
                !__any_sync(0xffffffffu, limit.over())) {}
-        for (int c = first; c < end; c += kBatch * kSumGroups) {
-            ulonglong2 w[kBatch];
-            bool all, again = false;
-            do {
-                all = true;
-#pragma unroll
-                for (int i = 0; i < kBatch; ++i) {
-                    w[i] = make_ulonglong2(tagged(number, 0u), tagged(number, 0u));
-                    if (c + i * kSumGroups < end) w[i] = ld_l2(record_word(sv, c + i * kSumGroups, q), again);
-                }
-#pragma unroll
-                for (int i = 0; i < kBatch; ++i) all = all && (int)(w[i].x >> 32) == number && (int)(w[i].y >> 32) == number;
-                again = true;
-            } while (!__all_sync(0xffffffffu, all) && !__any_sync(0xffffffffu, limit.over()));
+        ulonglong2 w[kBatch];
+        bool all, again = false;
+        do {
+            all = true;
 #pragma unroll
             for (int i = 0; i < kBatch; ++i) {
-                s0.add(__uint_as_float((unsigned)w[i].x));
-                s1.add(__uint_as_float((unsigned)w[i].y));
+                w[i] = make_ulonglong2(tagged(number, 0u), tagged(number, 0u));
+                if (c + i * kSumGroups < n) w[i] = ld_l2(record_word(sv, c + i * kSumGroups, q), again);
             }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) all = all && (int)(w[i].x >> 32) == number && (int)(w[i].y >> 32) == number;
+            again = true;
+        } while (!__all_sync(0xffffffffu, all) && !__any_sync(0xffffffffu, limit.over()));
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+            s0.add(__uint_as_float((unsigned)w[i].x));
+            s1.add(__uint_as_float((unsigned)w[i].y));
         }
     }
     sm.grp[g][q] = make_float2(s0.s, s0.c);
