@@ -245,9 +245,9 @@ class ClockSampler:
 
 
 # DRAM bytes one pixel-iteration of the ICP + photometric reduction moves, from
-# one ncu capture of a level-0 launch over 4 sessions (105.50 MB for 1,228,800
+# one ncu capture of a level-0 launch over 4 sessions (105.09 MB for 1,228,800
 # pixel-iterations, dram__bytes_read.sum + dram__bytes_write.sum): the roofline's traffic
-REDUCE_DRAM_BYTES_PER_PIXEL_ITER = (102.178048e6 + 3.364608e6) / 1228800
+REDUCE_DRAM_BYTES_PER_PIXEL_ITER = (102.09664e6 + 2.995456e6) / 1228800
 # DRAM bytes per raycast pixel, from one ncu capture of the SNORM raycast over 4
 # sessions with maps of 96 fused frames (74.60 MB read + 7.67 MB written for
 # 4 x 307,200 pixels; same counters), and its issue-active fraction there.  The
@@ -736,7 +736,7 @@ def run_ours(args):
                 "launches_per_step": n_launch, "peak_source": f"{peak_kind} hbm_gbs",
                 "algorithmic_bytes_per_launch": bytes_step / n_launch, "algorithmic_bytes_per_step": bytes_step,
                 "traffic_basis": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a level-0 launch at 4 "
-                                 "sessions: 85.9 B per pixel-iteration, "
+                                 "sessions: 85.5 B per pixel-iteration, "
                                  "times this run's pixel-iterations per launch" if traffic is not None else None,
                 "work_per_step": {"pixel_iterations": pix_iter, "integrated_blocks": (ib1 - ib0) / phases["ticks"]},
                 "timing": f"CUDA events around the phase over {phases['ticks']} ticks on the launching stream",

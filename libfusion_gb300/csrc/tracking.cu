@@ -752,9 +752,10 @@ __global__ void track_finish_kernel(const SessionView *__restrict__ svs, int fra
 // memory weighs as much as the arithmetic).  CTA 0 makes no rows: it sums the tiles'
 // records as they arrive, takes the step on the tracking state in its shared memory and
 // publishes the next pose, so that the step's code stays in one SM's instruction cache.
-// An iteration then takes 10 us at 160x120 and 320x240 and 15 us at 640x480
-// (two tiles per CTA: 7 us; step 3.7; each hop between CTAs 0.7), the run of a
-// 640x480 frame 0.25 -> 0.16 ms.  1024 threads of 64 registers spilled (0.25 ms);
+// An iteration then takes 9 us at 320x240 and below, 13 at 640x480 and 24 at 1280x720
+// (one, two and six tiles per CTA of 2.4 us each: 1.5 the rows, 0.65 the chains; the step
+// 3.7; each hop between CTAs 0.7; the records 1 to 2), the run of a 640x480 frame 0.25
+// -> 0.15 ms.  1024 threads of 64 registers spilled (0.25 ms);
 // the step by whichever CTA came last ran 25% slower from cold instruction
 // caches; coarse tiles split over two or four CTAs cost more in records than they saved.
 //
