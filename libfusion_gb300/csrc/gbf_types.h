@@ -28,6 +28,7 @@ constexpr int kReducePixelsPerThread = 4;
 constexpr int kCoarseReduceTile = 1024;
 constexpr int kReduceWidth = 58;        // 29 ICP + 29 RGB sums
 constexpr int kPartialStride = 64;      // floats per CTA partial record
+constexpr float kListSdf = 1.01f;       // truncations that a raycast's neighbour lists reach before the near plane
 constexpr int kMeshChunks = 256;        // chunks of blocks of a mesh's offset scan, at most
 constexpr int kMeshWords = kMeshChunks + 1;  // their sums and the block counter of the emission
 
@@ -57,6 +58,7 @@ enum Counter {
     C_MESH_BLOCKS = 6,
     C_MESH_TRIS = 7,
     C_GC_DELETED = 8, // blocks deleted by the last garbage collection
+    C_DEEP_SDF = 9,   // 1 once a map with an sdf below -kListSdf has been imported
     C_COUNT = 16,     // counters proper (reported, kept by snapshots)
     C_TRACK_PUB = 16, // 14 8-byte words published within a tracking run (gn_track_kernel)
     C_WORDS = 64      // ints in the arena

@@ -86,7 +86,11 @@ __device__ __forceinline__ void for_cells(int x0, int y0, int x1, int y1, const 
     }
 }
 
-// False when no sample of a raycast at this pose can lie in the block.
+// Whether a sample of a raycast at this pose, or the refined one of a hit, can lie in
+// the block.  The refined sample lies before the one that found the hit by sdf x
+// truncation, and so up to kListSdf truncations before the near plane (a fused sdf is
+// never below -1; with an imported one that is, mark_block takes every block).  Only a
+// block that a marched sample can meet marks slices.
 __device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tcw, float margin, const int4 bc) {
     const LevelK &K = sv.lv[0];
     const float h = 0.5f * sv.block_metric;
@@ -97,7 +101,7 @@ __device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tc
     const float hy = h * (fabsf(Tcw.m[4]) + fabsf(Tcw.m[5]) + fabsf(Tcw.m[6])) + margin;
     const float hz = h * (fabsf(Tcw.m[8]) + fabsf(Tcw.m[9]) + fabsf(Tcw.m[10])) + margin;
     const float z0 = p.z - hz, z1 = p.z + hz;
-    if (!(z1 >= sv.zmin_r)) return false;
+    if (!(z1 >= sv.zmin_r - kListSdf * sv.tau)) return false;
     int cx0 = 0, cx1 = sv.zr_w - 1, cy0 = 0, cy1 = sv.zr_h - 1;
     if (z0 > 0.25f * sv.zmin_r) {
         const float i0 = 1.f / z0, i1 = 1.f / z1;
@@ -110,6 +114,7 @@ __device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tc
         cy0 = max(0, (int)(vl * 0.125f));
         cy1 = min(cy1, (int)(vh * 0.125f));
     }
+    if (!(z1 >= sv.zmin_r)) return true;
     const float scale = slice_scale(sv);
     const int s0 = min(max((int)((z0 - sv.zmin_r) * scale), 0), kSlices - 1);
     const int s1 = min((int)((z1 - sv.zmin_r) * scale), kSlices - 1);
@@ -171,9 +176,10 @@ __device__ __forceinline__ void mark_zrange(const SessionView &sv, const Corner 
 }
 
 // The slices of an allocated block and, where rays may meet it, its neighbours' ids.
-__device__ __forceinline__ void mark_block(const SessionView &sv, const M34 &Tcw, float margin, const int4 bc, int id) {
+__device__ __forceinline__ void mark_block(const SessionView &sv, const M34 &Tcw, float margin, bool deep, const int4 bc,
+                                           int id) {
     const int c = threadIdx.x & 7;
-    if (mark_slices(sv, Tcw, margin, bc))
+    if (mark_slices(sv, Tcw, margin, bc) || deep)
         sv.bnext[(size_t)id * 8 + c] =
             c == 0 ? id : find_block(sv, bc.x + (c & 1), bc.y + ((c >> 1) & 1), bc.z + (c >> 2));
 }
@@ -201,6 +207,7 @@ __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__res
     __syncthreads();
     const int c = threadIdx.x & 7, per_cta = blockDim.x / 8, lists = LIST ? gridDim.x / 2 : 0;
     const int used = min(sv.ctr[C_NUSED], sv.pool);
+    const bool deep = sv.ctr[C_DEEP_SDF] != 0;
     if (LIST && blockIdx.x < lists) {
         const int nvis = sv.ctr[C_NVIS];
         // whole warps iterate together: the corners meet by shuffles
@@ -213,7 +220,7 @@ __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__res
     }
     const int first = (blockIdx.x - lists) * per_cta, stride = (gridDim.x - lists) * per_cta;
     if (LIST) {
-        for (int id = first + threadIdx.x / 8; id < used; id += stride) mark_block(sv, Tcw, margin, sv.bcoord[id], id);
+        for (int id = first + threadIdx.x / 8; id < used; id += stride) mark_block(sv, Tcw, margin, deep, sv.bcoord[id], id);
         return;
     }
     const int frame = sv.ctr[C_FRAME] + 1;
@@ -229,7 +236,7 @@ __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__res
         const int pos = warp_append(sv.ctr + C_NVIS, visible && c == 0);
         if (visible && c == 0) sv.vis[pos] = id | (sv.bfresh[id] ? (int)0x80000000 : 0);
         mark_zrange(sv, k, visible);
-        if (b < used) mark_block(sv, Tcw, margin, bc, id);
+        if (b < used) mark_block(sv, Tcw, margin, deep, bc, id);
         __syncwarp();
     }
 }
@@ -270,7 +277,8 @@ __device__ __forceinline__ float trilinear(float fx, float fy, float fz, float c
 
 // The trilinear read when the corners span two to eight blocks (about 1/3 of
 // the reads): out of line, so that the march loop's code stays small.  i000:
-// the block of corner (x0, y0, z0), looked up by the caller.
+// the block of corner (x0, y0, z0), looked up by the caller; the others from its
+// neighbour list.
 template <int LAYOUT, class SV>
 __device__ __noinline__ float interp_spanning(const SV sv, int i000, int x0, int x1, int y0, int y1, int z0, int z1,
                                               float fx, float fy, float fz, bool &valid) {

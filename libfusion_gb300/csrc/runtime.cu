@@ -187,6 +187,7 @@ __global__ void import_kernel(const SessionView *__restrict__ svs, int count, co
             for (int i = threadIdx.x; i < kBlockVoxels; i += blockDim.x) {
                 const size_t o = (size_t)b * kBlockVoxels + i, vi = (size_t)id * kBlockVoxels + i;
                 store_sw<LAYOUT>(sv, vi, sdf[o], w[o]);
+                if (LAYOUT == GBF_VOXEL_HALF && sdf[o] < -kListSdf) sv.ctr[C_DEEP_SDF] = 1;  // others hold -1 and up
                 sv.vox_rgb[vi] = make_uchar4(rgb[o * 3], rgb[o * 3 + 1], rgb[o * 3 + 2], 0);
             }
             if (threadIdx.x == 0) sv.bfresh[id] = 0;

@@ -135,3 +135,79 @@ def test_raycast_skips_only_empty_space(gbf, voxel, zmin, far):
             assert np.array_equal(gh, oh) and np.array_equal(g[gh], o[oh])
             hits += int(gh.sum())
     assert hits > 5000
+
+
+@pytest.mark.parametrize("before", ["new", "pruned", "restored"])
+def test_raycast_refined_samples_before_the_near_plane(gbf, before):
+    """A wall three voxels nearer than zmin_raycast, a block face between the two: a ray's
+    first sample lies behind the wall and its refined one up to a truncation before
+    the near plane, in a block that no marched sample can meet.  Vertices and hit masks are
+    the oracle's on a new session's first raycast, after a prune that moved block
+    ids, and after a restore into an arena that held another map."""
+    import oracle as O
+    import torch
+    L = gbf
+    K = L.IntrinsicMatrix(168, 120, 110.0, 105.0, 80.3, 61.7)
+    cfg = H.small_config(L, 0, truncation=0.05, zmin_update=0.2, num_blocks=1 << 14, num_buckets=1 << 16)
+    rgb = np.full((K.height, K.width, 3), 99, np.uint8)
+    T = np.eye(4)
+    T[2, 3] = 0.035  # block faces at depths 0.205 and 0.285
+    aside, back = T.copy(), T.copy()
+    aside[0, 3] = 20.0
+    back[2, 3] -= 1.0
+    vmap = torch.empty((K.height, K.width, 4), dtype=torch.float32, device="cuda")
+
+    def fuse(m, z, P, n=3):
+        for _ in range(n):
+            m.update(torch.full((K.height, K.width), z, device="cuda"), H.cuda(rgb), P)
+    m = L.System(K, cfg)
+    if before == "pruned":
+        fuse(m, 1.5, aside)
+    fuse(m, 0.27, T)
+    om = _oracle_map(L, cfg, K)
+    for _ in range(3):
+        om.fuse(np.full((K.height, K.width), 0.27, np.float32), rgb, T)
+    if before == "pruned":
+        m.raycast_check_visibility(vmap, back)  # every block's neighbours, by the ids before
+        assert m.prune(center=[0, 0, 0], radius=5.0) > 100
+    if before == "restored":
+        snap = m.snapshot()
+        m = L.System(K, cfg)
+        fuse(m, 1.2, T)
+        m.raycast_check_visibility(vmap, T)
+        m.restore(snap)
+    for dz in (0.0, 0.003, -0.004):
+        P = T.copy()
+        P[2, 3] += dz
+        m.raycast_check_visibility(vmap, P)
+        g, o = vmap.cpu().numpy(), om.raycast_check_visibility(P)
+        gh, oh = ~np.isnan(g[..., 2]), ~np.isnan(o[..., 2])
+        assert oh.mean() > 0.8 and np.nanmax(o[..., 2]) < cfg.zmin_raycast
+        assert np.array_equal(gh, oh), f"hit masks differ in {np.sum(gh != oh)} pixels"
+        assert np.array_equal(g[gh], o[oh])
+
+
+def test_raycast_of_an_imported_map_beyond_the_truncation(gbf):
+    """An imported map may hold any sdf.  Four times the sdf at a quarter of the truncation
+    is the same surface: where a ray's first sample is not interpolated (sdf < -1/2) it is
+    refined to the same point, two truncations before the near plane, with the same
+    neighbours around it, whatever raycasts came before."""
+    import torch
+    L = gbf
+    K = L.IntrinsicMatrix(168, 120, 110.0, 105.0, 80.3, 61.7)
+    cfg = [H.small_config(L, L.VOXEL_HALF, truncation=t, zmin_update=0.2, num_blocks=1 << 14, num_buckets=1 << 16)
+           for t in (0.0625, 0.015625)]
+    rgb = np.full((K.height, K.width, 3), 99, np.uint8)
+    T = np.eye(4)
+    T[2, 3] = 0.035  # block faces at depths 0.205 and 0.285
+    a, b = (L.DenseMapping(K, c) for c in cfg)
+    a.update(torch.full((K.height, K.width), 0.259, device="cuda"), H.cuda(rgb), T)
+    coords, sdf, w, col = a.export()
+    b.import_blocks(coords, 4 * sdf, w, col)
+    out = [torch.empty((K.height, K.width, 4), dtype=torch.float32, device="cuda") for _ in range(2)]
+    for m, v in zip((a, b), out):
+        m.raycast_check_visibility(v, T)
+    g, h = (v.cpu().numpy() for v in out)
+    hit = ~np.isnan(g[..., 2])
+    assert hit.mean() > 0.8 and np.nanmax(g[..., 2]) < cfg[0].zmin_raycast
+    assert np.array_equal(g, h, equal_nan=True), f"differ in {np.sum(hit != ~np.isnan(h[..., 2]))} hits"
