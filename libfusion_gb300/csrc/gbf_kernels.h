@@ -68,8 +68,9 @@ struct FuseImport {
 void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImport &in, const double pose[12],
                         cudaStream_t st);
 void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st);
-// the blocks of the frame's surface; also clears the visible count and the z-range grid
-void launch_alloc(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
+// the blocks of the frame's surface; also clears the visible count and, for a z-range
+// pass that follows, its grid
+void launch_alloc(const SessionView *d_sv, int nslots, const Extent &ex, bool zrange_follows, cudaStream_t st);
 // Phong shading of camera-frame vertex / normal maps into RGBA8 (rgb NULL = untextured)
 void launch_render(const float4 *vmap, long long vmap_pitch, const float4 *nmap, long long nmap_pitch,
                    const uint8_t *rgb, long long rgb_pitch, int rgb_stride, int w, int h, uchar4 *out,

@@ -118,12 +118,13 @@ __device__ __forceinline__ int3 pixel_block(const SessionView &sv, const M34 &T,
 // now it is the pixels' own arithmetic (64 sessions of 640x480, with the visible pass: 489
 // -> 408 us entry read first, 353 two rows a thread, 302 four, 276 with the list).
 template <int ROWS>
-__global__ void __launch_bounds__(kAllocThreads) alloc_kernel(const SessionView *svs) {
+__global__ void __launch_bounds__(kAllocThreads) alloc_kernel(const SessionView *svs, int zrange_follows) {
     chain_begin();
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     const int W = sv.lv[0].w, H = sv.lv[0].h;
-    clear_zrange(sv, blockIdx.x * kAllocThreads + threadIdx.x, gridDim.x * kAllocThreads);
+    // a frame's z-range pass comes next; an update alone leaves the last raycast's grid and count
+    if (zrange_follows) clear_zrange(sv, blockIdx.x * kAllocThreads + threadIdx.x, gridDim.x * kAllocThreads);
     const int tiles_x = (W + 31) / 32;
     const int x = (blockIdx.x % tiles_x) * 32 + (threadIdx.x & 31), y0 = (blockIdx.x / tiles_x) * (8 * ROWS);
     if (y0 >= H) return;  // uniform per CTA
@@ -361,14 +362,14 @@ void launch_fuse_import(const SessionView *d_sv, const Extent &ex, const FuseImp
 // without launching a CTA per 256 pool slots
 constexpr int kVisCtas = 152;
 
-void launch_alloc(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
+void launch_alloc(const SessionView *d_sv, int nslots, const Extent &ex, bool zrange_follows, cudaStream_t st) {
     // Rows of a thread: one where the image's CTAs then still start at once (8 per SM),
     // two up to four rounds of them, four beyond, where a block that several tiles see
     // costs more than the length of a CTA.  Allocation and visible pass in us with 1, 2, 4
     // rows: one 640x480 session 19.8, 20.4, 24.4; four 34.6, 32.8, 34.7; 64: 338, 300, 276.
     const auto alloc = [&](auto *kernel, int rows) {
         const dim3 g(((ex.w + 31) / 32) * ((ex.h + 8 * rows - 1) / (8 * rows)), nslots);
-        launch_kernel(kernel, g, kAllocThreads, ex.chain, st, d_sv);
+        launch_kernel(kernel, g, kAllocThreads, ex.chain, st, d_sv, zrange_follows ? 1 : 0);
     };
     const long long ctas = (long long)ex.w * ex.h / kAllocThreads * nslots;
     if (ctas <= 8 * 152) alloc(alloc_kernel<1>, 1);
@@ -390,7 +391,7 @@ void launch_integrate(const SessionView *d_sv, int nslots, const Extent &ex, con
 }
 
 void launch_fuse(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st) {
-    launch_alloc(d_sv, nslots, ex, st);
+    launch_alloc(d_sv, nslots, ex, false, st);
     const int gv = min(max((ex.max_pool + 255) / 256, 1), kVisCtas);
     launch_kernel(visible_kernel, dim3(gv, nslots), 256, ex.chain, st, d_sv);
     launch_integrate(d_sv, nslots, ex, layouts, st);

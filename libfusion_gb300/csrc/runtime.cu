@@ -295,7 +295,7 @@ void enqueue_first_half(const SessionView *d_sv, int nslots, const Extent &ex, c
 void enqueue_second_half(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st,
                          cudaEvent_t *ev = nullptr) {
     PhaseMarks mark(ev, st);
-    launch_alloc(d_sv, nslots, ex, st);
+    launch_alloc(d_sv, nslots, ex, true, st);
     launch_zrange(d_sv, nslots, ex, ZrangeOf::fuse, st);
     mark(3, st);
     launch_integrate(d_sv, nslots, ex, layouts, st);

@@ -211,3 +211,20 @@ def test_raycast_of_an_imported_map_beyond_the_truncation(gbf):
     hit = ~np.isnan(g[..., 2])
     assert hit.mean() > 0.8 and np.nanmax(g[..., 2]) < cfg[0].zmin_raycast
     assert np.array_equal(g, h, equal_nan=True), f"differ in {np.sum(hit != ~np.isnan(h[..., 2]))} hits"
+
+
+def test_update_keeps_the_last_raycasts_zrange(gbf):
+    """The z-range grid and the renderable count are the last raycast's until the next one:
+    an update in between makes neither."""
+    import torch
+    L = gbf
+    K = H.intrinsics(L)
+    m = L.DenseMapping(K, H.small_config(L, 2))
+    fr = H.frames(L, K, 2, step=10)
+    vmap = torch.empty((K.height, K.width, 4), dtype=torch.float32, device="cuda")
+    m.update(H.cuda(H.depth_m(fr[0][0])), H.cuda(fr[0][1]), fr[0][2])
+    m.raycast(vmap, fr[0][2])
+    grid, count = m.zrange(), m.stats().render_blocks_valid
+    assert count > 100 and grid.max() > 0.3
+    m.update(H.cuda(H.depth_m(fr[1][0])), H.cuda(fr[1][1]), fr[1][2])
+    assert m.stats().render_blocks_valid == count and np.array_equal(m.zrange(), grid)
