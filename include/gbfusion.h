@@ -434,9 +434,11 @@ typedef struct gbf_slot_result {
  * waits for that tick, then copies min(n, slots) records.  Reading tick k-1
  * after submitting tick k keeps the device busy while the host reads. */
 GBF_API gbf_status gbf_batch_results(gbf_batch *b, int32_t back, gbf_slot_result *out, int32_t n);
-/* Concurrent session groups per tick (1..4, default 2): the slots are split
- * into contiguous groups whose frames run as parallel branches of the tick
- * (graph branches / forked streams).  Results do not depend on it. */
+/* Concurrent session groups per tick (1..4): the slots are split into contiguous
+ * groups whose frames run as parallel branches of the tick (graph branches /
+ * forked streams).  Until it is called, or the tuner chooses: 1 for up to 4 slots,
+ * and for up to 16 of small images (1000 level-0 tiles of 1024 pixels together),
+ * which then track in one launch; 2 for more, and while staggered.  Results do not depend on it. */
 GBF_API gbf_status gbf_batch_set_groups(gbf_batch *b, int32_t groups);
 /* Staggered groups (default off; with 2+ groups): the odd groups run half a
  * frame out of phase -- each tick they fuse and raycast their previous frame,

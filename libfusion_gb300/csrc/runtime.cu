@@ -1591,7 +1591,7 @@ GBF_API gbf_status gbf_batch_tuning(gbf_batch *b, gbf_tuning *out) {
     memset(out, 0, sizeof(*out));
     out->state = b->tune_on ? b->tune_state : 0;
     out->from_table = b->tune_on && b->tune_state == 2 ? b->tune_cached : 0;
-    out->chosen.groups = b->groups;
+    out->chosen.groups = b->groups_set ? b->groups : tick_groups(b);
     out->chosen.stagger = b->stagger;
     out->chosen.ray_tile_w = b->ray_tw;
     out->chosen.median_ms = 0.f;

@@ -975,3 +975,29 @@ def test_tracking_runs_on_concurrent_streams(gbf):
         assert np.array_equal(more[i].get_camera_pose(), alone[i]), i
         assert ss[i].stats().status == 0 and more[i].stats().status == 0
     batch.close()
+
+
+def test_tuning_reports_the_groups_in_use(gbf):
+    """Where neither the caller nor the tuner has set the groups, gbf_batch_tuning reports
+    what the ticks run with: one branch for few sessions, two for more or while
+    staggered; and then what was set."""
+    L = gbf
+    K = H.intrinsics(L, 640, 480)
+    cfg = H.small_config(L, 2, num_blocks=1 << 10, num_buckets=1 << 12)
+    batch = L.FusionBatch(5)
+    ss, kernels = [L.System(K, cfg) for _ in range(5)], []
+    for i in range(5):
+        batch.set(i, ss[i])
+        groups = batch.tuning()["chosen"]["groups"]
+        assert groups == (1 if i < 4 else 2), i
+        kernels.append(batch.kernels_per_tick())
+        if i == 3:
+            batch.set_stagger(True)
+            assert batch.tuning()["chosen"]["groups"] == 2
+            batch.set_stagger(False)
+    assert len(set(kernels[:4])) == 1 and kernels[4] > 2 * kernels[0]
+    batch.set_groups(1)
+    assert batch.tuning()["chosen"]["groups"] == 1
+    batch.set_groups(3)
+    assert batch.tuning()["chosen"]["groups"] == 3
+    batch.close()
