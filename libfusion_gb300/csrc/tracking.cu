@@ -774,7 +774,8 @@ struct TrackSmem {
     TrackState ts;  // CTA 0: the run's tracking state
     float pose[12];
     float stddev, huber;
-    int item, seen, lost;
+    unsigned seen;
+    int item, lost;
 };
 
 // icp_row and rgb_row of one pixel, with their gathers issued together (a row
@@ -889,11 +890,13 @@ __device__ __forceinline__ void st_relaxed(unsigned long long *p, unsigned long 
 // second round trip, and leaves the readers' L1, with the maps they gather from,
 // alone.  CTA 0 publishes 14 of them after each step -- the estimate's 12 floats, the
 // photometric deviation and the work item; the others write the sums of their
-// tile, numbered like the publication that will follow.
+// tile, numbered like the publication that will follow.  The numbers run on over the
+// session's runs and wrap: one is newer by the sign of the difference.
 constexpr int kPubWords = 14;
-__device__ __forceinline__ unsigned long long tagged(int number, unsigned value) {
-    return ((unsigned long long)(unsigned)number << 32) | value;
+__device__ __forceinline__ unsigned long long tagged(unsigned number, unsigned value) {
+    return ((unsigned long long)number << 32) | value;
 }
+__device__ __forceinline__ unsigned number_of(unsigned long long word) { return (unsigned)(word >> 32); }
 
 // A run's work items are (level, iteration) packed; 0 is its end.
 __device__ __forceinline__ int first_item(const SessionView &sv, int level) {
@@ -915,7 +918,7 @@ __device__ __forceinline__ unsigned long long *record_word(const SessionView &sv
 // the lanes, left a 1280x720 image's whole second half).  Records past the last
 // count as zeros, which add nothing.
 static_assert(kTrackThreads == 32 * kSumGroups, "a warp per record group");
-__device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv, int n, int number) {
+__device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv, int n, unsigned number) {
     const int g = threadIdx.x >> 5, lane = threadIdx.x & 31, q = min(2 * lane, kReduceWidth - 2);
     WaitLimit limit;
     FSum s0, s1;
@@ -923,7 +926,7 @@ __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv
     for (int c = g; c < n; c += kBatch * kSumGroups) {
         const int r = c + lane * kSumGroups;
         const bool mine = lane < kBatch && r < n;
-        while (!__all_sync(0xffffffffu, !mine || (int)(ld_relaxed(record_word(sv, r, 0)) >> 32) == number) &&
+        while (!__all_sync(0xffffffffu, !mine || number_of(ld_relaxed(record_word(sv, r, 0))) == number) &&
                !__any_sync(0xffffffffu, limit.over())) {}
         ulonglong2 w[kBatch];
         bool all, again = false;
@@ -935,7 +938,7 @@ __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv
                 if (c + i * kSumGroups < n) w[i] = ld_l2(record_word(sv, c + i * kSumGroups, q), again);
             }
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) all = all && (int)(w[i].x >> 32) == number && (int)(w[i].y >> 32) == number;
+            for (int i = 0; i < kBatch; ++i) all = all && number_of(w[i].x) == number && number_of(w[i].y) == number;
             again = true;
         } while (!__all_sync(0xffffffffu, all) && !__any_sync(0xffffffffu, limit.over()));
 #pragma unroll
@@ -965,13 +968,13 @@ __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv
 
 // The newest publication after number `seen`, by one warp: lanes < 14 get the
 // values.  False when the wait ran out.
-__device__ __forceinline__ bool read_pub(const unsigned long long *pub, int &seen, unsigned &value) {
+__device__ __forceinline__ bool read_pub(const unsigned long long *pub, unsigned &seen, unsigned &value) {
     const int lane = threadIdx.x & 31;
     WaitLimit limit;
     for (;;) {
         const unsigned long long w = lane < kPubWords ? ld_relaxed(pub + lane) : 0ull;
-        const int n = (int)(w >> 32), n0 = __shfl_sync(0xffffffffu, n, 0);
-        if (__all_sync(0xffffffffu, lane >= kPubWords || n == n0) && n0 - seen > 0) {
+        const unsigned n = number_of(w), n0 = __shfl_sync(0xffffffffu, n, 0);
+        if (__all_sync(0xffffffffu, lane >= kPubWords || n == n0) && (int)(n0 - seen) > 0) {
             seen = n0;
             value = (unsigned)w;
             return true;
@@ -982,7 +985,7 @@ __device__ __forceinline__ bool read_pub(const unsigned long long *pub, int &see
 
 // The steps of a run: CTA 0 adds each item's records, takes the step on the
 // tracking state in shared memory and publishes what follows.
-__device__ __forceinline__ void track_steps(TrackSmem &sm, const SessionView &sv, int item, int seen, bool lost,
+__device__ __forceinline__ void track_steps(TrackSmem &sm, const SessionView &sv, int item, unsigned seen, bool lost,
                                             int frame_mode) {
     TrackState *ts = &sm.ts;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -1020,7 +1023,7 @@ __device__ __forceinline__ void track_steps(TrackSmem &sm, const SessionView &sv
 }
 
 // The tiles of a run: CTA cta of the ctas that follow CTA 0 makes its tiles' records of each item.
-__device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv, int item, int seen, int rs, int cta,
+__device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv, int item, unsigned seen, int rs, int cta,
                                             int ctas) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned long long *pub = reinterpret_cast<const unsigned long long *>(sv.ctr + C_TRACK_PUB);
@@ -1116,7 +1119,7 @@ __global__ void __launch_bounds__(kTrackThreads, 1)
     // Every CTA reads these before it arrives, and CTA 0 goes on once all have:
     // what it publishes, and the frame's end, change them.
     const int rs = sv.ts->idx;
-    const int seen = (int)(ld_relaxed(reinterpret_cast<const unsigned long long *>(sv.ctr + C_TRACK_PUB)) >> 32);
+    const unsigned seen = number_of(ld_relaxed(reinterpret_cast<const unsigned long long *>(sv.ctr + C_TRACK_PUB)));
     const int item = frame_mode && !sv.ts->has_ref ? 0 : first_item(sv, sv.levels - 1);
     if (tid < 12) sm.pose[tid] = (float)sv.ts->init[tid];
     if (tid == 12) sm.stddev = sm.huber = 0.f;

@@ -1,0 +1,91 @@
+// Drives sessions through the C API and reaches into one's arena for what no
+// caller can set: the numbers of the tracking run's words (csrc/tracking.cu).
+// Prints what differs and returns 1, or returns 0.
+#include <cstdio>
+#include <cstring>
+#include <vector>
+
+#include "../libfusion_gb300/csrc/gbf_internal.h"
+
+using namespace gbf;
+
+#define OK(call)                                                    \
+    do {                                                            \
+        if ((call) != 0) {                                          \
+            printf("%s: %s\n", #call, gbf_last_error());            \
+            return 1;                                               \
+        }                                                           \
+    } while (0)
+
+constexpr int kW = 320, kH = 240;
+
+struct Frames {
+    gbf_synth_scene *sc = nullptr;
+    gbf_intrinsics K{};
+    uint16_t *depth = nullptr;
+    uint8_t *rgb = nullptr;
+    int open() {
+        gbf_synth_params p;
+        OK(gbf_synth_default(&p));
+        OK(gbf_synth_create(&p, &sc));
+        K.width = kW;
+        K.height = kH;
+        K.fx = K.fy = 262.5f;
+        K.cx = 159.5f;
+        K.cy = 119.5f;
+        OK(cudaMalloc(&depth, kW * kH * 2));
+        OK(cudaMalloc(&rgb, kW * kH * 3));
+        return 0;
+    }
+    int render(int k) {
+        double T[16];
+        OK(gbf_synth_pose(sc, k, T));
+        OK(gbf_synth_render(sc, &K, T, k, depth, rgb, nullptr));
+        return 0;
+    }
+    int session(gbf_session **s) {
+        gbf_config c;
+        OK(gbf_config_default(&c));
+        c.zmax_update = c.zmax_raycast = 4.f;
+        c.num_buckets = 1 << 16;
+        c.num_blocks = 1 << 14;
+        OK(gbf_session_create(&c, &K, s));
+        double T[16];
+        OK(gbf_synth_pose(sc, 0, T));
+        OK(gbf_set_pose(*s, T, nullptr));
+        return 0;
+    }
+};
+
+// Frames of a session whose run numbers start at `number` give those of a new one.
+int numbers(Frames &f, unsigned number) {
+    gbf_session *a, *b;
+    if (f.session(&a) || f.session(&b)) return 1;
+    const std::vector<unsigned long long> words((b->lay.total - b->lay.track_rec) / 8, (unsigned long long)number << 32);
+    OK(cudaMemcpy(b->view.track_rec, words.data(), words.size() * 8, cudaMemcpyHostToDevice));
+    OK(cudaMemcpy(b->view.ctr + C_TRACK_PUB, words.data(), 14 * 8, cudaMemcpyHostToDevice));
+    for (int k = 0; k < 6; ++k) {
+        if (f.render(k)) return 1;
+        gbf_frame_stats x, y;
+        double p[16], q[16];
+        for (gbf_session *s : {a, b}) OK(gbf_process_frame(s, f.depth, kW * 2, f.rgb, kW * 3, nullptr));
+        OK(gbf_get_pose(a, p, nullptr));
+        OK(gbf_get_pose(b, q, nullptr));
+        OK(gbf_get_stats(a, &x, nullptr));
+        OK(gbf_get_stats(b, &y, nullptr));
+        if (memcmp(p, q, sizeof(p)) || x.status || y.status || x.pixel_iterations != y.pixel_iterations) {
+            printf("numbers from %#x, frame %d: status %u %u\n", number, k, x.status, y.status);
+            return 1;
+        }
+    }
+    OK(gbf_session_destroy(a));
+    OK(gbf_session_destroy(b));
+    return 0;
+}
+
+int main(int argc, char **argv) {
+    Frames f;
+    if (argc < 2 || f.open()) return 1;
+    if (!strcmp(argv[1], "numbers")) return numbers(f, 5u) || numbers(f, 0x7ffffff5u) || numbers(f, 0xfffffff5u);
+    return 1;
+}
