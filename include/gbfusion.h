@@ -79,7 +79,10 @@ enum {
     GBF_FLAG_TRACK_FAILED   = 1u << 3, /* a frame's tracking failed since the reset
                                           (pose kept for it); the last frame's result
                                           is gbf_frame_stats.track.success          */
-    GBF_FLAG_NAN_POSE       = 1u << 4  /* solver produced a non-finite pose          */
+    GBF_FLAG_NAN_POSE       = 1u << 4, /* solver produced a non-finite pose          */
+    GBF_FLAG_TRACK_WAIT     = 1u << 5  /* a wait within a frame's tracking ran out (2 s):
+                                          the frame counts as not tracked, though not
+                                          for what the camera saw                   */
 };
 
 typedef enum gbf_voxel_layout {

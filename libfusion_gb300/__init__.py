@@ -22,7 +22,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import (FLAG_COORD_RANGE, FLAG_HASH_FULL, FLAG_NAN_POSE, FLAG_POOL_EXHAUSTED, FLAG_TRACK_FAILED,
-                   MESH_COLOUR, MESH_NORMAL, MESH_VERTEX, VOXEL_HALF, VOXEL_REF, VOXEL_SNORM, GbfError, call,
+                   FLAG_TRACK_WAIT, MESH_COLOUR, MESH_NORMAL, MESH_VERTEX, VOXEL_HALF, VOXEL_REF, VOXEL_SNORM, GbfError, call,
                    default_config, lib, mat16)
 
 __all__ = [
@@ -30,7 +30,7 @@ __all__ = [
     "write_dump", "read_dump", "render_scene", "autotune_forget",
     "default_config", "session_bytes", "GbfError", "VOXEL_REF", "VOXEL_HALF", "VOXEL_SNORM", "MESH_VERTEX", "MESH_NORMAL",
     "MESH_COLOUR", "FLAG_POOL_EXHAUSTED", "FLAG_HASH_FULL", "FLAG_COORD_RANGE", "FLAG_TRACK_FAILED",
-    "FLAG_NAN_POSE", "version",
+    "FLAG_NAN_POSE", "FLAG_TRACK_WAIT", "version",
 ]
 
 

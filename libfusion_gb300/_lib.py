@@ -20,6 +20,7 @@ FLAG_HASH_FULL = 2
 FLAG_COORD_RANGE = 4
 FLAG_TRACK_FAILED = 8
 FLAG_NAN_POSE = 16
+FLAG_TRACK_WAIT = 32
 
 VOXEL_REF = 0
 VOXEL_HALF = 1

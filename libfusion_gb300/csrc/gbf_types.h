@@ -28,6 +28,7 @@ constexpr int kReducePixelsPerThread = 4;
 constexpr int kCoarseReduceTile = 1024;
 constexpr int kReduceWidth = 58;        // 29 ICP + 29 RGB sums
 constexpr int kPartialStride = 64;      // floats per CTA partial record
+constexpr long long kTrackWaitNs = 2000000000ll;  // longest wait within a tracking run
 constexpr float kListSdf = 1.01f;       // truncations that a raycast's neighbour lists reach before the near plane
 constexpr int kMeshChunks = 256;        // chunks of blocks of a mesh's offset scan, at most
 constexpr int kMeshWords = kMeshChunks + 1;  // their sums and the block counter of the emission
@@ -61,6 +62,8 @@ enum Counter {
     C_DEEP_SDF = 9,   // 1 once a map with an sdf below -kListSdf has been imported
     C_COUNT = 16,     // counters proper (reported, kept by snapshots)
     C_TRACK_PUB = 16, // 14 8-byte words published within a tracking run (gn_track_kernel)
+    C_TRACK_BASE = 44,    // arrivals of CTAs over the session's tracking runs until this one
+    C_TRACK_ARRIVED = 45, // and so far
     C_WORDS = 64      // ints in the arena
 };
 
@@ -141,6 +144,7 @@ struct SessionView {
     int zr_w, zr_h;
 
     TrackState *ts;
+    long long track_wait_ns;  // longest wait of a tracking run's CTA 0 for another
     float *partials;       // [red_ctas][kPartialStride]
     unsigned long long *track_rec;  // [red_ctas][kPartialStride] (gn_track_kernel)
     int *mesh_off;         // per-block triangle counts / offsets (pool + 1)

@@ -460,6 +460,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
     v.partials = reinterpret_cast<float *>(base + a.partials);
     v.mesh_sums = reinterpret_cast<int *>(base + a.mesh_sums);
     v.track_rec = reinterpret_cast<unsigned long long *>(base + a.track_rec);
+    v.track_wait_ns = kTrackWaitNs;
 
     Extent &ex = s->ex;
     memset(&ex, 0, sizeof(ex));

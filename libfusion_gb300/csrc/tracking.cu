@@ -775,7 +775,7 @@ struct TrackSmem {
     float pose[12];
     float stddev, huber;
     unsigned seen;
-    int item, lost;
+    int item, lost, late;
 };
 
 // icp_row and rgb_row of one pixel, with their gathers issued together (a row
@@ -843,29 +843,32 @@ __device__ __forceinline__ void chain_sums(const float4 *lo, const float4 *hi, i
     }
 }
 
-// A CTA of the run waits for another at most this long.  Every CTA is resident
-// and a step takes microseconds: the limit only bounds a wait that cannot happen.
-constexpr long long kTrackWaitNs = 2000000000ll;
+// A CTA of the run waits for another at most this long (CTA 0: SessionView::track_wait_ns).
+// Every CTA is resident and a step takes microseconds: the limit only bounds a wait that
+// cannot happen.
 struct WaitLimit {
-    long long t0 = 0;
-    int n = 0;
+    long long ns, t0 = 0;
+    int n = 0, every;
     bool ran_out = false;
+    __device__ __forceinline__ explicit WaitLimit(long long limit) : ns(limit), every(limit > 0 ? 63 : 0) {}
     __device__ __forceinline__ bool over() {
-        if (++n & 63) return false;
+        if (++n & every) return false;
         long long t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         if (!t0) t0 = t;
-        return ran_out = t - t0 > kTrackWaitNs;
+        return ran_out = t - t0 >= ns;
     }
 };
 
-__device__ __forceinline__ int ld_acquire(const int *p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned ld_acquire(const int *p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void red_release(int *p) {
-    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p) : "memory");
+__device__ __forceinline__ unsigned atom_add(int *p, unsigned n) {
+    unsigned v;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "r"(n) : "memory");
+    return v;
 }
 __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *p) {
     unsigned long long v;
@@ -893,6 +896,7 @@ __device__ __forceinline__ void st_relaxed(unsigned long long *p, unsigned long 
 // tile, numbered like the publication that will follow.  The numbers run on over the
 // session's runs and wrap: one is newer by the sign of the difference.
 constexpr int kPubWords = 14;
+constexpr unsigned kRunClosed = 1u << 20;  // above any count of CTAs
 __device__ __forceinline__ unsigned long long tagged(unsigned number, unsigned value) {
     return ((unsigned long long)number << 32) | value;
 }
@@ -920,7 +924,7 @@ __device__ __forceinline__ unsigned long long *record_word(const SessionView &sv
 static_assert(kTrackThreads == 32 * kSumGroups, "a warp per record group");
 __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv, int n, unsigned number) {
     const int g = threadIdx.x >> 5, lane = threadIdx.x & 31, q = min(2 * lane, kReduceWidth - 2);
-    WaitLimit limit;
+    WaitLimit limit(sv.track_wait_ns);
     FSum s0, s1;
     constexpr int kBatch = 10;  // at most a record per lane
     for (int c = g; c < n; c += kBatch * kSumGroups) {
@@ -970,7 +974,7 @@ __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv
 // values.  False when the wait ran out.
 __device__ __forceinline__ bool read_pub(const unsigned long long *pub, unsigned &seen, unsigned &value) {
     const int lane = threadIdx.x & 31;
-    WaitLimit limit;
+    WaitLimit limit(kTrackWaitNs);
     for (;;) {
         const unsigned long long w = lane < kPubWords ? ld_relaxed(pub + lane) : 0ull;
         const unsigned n = number_of(w), n0 = __shfl_sync(0xffffffffu, n, 0);
@@ -1011,6 +1015,7 @@ __device__ __forceinline__ void track_steps(TrackSmem &sm, const SessionView &sv
             // a wait ran out: the frame counts as not tracked, the other CTAs end, and the
             // numbers go on behind that of the records that may still come
             ts->invalid = 1;
+            if (lane == 0) raise_flag(sv, GBF_FLAG_TRACK_WAIT);
             if (lane < kPubWords) st_relaxed(pub + lane, tagged(seen + 1, 0u));
         }
         __syncwarp();
@@ -1019,12 +1024,12 @@ __device__ __forceinline__ void track_steps(TrackSmem &sm, const SessionView &sv
     __syncthreads();
     for (int i = tid; i < (int)(sizeof(TrackState) / 4); i += kTrackThreads)
         reinterpret_cast<int *>(sv.ts)[i] = reinterpret_cast<const int *>(ts)[i];
-    if (tid == 0) sv.ctr[C_TICKET] = 0;
 }
 
 // The tiles of a run: CTA cta of the ctas that follow CTA 0 makes its tiles' records of each item.
+// Thread 0's: the arrivals before this run, and before this CTA's.
 __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv, int item, unsigned seen, int rs, int cta,
-                                            int ctas) {
+                                            int ctas, unsigned base, unsigned arrival) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned long long *pub = reinterpret_cast<const unsigned long long *>(sv.ctr + C_TRACK_PUB);
     const float qnan = __int_as_float(0x7fffffff);
@@ -1066,6 +1071,7 @@ __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv
                 }
                 // meanwhile the next tile's pixels, or the first one's again for the next iteration
                 load(tile + ctas < tiles ? tile + ctas : cta);
+                if (tid == 0) sm.late = arrival - base >= (unsigned)ctas;  // (the count's answer has had the gathers' time)
                 __syncwarp();
                 __syncthreads();
                 if (warp < 8) {  // ICP chains, then photometric ones
@@ -1085,7 +1091,16 @@ __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv
                 }
             }
         } else {
+            if (tid == 0) sm.late = arrival - base >= (unsigned)ctas;
+            __syncwarp();
             __syncthreads();  // every warp has the item before the next one takes its place
+        }
+        if (sm.late) {
+            // CTA 0 had given up: `seen` may be what the next run starts from, so the
+            // records take a number that it does not wait for
+            for (int tile = cta; tile < tiles; tile += ctas)
+                if (tid < kReduceWidth) st_relaxed(record_word(sv, tile, tid), tagged(seen, 0u));
+            return;
         }
         if (warp == 0) {
             unsigned value = 0;
@@ -1129,16 +1144,31 @@ __global__ void __launch_bounds__(kTrackThreads, 1)
     __syncwarp();
     __syncthreads();
     if (!head) {
-        if (tid == 0) red_release(sv.ctr + C_TICKET);
+        unsigned base = 0, arrival = 0;
+        if (tid == 0) {
+            base = ld_acquire(sv.ctr + C_TRACK_BASE);
+            arrival = atom_add(sv.ctr + C_TRACK_ARRIVED, 1u);
+        }
         __syncwarp();
-        track_tiles(sm, sv, item, seen, rs, blockIdx.x - 1, gridDim.x - 1);
+        track_tiles(sm, sv, item, seen, rs, blockIdx.x - 1, gridDim.x - 1, base, arrival);
         return;
     }
     if (tid == 0) {
         track_begin(&sm.ts, frame_mode);
-        WaitLimit limit;
-        while (ld_acquire(sv.ctr + C_TICKET) != (int)gridDim.x - 1 && !limit.over()) {}
-        sm.lost = ld_acquire(sv.ctr + C_TICKET) != (int)gridDim.x - 1;
+        const unsigned base = ld_acquire(sv.ctr + C_TRACK_BASE), others = gridDim.x - 1;
+        // Arrivals are counted over the session's runs: every CTA of a run has arrived when
+        // the next one starts, but a run that gives up here ends before all have.  It adds
+        // kRunClosed to the count, which tells the CTAs that come then (by the order
+        // that they get, whichever base they read).
+        WaitLimit limit(sv.track_wait_ns);
+        while (ld_acquire(sv.ctr + C_TRACK_ARRIVED) - base != others && !limit.over()) {}
+        sm.lost = limit.ran_out;
+        unsigned next = base + others;
+        if (limit.ran_out) {
+            atom_add(sv.ctr + C_TRACK_ARRIVED, kRunClosed);
+            next += kRunClosed;
+        }
+        sv.ctr[C_TRACK_BASE] = (int)next;
     }
     __syncwarp();
     __syncthreads();

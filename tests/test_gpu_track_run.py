@@ -27,3 +27,9 @@ def test_run_numbers_wrap(program):
     """The numbers of a run's words go on from frame to frame for the session's life:
     past 2^31 and past 2^32 the frames are those of a new session."""
     program("numbers")
+
+
+def test_run_whose_wait_ran_out(program):
+    """CTA 0 gives up waiting: the run ends at once, the frame is not tracked and carries a
+    flag of its own, and the session's next run is as if that one had not been."""
+    program("lost")

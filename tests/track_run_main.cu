@@ -1,6 +1,9 @@
 // Drives sessions through the C API and reaches into one's arena for what no
-// caller can set: the numbers of the tracking run's words (csrc/tracking.cu).
+// caller can set: the numbers of the tracking run's words and the longest wait of
+// its CTA 0 (csrc/tracking.cu).
 // Prints what differs and returns 1, or returns 0.
+#include <chrono>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -83,9 +86,69 @@ int numbers(Frames &f, unsigned number) {
     return 0;
 }
 
+int set_wait(gbf_session *s, long long ns) {
+    OK(cudaMemcpy(reinterpret_cast<char *>(s->d_view) + offsetof(SessionView, track_wait_ns), &ns, sizeof(ns),
+                  cudaMemcpyHostToDevice));
+    return 0;
+}
+
+// Runs whose CTA 0 does not wait at all (it gives up on the CTAs' arrival or on the
+// first records): each ends at once, is told apart and leaves the next run as it was.
+int lost(Frames &f) {
+    gbf_session *s;
+    if (f.session(&s)) return 1;
+    for (int k = 0; k < 3; ++k) {
+        if (f.render(k)) return 1;
+        OK(gbf_process_frame(s, f.depth, kW * 2, f.rgb, kW * 3, nullptr));
+    }
+    double I[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1}, before[16], after[16];
+    gbf_track_result want{}, got{};
+    gbf_frame_stats st;
+    OK(gbf_track(s, I, &want, nullptr));
+    OK(gbf_get_stats(s, &st, nullptr));
+    if (!want.success || want.iterations < 5 || st.status) {
+        printf("success %d, %d iterations, status %u\n", want.success, want.iterations, st.status);
+        return 1;
+    }
+    const auto t0 = std::chrono::steady_clock::now();
+    for (int k = 0; k < 300; ++k) {
+        if (set_wait(s, 0)) return 1;
+        OK(gbf_track(s, I, &got, nullptr));
+        OK(gbf_get_stats(s, &st, nullptr));
+        if (got.success || memcmp(got.update, I, sizeof(I)) || st.status != GBF_FLAG_TRACK_WAIT) {
+            printf("lost run %d: success %d, status %u\n", k, got.success, st.status);
+            return 1;
+        }
+        if (set_wait(s, kTrackWaitNs)) return 1;
+        OK(gbf_track(s, I, &got, nullptr));
+        if (memcmp(&got, &want, sizeof(got))) {
+            printf("the run after lost run %d: success %d, %d iterations\n", k, got.success, got.iterations);
+            return 1;
+        }
+    }
+    const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    if (secs > 2.0) {  // one wait that ran its two seconds out
+        printf("600 runs took %.3f s\n", secs);
+        return 1;
+    }
+    // a frame: the pose stays, and the frame counts as not tracked
+    OK(gbf_get_pose(s, before, nullptr));
+    if (f.render(3) || set_wait(s, 0)) return 1;
+    OK(gbf_process_frame(s, f.depth, kW * 2, f.rgb, kW * 3, nullptr));
+    OK(gbf_get_pose(s, after, nullptr));
+    OK(gbf_get_stats(s, &st, nullptr));
+    if (memcmp(before, after, sizeof(before)) || st.track.success || st.status != (GBF_FLAG_TRACK_WAIT | GBF_FLAG_TRACK_FAILED)) {
+        printf("frame: success %d, status %u\n", st.track.success, st.status);
+        return 1;
+    }
+    OK(gbf_session_destroy(s));
+    return 0;
+}
+
 int main(int argc, char **argv) {
     Frames f;
     if (argc < 2 || f.open()) return 1;
     if (!strcmp(argv[1], "numbers")) return numbers(f, 5u) || numbers(f, 0x7ffffff5u) || numbers(f, 0xfffffff5u);
+    if (!strcmp(argv[1], "lost")) return lost(f);
     return 1;
 }
