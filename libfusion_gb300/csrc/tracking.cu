@@ -1247,9 +1247,12 @@ void prepare_track() { track_run_ctas(); }
 void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, bool alone, cudaStream_t st) {
     if (takes_run(nslots, ex, alone)) {
         void *args[] = {(void *)&d_sv, (void *)&frame_mode};
-        cudaLaunchCooperativeKernel((const void *)gn_track_kernel, dim3(track_run_ctas() / nslots, nslots),
-                                    dim3(kTrackThreads), args, sizeof(TrackSmem), st);
-        return;
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel((const void *)gn_track_kernel, dim3(track_run_ctas() / nslots, nslots),
+                                        dim3(kTrackThreads), args, sizeof(TrackSmem), st);
+        // a stream with fewer SMs than the device (a green context's) refuses the grid
+        if (e != cudaErrorCooperativeLaunchTooLarge) return;
+        cudaGetLastError();
     }
     track_begin_kernel<<<nslots, 32, 0, st>>>(d_sv, frame_mode);
     ReduceArgs a{};

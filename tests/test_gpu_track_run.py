@@ -14,7 +14,7 @@ def program(gbf, tmp_path_factory):
     from libfusion_gb300 import build as B
     exe = tmp_path_factory.mktemp("run") / "track_run"
     subprocess.run([B.nvcc(), *B.ARCH, "-O1", "-std=c++17", "--expt-relaxed-constexpr", str(HERE / "track_run_main.cu"),
-                    str(B.LIB), "-Xlinker", f"-rpath={B.LIB.parent}", "-o", str(exe)], check=True,
+                    str(B.LIB), "-Xlinker", f"-rpath={B.LIB.parent}", "-lcuda", "-o", str(exe)], check=True,
                    capture_output=True)
 
     def run(*args):
@@ -33,3 +33,9 @@ def test_run_whose_wait_ran_out(program):
     """CTA 0 gives up waiting: the run ends at once, the frame is not tracked and carries a
     flag of its own, and the session's next run is as if that one had not been."""
     program("lost")
+
+
+def test_frames_on_a_stream_with_few_sms(program):
+    """A green context's stream has too few SMs for the run's cooperative grid: the frame is
+    tracked in a launch per iteration, with the same result."""
+    program("few_sms")

@@ -2,6 +2,8 @@
 // caller can set: the numbers of the tracking run's words and the longest wait of
 // its CTA 0 (csrc/tracking.cu).
 // Prints what differs and returns 1, or returns 0.
+#include <cuda.h>
+
 #include <chrono>
 #include <cstddef>
 #include <cstdio>
@@ -145,10 +147,53 @@ int lost(Frames &f) {
     return 0;
 }
 
+// A stream of a green context with a few of the SMs, where the run's grid does not fit:
+// the frames are those of a stream with all of them.
+int few_sms(Frames &f) {
+    CUdevResource all{}, few{}, rest{};
+    CUdevResourceDesc desc{};
+    CUgreenCtx ctx{};
+    CUstream st{};
+    unsigned groups = 1;
+    OK(cuDeviceGetDevResource(0, &all, CU_DEV_RESOURCE_TYPE_SM));
+    OK(cuDevSmResourceSplitByCount(&few, &groups, &all, &rest, 0, 16));
+    OK(cuDevResourceGenerateDesc(&desc, &few, 1));
+    OK(cuGreenCtxCreate(&ctx, desc, 0, CU_GREEN_CTX_DEFAULT_STREAM));
+    OK(cuGreenCtxStreamCreate(&st, ctx, CU_STREAM_NON_BLOCKING, 0));
+    if (few.sm.smCount >= all.sm.smCount) {
+        printf("%u of %u SMs\n", few.sm.smCount, all.sm.smCount);
+        return 1;
+    }
+    gbf_session *a, *b;
+    if (f.session(&a) || f.session(&b)) return 1;
+    for (int k = 0; k < 4; ++k) {
+        if (f.render(k)) return 1;
+        OK(cudaDeviceSynchronize());
+        gbf_frame_stats x, y;
+        double p[16], q[16];
+        OK(gbf_process_frame(a, f.depth, kW * 2, f.rgb, kW * 3, nullptr));
+        OK(gbf_process_frame(b, f.depth, kW * 2, f.rgb, kW * 3, st));
+        OK(gbf_get_pose(a, p, nullptr));
+        OK(gbf_get_pose(b, q, st));
+        OK(gbf_get_stats(a, &x, nullptr));
+        OK(gbf_get_stats(b, &y, st));
+        if (memcmp(p, q, sizeof(p)) || x.status || y.status || x.pixel_iterations != y.pixel_iterations) {
+            printf("%u of %u SMs, frame %d: status %u %u\n", few.sm.smCount, all.sm.smCount, k, x.status, y.status);
+            return 1;
+        }
+    }
+    OK(gbf_session_destroy(a));
+    OK(gbf_session_destroy(b));
+    OK(cuStreamDestroy(st));
+    OK(cuGreenCtxDestroy(ctx));
+    return 0;
+}
+
 int main(int argc, char **argv) {
     Frames f;
     if (argc < 2 || f.open()) return 1;
     if (!strcmp(argv[1], "numbers")) return numbers(f, 5u) || numbers(f, 0x7ffffff5u) || numbers(f, 0xfffffff5u);
     if (!strcmp(argv[1], "lost")) return lost(f);
+    if (!strcmp(argv[1], "few_sms")) return few_sms(f);
     return 1;
 }
