@@ -40,6 +40,15 @@ gbf_status reset_map(gbf_session *s);
 // clear the table and insert every pool block [0, used) at its own id (gc.cu)
 void rebuild_table(gbf_session *s, cudaStream_t st);
 
+// The frames of a session, or the ticks of a batch: how many the host has sent and
+// how many the device has ended (done: a pinned word that their last launch writes).
+struct Flight {
+    unsigned sent = 0;
+    unsigned *done = nullptr;
+    cudaStream_t stream = nullptr;
+    int device = 0;
+};
+
 }  // namespace gbf
 
 struct gbf_session {
@@ -52,6 +61,7 @@ struct gbf_session {
     gbf::Extent ex{};
     int layouts[gbf::kNumLayouts] = {};
     int device = 0;
+    gbf::Flight flight;
 };
 
 struct gbf_batch {
@@ -64,7 +74,8 @@ struct gbf_batch {
     gbf::SessionView *d_views = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     bool ev_used[2] = {false, false};
-    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    cudaGraphExec_t exec[2][2] = {};  // per mirror: alone on the chip, beside other streams' work
+    gbf::Flight flight;
     cudaStream_t own = nullptr;
     int flip = 0;
     int nslots = 0;

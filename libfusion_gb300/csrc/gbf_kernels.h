@@ -98,7 +98,8 @@ void launch_nmap_of(const float4 *vmap, long long vmap_pitch, float4 *nmap, long
                     cudaStream_t st);
 // kernel launches of one launch_post
 int post_launches(const Extent &ex);
-void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st);
+// done (optional): where the frame's number is noted as it ends
+void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, unsigned *done, unsigned number, cudaStream_t st);
 
 // The ICP gates sine < angle and length <= dist (pose_estimator.cu:200) as bounds on
 // the squares whose rounded roots they compare: the root rounded to nearest is
@@ -117,8 +118,8 @@ inline void square_gates(SessionView &v, float dist, float angle) {
 
 // ---- tracking (tracking.cu) -----------------------------------------------------
 // mode 0: full Gauss-Newton (gbf_track / process frame), stops at the schedule end
-// alone: no other launch of this library runs beside it (not one of several
-// branches of a tick), so a few sessions may take the whole chip.
+// alone: little of this library's work runs beside it (not one of several branches of a
+// tick, nor one of several streams' frames), so a few sessions may take the whole chip.
 // kernel launches of one launch_track over nslots sessions
 int track_launches(int nslots, const Extent &ex, bool alone);
 void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, bool alone, cudaStream_t st);

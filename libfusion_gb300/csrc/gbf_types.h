@@ -144,6 +144,8 @@ struct SessionView {
     int zr_w, zr_h;
 
     TrackState *ts;
+    unsigned *tick_done;   // first slot of a batch: where the tick's end is noted, and its number
+    unsigned tick_number;
     long long track_wait_ns;  // longest wait of a tracking run's CTA 0 for another
     float *partials;       // [red_ctas][kPartialStride]
     unsigned long long *track_rec;  // [red_ctas][kPartialStride] (gn_track_kernel)

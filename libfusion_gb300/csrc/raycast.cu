@@ -562,8 +562,10 @@ __device__ __forceinline__ float4 mean4(const float4 a, const float4 b, const fl
 // (in turn, with their coordinates divided out, they left a session's few CTAs waiting:
 // 640x480 14.1 -> 12.5 us, four sessions 25.3 -> 22.6, 64 250 -> 242).
 constexpr int kPostTile = 32;
-__global__ void __launch_bounds__(256) post_pyramid_kernel(const SessionView *__restrict__ svs) {
+__global__ void __launch_bounds__(256) post_pyramid_kernel(const SessionView *__restrict__ svs, unsigned *done,
+                                                           unsigned number) {
     chain_begin();
+    if (done && blockIdx.x == 0 && threadIdx.x == 0) *static_cast<volatile unsigned *>(done) = number;
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     const int w0 = sv.lv[0].w, h0 = sv.lv[0].h;
@@ -668,8 +670,9 @@ __global__ void nmap_of_kernel(const float4 *vmap, long long vmap_pitch, float4 
         normal_at(vmap, vmap_pitch / 16, x, y, w, h);
 }
 
-__global__ void nmap_all_kernel(const SessionView *__restrict__ svs) {
+__global__ void nmap_all_kernel(const SessionView *__restrict__ svs, unsigned *done, unsigned number) {
     chain_begin();
+    if (done && blockIdx.x == 0 && threadIdx.x == 0) *static_cast<volatile unsigned *>(done) = number;
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     int b = blockIdx.x, level = 0;
@@ -729,10 +732,10 @@ void launch_nmap_of(const float4 *vmap, long long vmap_pitch, float4 *nmap, long
 
 int post_launches(const Extent &ex) { return ex.levels <= 3 ? 1 : ex.levels; }
 
-void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, cudaStream_t st) {
+void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, unsigned *done, unsigned number, cudaStream_t st) {
     if (ex.levels <= 3) {
         const int tiles = ((ex.w + kPostTile - 1) / kPostTile) * ((ex.h + kPostTile - 1) / kPostTile);
-        launch_kernel(post_pyramid_kernel, dim3(tiles, nslots), 256, ex.chain, st, d_sv);
+        launch_kernel(post_pyramid_kernel, dim3(tiles, nslots), 256, ex.chain, st, d_sv, done, number);
         return;
     }
     int w = ex.w, h = ex.h, total = (w * h + 255) / 256;
@@ -741,7 +744,7 @@ void launch_post(const SessionView *d_sv, int nslots, const Extent &ex, cudaStre
         launch_kernel(vmap_down_kernel, dim3((w * h + 255) / 256, nslots), 256, ex.chain, st, d_sv, l);
         total += (w * h + 255) / 256;
     }
-    launch_kernel(nmap_all_kernel, dim3(total, nslots), 256, ex.chain, st, d_sv);
+    launch_kernel(nmap_all_kernel, dim3(total, nslots), 256, ex.chain, st, d_sv, done, number);
 }
 
 void launch_raycast(const SessionView *d_sv, const Extent &ex, const double pose[12], bool check_visibility,

@@ -135,6 +135,68 @@ ArenaLayout plan_arena(const gbf_config &c, const gbf_intrinsics &K) {
 
 namespace {
 
+// Flights that may have work on the device.  A tracking run holds every SM until it
+// ends, so beside frames of two or more other streams a launch per iteration is the
+// better one: rounds of 2, 4, 8, 16 sessions at 320x240, a stream each, 427, 735, 1405, 2932 us
+// with runs and 452, 531, 825, 1194 without (one alone 280 and 425); at 640x480 593,
+// 985, 1913, 3882 and 570, 800, 1318, 2493.  Beside one other stream, a 64-session batch's,
+// a frame of 640x480 takes 1.07 ms with the run and 5.44 without.
+// (Never destroyed: sessions may be closed while the process exits.)
+std::mutex &g_flight_mu = *new std::mutex;
+std::vector<Flight *> &g_flights = *new std::vector<Flight *>;
+
+unsigned flight_done(const Flight &f) { return *static_cast<volatile unsigned *>(f.done); }
+
+cudaError_t flight_open(Flight &f) {
+    cudaGetDevice(&f.device);
+    const cudaError_t e = cudaHostAlloc(&f.done, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e == cudaSuccess) *f.done = 0;
+    return e;
+}
+
+void flight_close(Flight &f) {  // the device is idle
+    {
+        std::lock_guard<std::mutex> lock(g_flight_mu);
+        g_flights.erase(std::remove(g_flights.begin(), g_flights.end(), &f), g_flights.end());
+    }
+    if (f.done) cudaFreeHost(f.done);
+    f.done = nullptr;
+}
+
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+// Counts one more frame (or tick) as sent to `st`.  True where it may take the chip.  A captured
+// frame is not counted: what its replays run beside is not known.
+bool flight_send(Flight &f, cudaStream_t st, unsigned *number) {
+    *number = 0;
+    if (capturing(st)) return true;
+    std::lock_guard<std::mutex> lock(g_flight_mu);
+    g_flights.erase(std::remove_if(g_flights.begin(), g_flights.end(),
+                                   [&](Flight *o) { return o == &f || (int)(o->sent - flight_done(*o)) <= 0; }),
+                    g_flights.end());
+    const Flight *beside = nullptr;
+    bool few = true;
+    for (const Flight *o : g_flights)
+        if (o->device == f.device && o->stream != st) {
+            if (beside && beside->stream != o->stream) few = false;
+            beside = o;
+        }
+    f.stream = st;
+    *number = ++f.sent;
+    g_flights.push_back(&f);
+    return few;
+}
+
+// The host has waited for everything sent.
+void flight_ended(Flight &f, unsigned number) {
+    if (number) *static_cast<volatile unsigned *>(f.done) = number;
+}
+
 __global__ void reset_table_kernel(HashSlot *t, int cap) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += gridDim.x * blockDim.x) {
         HashSlot s;
@@ -293,7 +355,7 @@ void enqueue_first_half(const SessionView *d_sv, int nslots, const Extent &ex, c
 // Second half: allocation, visibility (with the z-range of the raycast, at the same
 // pose), integration and the raycast that makes the next frame's reference maps.
 void enqueue_second_half(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, cudaStream_t st,
-                         cudaEvent_t *ev = nullptr) {
+                         cudaEvent_t *ev = nullptr, unsigned *done = nullptr, unsigned number = 0) {
     PhaseMarks mark(ev, st);
     launch_alloc(d_sv, nslots, ex, true, st);
     launch_zrange(d_sv, nslots, ex, ZrangeOf::fuse, st);
@@ -303,14 +365,25 @@ void enqueue_second_half(const SessionView *d_sv, int nslots, const Extent &ex, 
     mark(5, st);  // (no launch of its own any more)
     launch_march(d_sv, nslots, ex, nullptr, 0, layouts, st);
     mark(6, st);
-    launch_post(d_sv, nslots, ex, st);
+    launch_post(d_sv, nslots, ex, done, number, st);
     mark(7, st);
 }
 
 void enqueue_frame(const SessionView *d_sv, int nslots, const Extent &ex, const int *layouts, const IngestArgs &in,
-                   bool alone, cudaStream_t st, cudaEvent_t *ev = nullptr) {
+                   bool alone, cudaStream_t st, cudaEvent_t *ev = nullptr, unsigned *done = nullptr,
+                   unsigned number = 0) {
     enqueue_first_half(d_sv, nslots, ex, in, alone, st, ev);
-    enqueue_second_half(d_sv, nslots, ex, layouts, st, ev);
+    enqueue_second_half(d_sv, nslots, ex, layouts, st, ev, done, number);
+}
+
+// A frame of a session on its own.
+gbf_status session_frame(gbf_session *s, const IngestArgs &in, cudaStream_t st, const char *where) {
+    unsigned number;
+    const bool alone = flight_send(s->flight, st, &number);
+    enqueue_frame(s->d_view, 1, s->ex, s->layouts, in, alone, st, nullptr, number ? s->flight.done : nullptr, number);
+    const gbf_status r = check_cuda(where);
+    if (r != GBF_OK) flight_ended(s->flight, number);  // nothing will note its end
+    return r;
 }
 
 // kernels launched by enqueue_frame
@@ -397,6 +470,11 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
         cudaFree(s->arena);
         delete s;
         return cuda_error(e, "gbf_session_create: view");
+    }
+    e = flight_open(s->flight);
+    if (e != cudaSuccess) {
+        gbf_session_destroy(s);
+        return cuda_error(e, "gbf_session_create: host word");
     }
     char *base = static_cast<char *>(s->arena);
     const ArenaLayout &a = s->lay;
@@ -499,6 +577,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
 GBF_API gbf_status gbf_session_destroy(gbf_session *s) {
     if (!s) return GBF_OK;
     cudaDeviceSynchronize();
+    flight_close(s->flight);
     if (s->d_view) cudaFree(s->d_view);
     if (s->arena) cudaFree(s->arena);
     delete s;
@@ -736,12 +815,14 @@ GBF_API gbf_status gbf_track(gbf_session *s, const double init[16], gbf_track_re
     to34(init, p);
     cudaError_t e = cudaMemcpyAsync(s->view.ts->init, p, sizeof(p), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_error(e, "gbf_track");
-    launch_track(s->d_view, 1, s->ex, 0, true, st);
-    gbf_status r = check_cuda("gbf_track");
-    if (r != GBF_OK) return r;
+    unsigned number;
+    const bool alone = flight_send(s->flight, st, &number);
+    launch_track(s->d_view, 1, s->ex, 0, alone, st);
+    e = cudaGetLastError();
     TrackState t;
-    e = cudaMemcpyAsync(&t, s->view.ts, sizeof(t), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&t, s->view.ts, sizeof(t), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    flight_ended(s->flight, number);
     if (e != cudaSuccess) return cuda_error(e, "gbf_track");
     fill_result(t, out);
     return GBF_OK;
@@ -784,15 +865,13 @@ GBF_API gbf_status gbf_process_frame(gbf_session *s, const uint16_t *depth, int6
     if (!rows_aligned(depth, depth_pitch, 2))
         return set_error(GBF_ERR_INVALID_ARG, "gbf_process_frame: depth rows must be 2-byte aligned");
     IngestArgs a{0, 1, depth, depth_pitch, rgb, rgb_pitch};
-    enqueue_frame(s->d_view, 1, s->ex, s->layouts, a, true, (cudaStream_t)stream);
-    return check_cuda("gbf_process_frame");
+    return session_frame(s, a, (cudaStream_t)stream, "gbf_process_frame");
 }
 
 GBF_API gbf_status gbf_process_frame_staged(gbf_session *s, void *stream) {
     if (!s) return set_error(GBF_ERR_INVALID_ARG, "gbf_process_frame_staged: null");
     IngestArgs a{0, 0, nullptr, 0, nullptr, 0};
-    enqueue_frame(s->d_view, 1, s->ex, s->layouts, a, true, (cudaStream_t)stream);
-    return check_cuda("gbf_process_frame_staged");
+    return session_frame(s, a, (cudaStream_t)stream, "gbf_process_frame_staged");
 }
 
 GBF_API gbf_status gbf_map_export(gbf_session *s, int32_t *coords, float *sdf, float *weight, uint8_t *rgb,
@@ -943,6 +1022,7 @@ GBF_API gbf_status gbf_batch_create(int32_t max_sessions, gbf_batch **out) {
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[g], cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = flight_open(b->flight);
     for (int k = 0; k < 2; ++k) {
         b->stg_depth[k].assign(max_sessions, nullptr);
         b->stg_rgb[k].assign(max_sessions, nullptr);
@@ -967,10 +1047,11 @@ GBF_API gbf_status gbf_batch_create(int32_t max_sessions, gbf_batch **out) {
 
 static void batch_invalidate(gbf_batch *b) {
     for (int k = 0; k < 2; ++k)
-        if (b->exec[k]) {
-            cudaGraphExecDestroy(b->exec[k]);
-            b->exec[k] = nullptr;
-        }
+        for (cudaGraphExec_t &x : b->exec[k])
+            if (x) {
+                cudaGraphExecDestroy(x);
+                x = nullptr;
+            }
 }
 
 GBF_API gbf_status gbf_batch_destroy(gbf_batch *b) {
@@ -982,6 +1063,7 @@ GBF_API gbf_status gbf_batch_destroy(gbf_batch *b) {
     if (b->d_views_b) batch_flush(b, nullptr);  // the sessions outlive the batch: fuse what is owed
     cudaDeviceSynchronize();
     batch_invalidate(b);
+    flight_close(b->flight);
     for (int k = 0; k < 2; ++k) {
         if (b->h_views[k]) cudaFreeHost(b->h_views[k]);
         if (b->h_views_b[k]) cudaFreeHost(b->h_views_b[k]);
@@ -1129,7 +1211,7 @@ static int effective_groups(const gbf_batch *b) { return b->timing ? 1 : tick_gr
 static bool staggered(const gbf_batch *b) { return b->stagger && effective_groups(b) >= 2; }
 static int group_lo(const gbf_batch *b, int g, int groups) { return b->nslots * g / groups; }
 
-static void batch_enqueue(gbf_batch *b, int k, cudaStream_t st) {
+static void batch_enqueue(gbf_batch *b, int k, bool alone, cudaStream_t st) {
     cudaMemcpyAsync(b->d_views, b->h_views[k], sizeof(SessionView) * b->nslots, cudaMemcpyHostToDevice, st);
     IngestArgs a{0, 0, nullptr, 0, nullptr, 0};
     const int groups = effective_groups(b);
@@ -1137,7 +1219,7 @@ static void batch_enqueue(gbf_batch *b, int k, cudaStream_t st) {
     if (stag)
         cudaMemcpyAsync(b->d_views_b, b->h_views_b[k], sizeof(SessionView) * b->nslots, cudaMemcpyHostToDevice, st);
     if (groups <= 1) {
-        enqueue_frame(b->d_views, b->nslots, b->ex, b->layouts, a, true, st, b->timing ? b->pev[k] : nullptr);
+        enqueue_frame(b->d_views, b->nslots, b->ex, b->layouts, a, alone, st, b->timing ? b->pev[k] : nullptr);
         batch_results(b, k, st);
         return;
     }
@@ -1418,23 +1500,30 @@ GBF_API gbf_status gbf_batch_process(gbf_batch *b, const uint8_t *active, int32_
             if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: tuner event");
         }
     }
+    unsigned number;
+    const bool few = flight_send(b->flight, st, &number);
+    hv[0].tick_done = number ? b->flight.done : nullptr;
+    hv[0].tick_number = number;
+    // the launches differ only where the sessions would track in one run
+    const bool alone = few || effective_groups(b) > 1 || !track_run_fits(b->nslots, b->ex);
     if (use_graph) {
-        if (!b->exec[k]) {
+        cudaGraphExec_t &exec = b->exec[k][alone ? 0 : 1];
+        if (!exec) {
             cudaGraph_t g = nullptr;
             cudaError_t e = cudaStreamBeginCapture(b->own, cudaStreamCaptureModeThreadLocal);
             if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: begin capture");
-            batch_enqueue(b, k, b->own);
+            batch_enqueue(b, k, alone, b->own);
             e = cudaStreamEndCapture(b->own, &g);
             if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: end capture");
-            e = cudaGraphInstantiate(&b->exec[k], g, 0);
+            e = cudaGraphInstantiate(&exec, g, 0);
             cudaGraphDestroy(g);
             if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: instantiate");
             b->captures += 1;
         }
-        cudaError_t e = cudaGraphLaunch(b->exec[k], st);
+        cudaError_t e = cudaGraphLaunch(exec, st);
         if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: launch");
     } else {
-        batch_enqueue(b, k, st);
+        batch_enqueue(b, k, alone, st);
     }
     if (b->tick_cand[k] >= 0) {
         cudaError_t e = cudaEventRecord(b->tev[k][1], st);

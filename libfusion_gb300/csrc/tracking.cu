@@ -1292,6 +1292,7 @@ __global__ void slot_results_kernel(const SessionView *__restrict__ svs, int n, 
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const SessionView &sv = svs[i];
+    if (sv.tick_done) *static_cast<volatile unsigned *>(sv.tick_done) = sv.tick_number;
     gbf_slot_result r;
     if (!sv.ts) {  // empty slot
         for (int j = 0; j < 16; ++j) r.pose[j] = 0.0;

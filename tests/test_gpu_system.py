@@ -1001,3 +1001,50 @@ def test_tuning_reports_the_groups_in_use(gbf):
     batch.set_groups(3)
     assert batch.tuning()["chosen"]["groups"] == 3
     batch.close()
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_frames_on_streams_of_their_own_overlap(gbf, batched):
+    """Eight sessions, or batches of two, each on a stream of its own: beside the frames of
+    several other streams none takes the whole chip for its tracking, and a round of
+    all eight takes less than half of what it takes on one stream."""
+    import time
+
+    import torch
+    L = gbf
+    K = H.intrinsics(L, 320, 240)
+    cfg = H.small_config(L, 2, num_blocks=1 << 14, num_buckets=1 << 16)
+    n, nf, per = 8, 24, 2 if batched else 1
+    fr = [(H.cuda(d), H.cuda(c), T) for d, c, T in H.frames(L, K, nf, seed=3)]
+    ss = [L.System(K, cfg) for _ in range(n * per)]
+    batches = [L.FusionBatch(per) for _ in range(n if batched else 0)]
+    for i, b in enumerate(batches):
+        for j in range(per):
+            b.set(j, ss[i * per + j])
+
+    def rounds(streams):
+        for s in ss:
+            s.reset()
+            s.set_pose(fr[0][2])
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        for d, c, _ in fr:
+            for i in range(n):
+                if batched:
+                    for j in range(per):
+                        batches[i].set_inputs(j, d.data_ptr(), c.data_ptr())
+                    batches[i].process([True] * per, stream=streams[i])
+                else:
+                    ss[i].process_images(d, c, stream=streams[i])
+        torch.cuda.synchronize()
+        t = time.perf_counter() - t
+        poses = np.stack([s.get_camera_pose() for s in ss])
+        assert np.array_equal(poses, np.broadcast_to(poses[0], poses.shape))
+        return t, poses[0]
+    streams = [torch.cuda.Stream() for _ in range(n)]
+    runs = [(rounds(streams[:1] * n), rounds(streams)) for _ in range(4)][1:]  # the first captures the ticks
+    (one, p), (own, q) = (min((r[i] for r in runs), key=lambda x: x[0]) for i in (0, 1))
+    assert np.array_equal(p, q)
+    assert own < 0.5 * one, f"{1e6 * own / nf:.0f} us a round on eight streams, {1e6 * one / nf:.0f} on one"
+    for b in batches:
+        b.close()
