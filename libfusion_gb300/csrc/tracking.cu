@@ -875,15 +875,6 @@ __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long lon
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-// Two words from L2; each carries its own number, so they need not arrive together.  The
-// plain load moves five times the bytes of relaxed ones, but only those are sure to see
-// a store in the end: whoever reads again reads relaxed.
-__device__ __forceinline__ ulonglong2 ld_l2(const unsigned long long *p, bool again) {
-    if (again) return make_ulonglong2(ld_relaxed(p), ld_relaxed(p + 1));
-    ulonglong2 v;
-    asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ void st_relaxed(unsigned long long *p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -916,8 +907,10 @@ __device__ __forceinline__ unsigned long long *record_word(const SessionView &sv
 // The sums of the item numbered `number`, by all threads of CTA 0: warp g waits
 // for ten of the records g, g + 16, ... at a time (a lane per record looks at its first
 // word), then lane q adds columns 2 q and 2 q + 1 of them in turn; the 16 groups follow in
-// order (the sums and the order of sum_partials).  The words are read ten in
-// flight (ld_l2) and checked by their numbers.  Only the records that come last are
+// order (the sums and the order of sum_partials).  The words are read twenty in
+// flight and checked by their numbers: one relaxed load a word, since another CTA may be
+// storing it (a plain load of two words promises neither whole words nor that a
+// store is seen, and took longer: a 1280x720 run 224 us, 217 so).  Only the records that come last are
 // then left to read when the last tile is done (waiting for thirty at a time, as many as fit
 // the lanes, left a 1280x720 image's whole second half).  Records past the last
 // count as zeros, which add nothing.
@@ -933,17 +926,17 @@ __device__ __forceinline__ bool sum_records(TrackSmem &sm, const SessionView &sv
         while (!__all_sync(0xffffffffu, !mine || number_of(ld_relaxed(record_word(sv, r, 0))) == number) &&
                !__any_sync(0xffffffffu, limit.over())) {}
         ulonglong2 w[kBatch];
-        bool all, again = false;
+        bool all;
         do {
             all = true;
 #pragma unroll
             for (int i = 0; i < kBatch; ++i) {
                 w[i] = make_ulonglong2(tagged(number, 0u), tagged(number, 0u));
-                if (c + i * kSumGroups < n) w[i] = ld_l2(record_word(sv, c + i * kSumGroups, q), again);
+                const unsigned long long *p = record_word(sv, c + i * kSumGroups, q);
+                if (c + i * kSumGroups < n) w[i] = make_ulonglong2(ld_relaxed(p), ld_relaxed(p + 1));
             }
 #pragma unroll
             for (int i = 0; i < kBatch; ++i) all = all && number_of(w[i].x) == number && number_of(w[i].y) == number;
-            again = true;
         } while (!__all_sync(0xffffffffu, all) && !__any_sync(0xffffffffu, limit.over()));
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) {
