@@ -96,8 +96,8 @@ __global__ void __launch_bounds__(kTileThreads, 4) ingest_kernel(const SessionVi
                 }
             }
         };
-        if (a.src == 2) load([](const char *row, int x) { return __ldg(reinterpret_cast<const float *>(row) + x); });
-        else load([](const char *row, int x) { return (float)__ldg(reinterpret_cast<const uint16_t *>(row) + x) * 0.001f; });
+        if (a.src == 2) load([](const char *row, int x) { return reinterpret_cast<const float *>(row)[x]; });
+        else load([](const char *row, int x) { return (float)reinterpret_cast<const uint16_t *>(row)[x] * 0.001f; });
     }
     {
         const uint8_t *rgb = a.src == 0 ? sv.in_rgb : a.rgb;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) ingest_kernel(const SessionVi
             const bool in = r < kG && y >= 0 && y < H && (levels > 1 || (r >= kGrey && r < kGrey + kTile));
             const auto load = [&](int x) {
                 const uint8_t *px = rgb + y * pitch + (long long)x * 3;
-                return make_uchar4(__ldg(px), __ldg(px + 1), __ldg(px + 2), 0);
+                return make_uchar4(px[0], px[1], px[2], 0);
             };
             ca[k] = cb[k] = make_uchar4(0, 0, 0, 0);
             if (in && x0 + lane < W) ca[k] = load(x0 + lane);

@@ -247,11 +247,11 @@ __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__res
 template <int LAYOUT, class SV>
 __device__ __forceinline__ float sdf_raw(const SV &sv, int i, bool &valid) {
     if (LAYOUT == GBF_VOXEL_REF) {
-        const uint2 q = __ldg(reinterpret_cast<const uint2 *>(sv.vox_sw) + i);
+        const uint2 q = reinterpret_cast<const uint2 *>(sv.vox_sw)[i];
         valid = __uint_as_float(q.y) != 0.f;
         return sdf_ref_unpack((short)(q.x & 0xffffu));
     } else {
-        const unsigned q = __ldg(reinterpret_cast<const unsigned *>(sv.vox_sw) + i);
+        const unsigned q = reinterpret_cast<const unsigned *>(sv.vox_sw)[i];
         valid = (q & 0x7fff0000u) != 0u;  // binary16 weight != +-0 (NaN counts as observed, as w != 0.f)
         return sdf_word_unpack<LAYOUT>((unsigned short)(q & 0xffffu));
     }
@@ -285,9 +285,9 @@ __device__ __noinline__ float interp_spanning(const SV sv, int i000, int x0, int
     // corner k = (x, y, z bits) lies in the block of k's bits that step over a block face
     const int step = ((x1 >> 3) != (x0 >> 3) ? 1 : 0) | ((y1 >> 3) != (y0 >> 3) ? 2 : 0) | ((z1 >> 3) != (z0 >> 3) ? 4 : 0);
     const int *next = sv.bnext + (size_t)i000 * 8;
-    const int i100 = __ldg(next + (1 & step)), i010 = __ldg(next + (2 & step)), i110 = __ldg(next + (3 & step));
-    const int i001 = __ldg(next + (4 & step)), i101 = __ldg(next + (5 & step)), i011 = __ldg(next + (6 & step));
-    const int i111 = __ldg(next + (7 & step));
+    const int i100 = next[1 & step], i010 = next[2 & step], i110 = next[3 & step];
+    const int i001 = next[4 & step], i101 = next[5 & step], i011 = next[6 & step];
+    const int i111 = next[7 & step];
     bool v0, v1, v2, v3, v4, v5, v6, v7;
     const float c000 = vox_in<LAYOUT>(sv, i000, x0, y0, z0, v0), c100 = vox_in<LAYOUT>(sv, i100, x1, y0, z0, v1);
     const float c010 = vox_in<LAYOUT>(sv, i010, x0, y1, z0, v2), c110 = vox_in<LAYOUT>(sv, i110, x1, y1, z0, v3);
