@@ -86,12 +86,18 @@ __device__ __forceinline__ void for_cells(int x0, int y0, int x1, int y1, const 
     }
 }
 
+__device__ __forceinline__ float list_near(const SessionView &sv) {
+    return sv.ctr[C_DEEP_SDF] ? __int_as_float(0xff800000) : sv.zmin_r - kListSdf * sv.tau;
+}
+
 // Whether a sample of a raycast at this pose, or the refined one of a hit, can lie in
 // the block.  The refined sample lies before the one that found the hit by sdf x
 // truncation, and so up to kListSdf truncations before the near plane (a fused sdf is
-// never below -1; with an imported one that is, mark_block takes every block).  Only a
+// never below -1; with an imported one that is, every block counts).  Only a
 // block that a marched sample can meet marks slices.
-__device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tcw, float margin, const int4 bc) {
+// near: the depth from which blocks count (list_near).
+__device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tcw, float margin, float near,
+                                            const int4 bc) {
     const LevelK &K = sv.lv[0];
     const float h = 0.5f * sv.block_metric;
     const float3 p = Tcw.apply(((float)bc.x + 0.5f) * sv.block_metric, ((float)bc.y + 0.5f) * sv.block_metric,
@@ -101,14 +107,14 @@ __device__ __forceinline__ bool mark_slices(const SessionView &sv, const M34 &Tc
     const float hy = h * (fabsf(Tcw.m[4]) + fabsf(Tcw.m[5]) + fabsf(Tcw.m[6])) + margin;
     const float hz = h * (fabsf(Tcw.m[8]) + fabsf(Tcw.m[9]) + fabsf(Tcw.m[10])) + margin;
     const float z0 = p.z - hz, z1 = p.z + hz;
-    if (!(z1 >= sv.zmin_r - kListSdf * sv.tau)) return false;
+    if (!(z1 >= near)) return false;
     int cx0 = 0, cx1 = sv.zr_w - 1, cy0 = 0, cy1 = sv.zr_h - 1;
     if (z0 > 0.25f * sv.zmin_r) {
         const float i0 = 1.f / z0, i1 = 1.f / z1;
         const float xl = p.x - hx, xh = p.x + hx, yl = p.y - hy, yh = p.y + hy;
         const float ul = K.fx * (xl * (xl < 0.f ? i0 : i1)) + K.cx - 2.f, uh = K.fx * (xh * (xh < 0.f ? i1 : i0)) + K.cx + 2.f;
         const float vl = K.fy * (yl * (yl < 0.f ? i0 : i1)) + K.cy - 2.f, vh = K.fy * (yh * (yh < 0.f ? i1 : i0)) + K.cy + 2.f;
-        if (uh < 0.f || vh < 0.f || ul > (float)K.w || vl > (float)K.h) return false;
+        if (uh < 0.f || vh < 0.f || ul > (float)K.w || vl > (float)K.h) return isinf(near);
         cx0 = max(0, (int)(ul * 0.125f));
         cx1 = min(cx1, (int)(uh * 0.125f));
         cy0 = max(0, (int)(vl * 0.125f));
@@ -176,10 +182,10 @@ __device__ __forceinline__ void mark_zrange(const SessionView &sv, const Corner 
 }
 
 // The slices of an allocated block and, where rays may meet it, its neighbours' ids.
-__device__ __forceinline__ void mark_block(const SessionView &sv, const M34 &Tcw, float margin, bool deep, const int4 bc,
+__device__ __forceinline__ void mark_block(const SessionView &sv, const M34 &Tcw, float margin, float near, const int4 bc,
                                            int id) {
     const int c = threadIdx.x & 7;
-    if (mark_slices(sv, Tcw, margin, bc) || deep)
+    if (mark_slices(sv, Tcw, margin, near, bc))
         sv.bnext[(size_t)id * 8 + c] =
             c == 0 ? id : find_block(sv, bc.x + (c & 1), bc.y + ((c >> 1) & 1), bc.z + (c >> 2));
 }
@@ -201,13 +207,13 @@ __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__res
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     __shared__ M34 Tcw;
-    __shared__ float margin;
+    __shared__ float margin, near;
     if (threadIdx.x < 12) Tcw.m[threadIdx.x] = sv.ts->map_tcw[threadIdx.x];
     if (threadIdx.x == 32) margin = ray_margin(sv);
+    if (threadIdx.x == 64) near = list_near(sv);
     __syncthreads();
     const int c = threadIdx.x & 7, per_cta = blockDim.x / 8, lists = LIST ? gridDim.x / 2 : 0;
     const int used = min(sv.ctr[C_NUSED], sv.pool);
-    const bool deep = sv.ctr[C_DEEP_SDF] != 0;
     if (LIST && blockIdx.x < lists) {
         const int nvis = sv.ctr[C_NVIS];
         // whole warps iterate together: the corners meet by shuffles
@@ -220,7 +226,7 @@ __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__res
     }
     const int first = (blockIdx.x - lists) * per_cta, stride = (gridDim.x - lists) * per_cta;
     if (LIST) {
-        for (int id = first + threadIdx.x / 8; id < used; id += stride) mark_block(sv, Tcw, margin, deep, sv.bcoord[id], id);
+        for (int id = first + threadIdx.x / 8; id < used; id += stride) mark_block(sv, Tcw, margin, near, sv.bcoord[id], id);
         return;
     }
     const int frame = sv.ctr[C_FRAME] + 1;
@@ -236,7 +242,7 @@ __global__ void __launch_bounds__(256, 6) zrange_kernel(const SessionView *__res
         const int pos = warp_append(sv.ctr + C_NVIS, visible && c == 0);
         if (visible && c == 0) sv.vis[pos] = id | (sv.bfresh[id] ? (int)0x80000000 : 0);
         mark_zrange(sv, k, visible);
-        if (b < used) mark_block(sv, Tcw, margin, deep, bc, id);
+        if (b < used) mark_block(sv, Tcw, margin, near, bc, id);
         __syncwarp();
     }
 }
