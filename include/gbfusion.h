@@ -280,7 +280,11 @@ GBF_API gbf_status gbf_get_image(gbf_session *s, int32_t which, int32_t kind, in
 /* ---- full frame: System::process_images -------------------------------------- */
 /* ingest (u16 mm -> m, rgb -> gray, pyramids) -> track against the model
  * prediction -> fuse raw depth at the new pose -> raycast the new reference
- * vertex map -> rebuild its pyramid.  No host synchronisation. */
+ * vertex map -> rebuild its pyramid.  No host synchronisation.
+ * Tracking takes one launch over every SM, or, beside frames and ticks on two or more
+ * other streams, a launch per iteration.  The one launch starts when the SMs are free: a
+ * caller's kernel that stays on the GPU until a frame has ended would wait for ever
+ * (so for gbf_track, and for ticks of one group, see gbf_batch_set_groups). */
 GBF_API gbf_status gbf_process_frame(gbf_session *s, const uint16_t *depth_mm_dev, int64_t depth_pitch,
                                      const uint8_t *rgb_dev, int64_t rgb_pitch, void *stream);
 /* Same, from the session's own staging buffers (gbf_session_inputs). */
@@ -495,7 +499,8 @@ GBF_API gbf_status gbf_batch_set_timing(gbf_batch *b, int32_t enable);
 /* Mean durations (ms) of the 7 phases over the ticks since timing was enabled
  * (waits for the outstanding ticks); ms[7], when n > 7, receives the tick count. */
 GBF_API gbf_status gbf_batch_phase_ms(gbf_batch *b, float *ms, int32_t n);
-/* Number of kernel launches one tick makes. */
+/* Number of kernel launches one tick makes (where few sessions track in one
+ * launch, as gbf_batch_set_groups says: with no other stream's frames beside it). */
 GBF_API gbf_status gbf_batch_kernels(gbf_batch *b, int32_t *n);
 /* Tick graphs the batch has captured so far (one per tick parity for each tick
  * shape; a change of shape, groups, stagger, tile or timing drops them.  Few

@@ -698,18 +698,17 @@ __global__ void nmap_all_kernel(const SessionView *__restrict__ svs, unsigned *d
 
 }  // namespace
 
-// CTAs per session: up to three resident ones per SM, fewer of many sessions, whose CTAs loop
+// CTAs per session: six per SM, as many as are resident (an even number: with a
+// list, half of them take it), fewer of many sessions, whose CTAs loop
 static int zrange_ctas(const Extent &ex, int nslots) {
-    return min(max((ex.max_pool + 31) / 32, 1), max(152, 152 * 3 / nslots));
+    return 2 * min(max((ex.max_pool + 31) / 32, 1), max(152, 152 * 3 / nslots));
 }
 void launch_zrange(const SessionView *d_sv, int nslots, const Extent &ex, ZrangeOf of, cudaStream_t st) {
-    const int n = zrange_ctas(ex, nslots);
-    const auto go = [&](auto *kernel, int halves) {
-        launch_kernel(kernel, dim3(n * halves, nslots), 256, ex.chain, st, d_sv);
-    };
-    if (of == ZrangeOf::list) go(zrange_kernel<true, false>, 2);
-    else if (of == ZrangeOf::frustum) go(zrange_kernel<false, false>, 2);
-    else go(zrange_kernel<false, true>, 2);
+    const dim3 g(zrange_ctas(ex, nslots), nslots);
+    const auto go = [&](auto *kernel) { launch_kernel(kernel, g, 256, ex.chain, st, d_sv); };
+    if (of == ZrangeOf::list) go(zrange_kernel<true, false>);
+    else if (of == ZrangeOf::frustum) go(zrange_kernel<false, false>);
+    else go(zrange_kernel<false, true>);
 }
 
 void launch_march(const SessionView *d_sv, int nslots, const Extent &ex, float4 *vmap_ext, long long vmap_pitch,
