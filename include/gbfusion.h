@@ -503,9 +503,7 @@ GBF_API gbf_status gbf_batch_phase_ms(gbf_batch *b, float *ms, int32_t n);
  * launch, as gbf_batch_set_groups says: with no other stream's frames beside it). */
 GBF_API gbf_status gbf_batch_kernels(gbf_batch *b, int32_t *n);
 /* Tick graphs the batch has captured so far (one per tick parity for each tick
- * shape; a change of shape, groups, stagger, tile or timing drops them.  Few
- * sessions, which track in one launch, have a second one for ticks beside frames
- * on two or more other streams).  A
+ * shape; a change of shape, groups, stagger, tile or timing drops them).  A
  * server watches it to see that admissions and evictions do not re-capture. */
 GBF_API gbf_status gbf_batch_captures(gbf_batch *b, int64_t *n);
 

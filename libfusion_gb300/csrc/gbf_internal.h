@@ -74,7 +74,7 @@ struct gbf_batch {
     gbf::SessionView *d_views = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     bool ev_used[2] = {false, false};
-    cudaGraphExec_t exec[2][2] = {};  // per mirror: alone on the chip, beside other streams' work
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};
     gbf::Flight flight;
     cudaStream_t own = nullptr;
     int flip = 0;

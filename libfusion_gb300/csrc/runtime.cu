@@ -147,19 +147,30 @@ std::vector<Flight *> &g_flights = *new std::vector<Flight *>;
 
 unsigned flight_done(const Flight &f) { return *static_cast<volatile unsigned *>(f.done); }
 
-cudaError_t flight_open(Flight &f) {
+// The words come from pinned pages of 1,024 that stay for the process and serve one session
+// or batch after the other.  Without one (no page to be had) nothing is counted.
+std::vector<unsigned *> &g_flight_words = *new std::vector<unsigned *>;
+
+void flight_open(Flight &f) {
     cudaGetDevice(&f.device);
-    const cudaError_t e = cudaHostAlloc(&f.done, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
-    if (e == cudaSuccess) *f.done = 0;
-    return e;
+    std::lock_guard<std::mutex> lock(g_flight_mu);
+    if (g_flight_words.empty()) {
+        unsigned *page = nullptr;
+        if (cudaHostAlloc(&page, 4096, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        for (int i = 0; i < 1024; ++i) g_flight_words.push_back(page + i);
+    }
+    f.done = g_flight_words.back();
+    g_flight_words.pop_back();
+    *static_cast<volatile unsigned *>(f.done) = 0;
 }
 
-void flight_close(Flight &f) {  // the device is idle
-    {
-        std::lock_guard<std::mutex> lock(g_flight_mu);
-        g_flights.erase(std::remove(g_flights.begin(), g_flights.end(), &f), g_flights.end());
-    }
-    if (f.done) cudaFreeHost(f.done);
+void flight_close(Flight &f) {
+    std::lock_guard<std::mutex> lock(g_flight_mu);
+    g_flights.erase(std::remove(g_flights.begin(), g_flights.end(), &f), g_flights.end());
+    if (f.done) g_flight_words.push_back(f.done);
     f.done = nullptr;
 }
 
@@ -174,7 +185,7 @@ bool capturing(cudaStream_t st) {
 // frame is not counted: what its replays run beside is not known.
 bool flight_send(Flight &f, cudaStream_t st, unsigned *number) {
     *number = 0;
-    if (capturing(st)) return true;
+    if (!f.done || capturing(st)) return true;
     std::lock_guard<std::mutex> lock(g_flight_mu);
     g_flights.erase(std::remove_if(g_flights.begin(), g_flights.end(),
                                    [&](Flight *o) { return o == &f || (int)(o->sent - flight_done(*o)) <= 0; }),
@@ -471,11 +482,7 @@ GBF_API gbf_status gbf_session_create(const gbf_config *cfg, const gbf_intrinsic
         delete s;
         return cuda_error(e, "gbf_session_create: view");
     }
-    e = flight_open(s->flight);
-    if (e != cudaSuccess) {
-        gbf_session_destroy(s);
-        return cuda_error(e, "gbf_session_create: host word");
-    }
+    flight_open(s->flight);
     char *base = static_cast<char *>(s->arena);
     const ArenaLayout &a = s->lay;
     SessionView &v = s->view;
@@ -1022,7 +1029,7 @@ GBF_API gbf_status gbf_batch_create(int32_t max_sessions, gbf_batch **out) {
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[g], cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = flight_open(b->flight);
+    if (e == cudaSuccess) flight_open(b->flight);
     for (int k = 0; k < 2; ++k) {
         b->stg_depth[k].assign(max_sessions, nullptr);
         b->stg_rgb[k].assign(max_sessions, nullptr);
@@ -1047,11 +1054,10 @@ GBF_API gbf_status gbf_batch_create(int32_t max_sessions, gbf_batch **out) {
 
 static void batch_invalidate(gbf_batch *b) {
     for (int k = 0; k < 2; ++k)
-        for (cudaGraphExec_t &x : b->exec[k])
-            if (x) {
-                cudaGraphExecDestroy(x);
-                x = nullptr;
-            }
+        if (b->exec[k]) {
+            cudaGraphExecDestroy(b->exec[k]);
+            b->exec[k] = nullptr;
+        }
 }
 
 GBF_API gbf_status gbf_batch_destroy(gbf_batch *b) {
@@ -1504,23 +1510,24 @@ GBF_API gbf_status gbf_batch_process(gbf_batch *b, const uint8_t *active, int32_
     const bool few = flight_send(b->flight, st, &number);
     hv[0].tick_done = number ? b->flight.done : nullptr;
     hv[0].tick_number = number;
-    // the launches differ only where the sessions would track in one run
+    // Where the sessions would track in one run but had better not, the tick is launched
+    // directly: a second graph would be captured whenever such a tick first comes, and no thread may
+    // wait for the device meanwhile.
     const bool alone = few || effective_groups(b) > 1 || !track_run_fits(b->nslots, b->ex);
-    if (use_graph) {
-        cudaGraphExec_t &exec = b->exec[k][alone ? 0 : 1];
-        if (!exec) {
+    if (use_graph && alone) {
+        if (!b->exec[k]) {
             cudaGraph_t g = nullptr;
             cudaError_t e = cudaStreamBeginCapture(b->own, cudaStreamCaptureModeThreadLocal);
             if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: begin capture");
-            batch_enqueue(b, k, alone, b->own);
+            batch_enqueue(b, k, true, b->own);
             e = cudaStreamEndCapture(b->own, &g);
             if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: end capture");
-            e = cudaGraphInstantiate(&exec, g, 0);
+            e = cudaGraphInstantiate(&b->exec[k], g, 0);
             cudaGraphDestroy(g);
             if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: instantiate");
             b->captures += 1;
         }
-        cudaError_t e = cudaGraphLaunch(exec, st);
+        cudaError_t e = cudaGraphLaunch(b->exec[k], st);
         if (e != cudaSuccess) return cuda_error(e, "gbf_batch_process: launch");
     } else {
         batch_enqueue(b, k, alone, st);
