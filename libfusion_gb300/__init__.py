@@ -118,8 +118,8 @@ class _Session:
 
     def close(self) -> None:
         if self._h:
-            call("gbf_session_destroy", self._h)
-            self._h = C.c_void_p()
+            h, self._h = self._h, C.c_void_p()  # gone whatever the call returns
+            call("gbf_session_destroy", h)
 
     def __del__(self):
         try:
@@ -465,8 +465,8 @@ class FusionBatch:
         """Destroy the batch and let go of the sessions in its slots (they stay
         usable on their own)."""
         if self._h:
-            call("gbf_batch_destroy", self._h)
-            self._h = C.c_void_p()
+            h, self._h = self._h, C.c_void_p()  # gone whatever the call returns
+            call("gbf_batch_destroy", h)
         self.slots = [None] * len(self.slots)
 
     def __del__(self):
@@ -560,8 +560,8 @@ class SynthScene:
 
     def close(self):
         if self._h:
-            call("gbf_synth_destroy", self._h)
-            self._h = C.c_void_p()
+            h, self._h = self._h, C.c_void_p()
+            call("gbf_synth_destroy", h)
 
     def __del__(self):
         try:

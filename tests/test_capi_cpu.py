@@ -84,3 +84,25 @@ def test_session_create_without_gpu_fails_loudly(L):
     with pytest.raises(L.GbfError) as e:
         L.System(K, L.default_config())
     assert e.value.status in (2, 5)
+
+
+@pytest.mark.parametrize("kind,name", [("System", "gbf_session_destroy"), ("FusionBatch", "gbf_batch_destroy"),
+                                       ("SynthScene", "gbf_synth_destroy")])
+def test_a_failed_destroy_is_not_repeated(L, monkeypatch, kind, name):
+    """Destroying frees the handle whatever it returns (an error of the device's, say): closing
+    again, or the collector, must not pass it on a second time."""
+    calls = []
+
+    def call(what, *args):
+        calls.append((what, args[0].value))
+        raise L.GbfError(5, what, "device error")
+    cls = getattr(L, kind)
+    x = object.__new__(cls)
+    x._h = C.c_void_p(4096)
+    x.slots = []
+    monkeypatch.setattr(L, "call", call)
+    with pytest.raises(L.GbfError):
+        x.close()
+    x.close()
+    x.__del__()
+    assert calls == [(name, 4096)]
