@@ -281,10 +281,8 @@ GBF_API gbf_status gbf_get_image(gbf_session *s, int32_t which, int32_t kind, in
 /* ingest (u16 mm -> m, rgb -> gray, pyramids) -> track against the model
  * prediction -> fuse raw depth at the new pose -> raycast the new reference
  * vertex map -> rebuild its pyramid.  No host synchronisation.
- * Tracking takes one launch over every SM, or, beside frames and ticks on two or more
- * other streams, a launch per iteration.  The one launch starts when the SMs are free: a
- * caller's kernel that stays on the GPU until a frame has ended would wait for ever
- * (so for gbf_track, and for ticks of one group, see gbf_batch_set_groups). */
+ * Tracking takes one launch over the SMs that no other kernel holds, or, beside frames
+ * and ticks on two or more other streams, a launch per iteration; the results are the same. */
 GBF_API gbf_status gbf_process_frame(gbf_session *s, const uint16_t *depth_mm_dev, int64_t depth_pitch,
                                      const uint8_t *rgb_dev, int64_t rgb_pitch, void *stream);
 /* Same, from the session's own staging buffers (gbf_session_inputs). */

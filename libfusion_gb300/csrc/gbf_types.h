@@ -64,6 +64,7 @@ enum Counter {
     C_TRACK_PUB = 16, // 14 8-byte words published within a tracking run (gn_track_kernel)
     C_TRACK_BASE = 44,    // arrivals of CTAs over the session's tracking runs until this one
     C_TRACK_ARRIVED = 45, // and so far
+    C_TRACK_CREW = 46,    // 8-byte word: the CTAs that share the run's tiles
     C_WORDS = 64      // ints in the arena
 };
 

@@ -736,7 +736,7 @@ __global__ void track_finish_kernel(const SessionView *__restrict__ svs, int fra
 
 // ---------------------------------------------------------------------------
 // A whole tracking run (every level and iteration, from the initial estimate to
-// the frame's pose) in one cooperative launch, for launches of few sessions.
+// the frame's pose) in one launch, for launches of few sessions.
 //
 // What bounds such a run is latency.  A launch per iteration costs one 640x480
 // session about 18 us: the launch, the dependent loads from the descriptor to the
@@ -774,8 +774,8 @@ struct TrackSmem {
     TrackState ts;  // CTA 0: the run's tracking state
     float pose[12];
     float stddev, huber;
-    unsigned seen;
-    int item, lost, late;
+    unsigned seen, base, order;
+    int item, lost, crew;
 };
 
 // icp_row and rgb_row of one pixel, with their gathers issued together (a row
@@ -844,8 +844,8 @@ __device__ __forceinline__ void chain_sums(const float4 *lo, const float4 *hi, i
 }
 
 // A CTA of the run waits for another at most this long (CTA 0: SessionView::track_wait_ns).
-// Every CTA is resident and a step takes microseconds: the limit only bounds a wait that
-// cannot happen.
+// The CTAs of a run are resident (gather_crew) and a step takes microseconds: the limit
+// only bounds a wait that cannot happen.
 struct WaitLimit {
     long long ns, t0 = 0;
     int n = 0, every;
@@ -1019,10 +1019,45 @@ __device__ __forceinline__ void track_steps(TrackSmem &sm, const SessionView &sv
         reinterpret_cast<int *>(sv.ts)[i] = reinterpret_cast<const int *>(ts)[i];
 }
 
-// The tiles of a run: CTA cta of the ctas that follow CTA 0 makes its tiles' records of each item.
-// Thread 0's: the arrivals before this run, and before this CTA's.
-__device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv, int item, unsigned seen, int rs, int cta,
-                                            int ctas, unsigned base, unsigned arrival) {
+// How many CTAs share a run's tiles: CTA 0 waits until the launch's ctas have arrived, or
+// for so long that the rest are not about to (another stream's kernel holds their SMs,
+// or the stream has fewer), and goes on with those that have: they run, and so every
+// wait of the run ends, without a cooperative launch, which starts only once all can.  (A
+// 320x240 frame beside a kernel of one CTA and 5 ms on another stream took 4.96 ms so,
+// and takes 0.31; on a stream of 64 SMs, which refuses the cooperative grid, 0.42 ms with
+// launches per iteration and 0.33 so.)  Not long where most have come, longer where few
+// have, as while another kernel's CTAs end: patience of 100 or 250 us gained nothing
+// beside matrix products or a batch's ticks, and cost a stream of 64 SMs 57 or 203 us.
+// False when it took too long or no other CTA came.
+constexpr long long kCrewQuiet = 40000, kCrewPatience = 80000;  // cycles: 20 and 40 us
+__device__ __forceinline__ unsigned long long *crew_word(const SessionView &sv) {
+    return reinterpret_cast<unsigned long long *>(sv.ctr + C_TRACK_CREW);
+}
+__device__ __forceinline__ bool gather_crew(const SessionView &sv, unsigned base, unsigned ctas, int item, unsigned seen) {
+    WaitLimit limit(sv.track_wait_ns);
+    const long long start = clock64();
+    long long quiet = start;
+    unsigned n, last = 0;
+    while ((n = ld_acquire(sv.ctr + C_TRACK_ARRIVED) - base) != ctas && !limit.over()) {
+        const long long t = clock64();
+        if (n != last) quiet = t;
+        last = n;
+        if (n > 1 && t - quiet > kCrewQuiet && (2 * n > ctas || t - start > kCrewPatience)) break;
+    }
+    unsigned next = base + ctas;
+    if (n != ctas) {
+        n = atom_add(sv.ctr + C_TRACK_ARRIVED, kRunClosed) - base;
+        next += kRunClosed;
+    }
+    sv.ctr[C_TRACK_BASE] = (int)next;
+    // (a run without items publishes nothing, so that the next one starts from the same number)
+    if (item > 0) st_relaxed(crew_word(sv), tagged(seen + 1, n - 1));
+    return !limit.ran_out && n > 1;
+}
+
+// The tiles of a run: CTA cta of those that follow CTA 0 makes its tiles' records of each item.
+__device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv, int item, unsigned seen, int rs,
+                                            int cta) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned long long *pub = reinterpret_cast<const unsigned long long *>(sv.ctr + C_TRACK_PUB);
     const float qnan = __int_as_float(0x7fffffff);
@@ -1030,6 +1065,18 @@ __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv
     float4 v[kTrackPixels], m[kTrackPixels];  // this thread's reference pixels of the CTA's next tile
     float il[kTrackPixels];
     int loaded = -1;  // the level they belong to
+    int ctas = 0;     // not known before the first tile's rows are made
+    const auto read_crew = [&]() {
+        if (warp == 0) {
+            WaitLimit limit(kTrackWaitNs);
+            unsigned long long w = ld_relaxed(crew_word(sv));
+            while (number_of(w) != seen + 1 && !limit.over()) w = ld_relaxed(crew_word(sv));
+            if (lane == 0) sm.crew = limit.ran_out ? 0 : (int)(unsigned)w;
+            __syncwarp();
+        }
+        __syncthreads();
+        ctas = sm.crew;
+    };
     while (item > 0) {
         const int level = (item >> 10) - 1;
         const LevelIn in = level_in(sv, level, 1 - rs);
@@ -1056,15 +1103,16 @@ __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv
 #pragma unroll
             for (int i = 0; i < 12; ++i) T.m[i] = sm.pose[i];
             const PhotoConst pc = photo_const(sm.stddev, sm.huber);
-            for (int tile = cta; tile < tiles; tile += ctas) {
+            for (int tile = cta; tile < tiles; tile += ctas) {  // (ctas is known from the first one's on)
 #pragma unroll
                 for (int j = 0; j < kTrackPixels; ++j) {
                     const int k = tid + j * kTrackThreads;
                     pixel_rows(in, T, pc, v[j], m[j], il[j], sm.lo[0] + k, sm.hi[0] + k, sm.lo[1] + k, sm.hi[1] + k);
                 }
+                if (!ctas) read_crew();
+                if (!ctas) return;
                 // meanwhile the next tile's pixels, or the first one's again for the next iteration
                 load(tile + ctas < tiles ? tile + ctas : cta);
-                if (tid == 0) sm.late = arrival - base >= (unsigned)ctas;  // (the count's answer has had the gathers' time)
                 __syncwarp();
                 __syncthreads();
                 if (warp < 8) {  // ICP chains, then photometric ones
@@ -1084,16 +1132,9 @@ __device__ __forceinline__ void track_tiles(TrackSmem &sm, const SessionView &sv
                 }
             }
         } else {
-            if (tid == 0) sm.late = arrival - base >= (unsigned)ctas;
-            __syncwarp();
             __syncthreads();  // every warp has the item before the next one takes its place
-        }
-        if (sm.late) {
-            // CTA 0 had given up: `seen` may be what the next run starts from, so the
-            // records take a number that it does not wait for
-            for (int tile = cta; tile < tiles; tile += ctas)
-                if (tid < kReduceWidth) st_relaxed(record_word(sv, tile, tid), tagged(seen, 0u));
-            return;
+            if (!ctas) read_crew();
+            if (!ctas) return;
         }
         if (warp == 0) {
             unsigned value = 0;
@@ -1123,45 +1164,39 @@ __global__ void __launch_bounds__(kTrackThreads, 1)
     const SessionView &sv = svs[blockIdx.y];
     if (!sv.active) return;
     const int tid = threadIdx.x;
-    const bool head = blockIdx.x == 0;
-    // Every CTA reads these before it arrives, and CTA 0 goes on once all have:
-    // what it publishes, and the frame's end, change them.
+    // Every CTA reads these before it arrives: what CTA 0 publishes, and the frame's
+    // end, change them.
     const int rs = sv.ts->idx;
     const unsigned seen = number_of(ld_relaxed(reinterpret_cast<const unsigned long long *>(sv.ctr + C_TRACK_PUB)));
     const int item = frame_mode && !sv.ts->has_ref ? 0 : first_item(sv, sv.levels - 1);
     if (tid < 12) sm.pose[tid] = (float)sv.ts->init[tid];
     if (tid == 12) sm.stddev = sm.huber = 0.f;
-    if (head)
-        for (int i = tid; i < (int)(sizeof(TrackState) / 4); i += kTrackThreads)
-            reinterpret_cast<int *>(&sm.ts)[i] = reinterpret_cast<const int *>(sv.ts)[i];
     __syncwarp();
     __syncthreads();
-    if (!head) {
-        unsigned base = 0, arrival = 0;
-        if (tid == 0) {
-            base = ld_acquire(sv.ctr + C_TRACK_BASE);
-            arrival = atom_add(sv.ctr + C_TRACK_ARRIVED, 1u);
-        }
-        __syncwarp();
-        track_tiles(sm, sv, item, seen, rs, blockIdx.x - 1, gridDim.x - 1, base, arrival);
+    // The order of arrival is the CTA's place in the run, 0 that of "CTA 0" above.  Arrivals are
+    // counted over the session's runs: all of a run's have been made when the next one starts.
+    // A run that goes on without some of its CTAs has added kRunClosed to the count, and
+    // whichever base these read, their order is past any place.
+    if (tid == 0) {
+        const unsigned base = ld_acquire(sv.ctr + C_TRACK_BASE);
+        sm.base = base;
+        sm.order = atom_add(sv.ctr + C_TRACK_ARRIVED, 1u) - base;
+    }
+    __syncwarp();
+    __syncthreads();
+    const unsigned order = sm.order, ctas = gridDim.x;
+    if (order >= ctas) return;
+    if (order > 0) {
+        track_tiles(sm, sv, item, seen, rs, (int)order - 1);
         return;
     }
+    for (int i = tid; i < (int)(sizeof(TrackState) / 4); i += kTrackThreads)
+        reinterpret_cast<int *>(&sm.ts)[i] = reinterpret_cast<const int *>(sv.ts)[i];
+    __syncwarp();
+    __syncthreads();
     if (tid == 0) {
         track_begin(&sm.ts, frame_mode);
-        const unsigned base = ld_acquire(sv.ctr + C_TRACK_BASE), others = gridDim.x - 1;
-        // Arrivals are counted over the session's runs: every CTA of a run has arrived when
-        // the next one starts, but a run that gives up here ends before all have.  It adds
-        // kRunClosed to the count, which tells the CTAs that come then (by the order
-        // that they get, whichever base they read).
-        WaitLimit limit(sv.track_wait_ns);
-        while (ld_acquire(sv.ctr + C_TRACK_ARRIVED) - base != others && !limit.over()) {}
-        sm.lost = limit.ran_out;
-        unsigned next = base + others;
-        if (limit.ran_out) {
-            atom_add(sv.ctr + C_TRACK_ARRIVED, kRunClosed);
-            next += kRunClosed;
-        }
-        sv.ctr[C_TRACK_BASE] = (int)next;
+        sm.lost = !gather_crew(sv, sm.base, ctas, item, seen);
     }
     __syncwarp();
     __syncthreads();
@@ -1185,8 +1220,7 @@ constexpr int kTrackSubgroup = 64;
 constexpr int kDeferStepSessions = 32;
 static bool defer_step(int sessions) { return sessions >= kDeferStepSessions; }
 
-// Whether a launch that has the chip to itself takes the tracking run in one
-// cooperative kernel: track 0.25 -> 0.154 ms for one 640x480 session, 0.28 -> 0.18 for
+// Whether a launch that may take the chip tracks in one run: track 0.25 -> 0.154 ms for one 640x480 session, 0.28 -> 0.18 for
 // two, 0.34 -> 0.23 for three, 0.39 -> 0.29 for four.  More sessions share the CTAs, which
 // are then busy with their tiles most of the time; small images leave the run ahead of
 // two concurrent groups of launches (ticks of 6 sessions at 320x240, 450 level-0 tiles, 0.80
@@ -1198,8 +1232,8 @@ bool track_run_fits(int nslots, const Extent &ex) {
     return nslots <= kTrackRunFew || (nslots <= kTrackRunSessions && nslots * ex.max_red[0] <= kTrackRunTiles);
 }
 
-// CTAs of one cooperative launch of gn_track_kernel on the current device (one
-// per SM), or 0 where it cannot be launched.
+// CTAs of one launch of gn_track_kernel on the current device (one per SM), or 0 where
+// it cannot be launched.
 static int track_run_ctas() {
     static std::atomic<int> known[64];  // per device: CTAs + 1
     int dev = 0;
@@ -1207,10 +1241,9 @@ static int track_run_ctas() {
     std::atomic<int> &k = known[dev & 63];
     int c = k.load(std::memory_order_acquire);
     if (c == 0) {
-        int sms = 0, coop = 0, per = 0;
+        int sms = 0, per = 0;
         c = 1;
-        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
             cudaFuncSetAttribute(gn_track_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(TrackSmem)) ==
                 cudaSuccess &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, gn_track_kernel, kTrackThreads, sizeof(TrackSmem)) ==
@@ -1239,13 +1272,9 @@ void prepare_track() { track_run_ctas(); }
 
 void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, bool alone, cudaStream_t st) {
     if (takes_run(nslots, ex, alone)) {
-        void *args[] = {(void *)&d_sv, (void *)&frame_mode};
-        const cudaError_t e =
-            cudaLaunchCooperativeKernel((const void *)gn_track_kernel, dim3(track_run_ctas() / nslots, nslots),
-                                        dim3(kTrackThreads), args, sizeof(TrackSmem), st);
-        // a stream with fewer SMs than the device (a green context's) refuses the grid
-        if (e != cudaErrorCooperativeLaunchTooLarge) return;
-        cudaGetLastError();
+        launch_kernel_smem(gn_track_kernel, dim3(track_run_ctas() / nslots, nslots), kTrackThreads, sizeof(TrackSmem),
+                           ex.chain, st, d_sv, frame_mode);
+        return;
     }
     track_begin_kernel<<<nslots, 32, 0, st>>>(d_sv, frame_mode);
     ReduceArgs a{};

@@ -1048,3 +1048,46 @@ def test_frames_on_streams_of_their_own_overlap(gbf, batched):
     assert own < 0.5 * one, f"{1e6 * own / nf:.0f} us a round on eight streams, {1e6 * one / nf:.0f} on one"
     for b in batches:
         b.close()
+
+
+@pytest.mark.parametrize("n", [1, 4])
+def test_frames_beside_a_kernel_that_holds_an_sm(gbf, n):
+    """A caller's kernel on another stream, one CTA that spins for a fifth of a second: the
+    frames of a session, and the ticks of a few, are done before it ends, with the
+    poses they have alone."""
+    import torch
+    L = gbf
+    K = H.intrinsics(L, 320, 240)
+    cfg = H.small_config(L, 2, num_blocks=1 << 14, num_buckets=1 << 16)
+    fr = [(H.cuda(d), H.cuda(c), T) for d, c, T in H.frames(L, K, 5, seed=6)]
+    side, own = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def run(beside):
+        ss, b = [L.System(K, cfg) for _ in range(n)], L.FusionBatch(n)
+        for i, s in enumerate(ss):
+            s.set_pose(fr[0][2])
+            b.set(i, s)
+        poses, early = [], True
+        for k, (d, c, _) in enumerate(fr):
+            end = torch.cuda.Event()
+            if beside and k >= 2:  # (the ticks' graphs are captured by then)
+                with torch.cuda.stream(side):
+                    torch.cuda._sleep(400_000_000)
+                    end.record()
+            if n > 1:
+                for i in range(n):
+                    b.set_inputs(i, d.data_ptr(), c.data_ptr())
+                b.process([True] * n, stream=own)
+            else:
+                ss[0].process_images(d, c, stream=own)
+            poses.append([s.get_camera_pose(stream=own) for s in ss])
+            if beside and k >= 2:
+                early = early and not end.query()
+            torch.cuda.synchronize()
+        status = [s.stats().status for s in ss]
+        b.close()
+        return np.array(poses), status, early
+    p, st, _ = run(False)
+    q, su, early = run(True)
+    assert np.array_equal(p, q) and st == su
+    assert early, "a frame waited for the other stream's kernel"

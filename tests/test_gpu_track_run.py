@@ -1,4 +1,4 @@
-"""Inside the cooperative tracking run (csrc/tracking.cu, gn_track_kernel): what no call
+"""Inside the tracking run (csrc/tracking.cu, gn_track_kernel): what no call
 of the library reaches, by a program that shares its arena."""
 import subprocess
 from pathlib import Path
@@ -36,6 +36,6 @@ def test_run_whose_wait_ran_out(program):
 
 
 def test_frames_on_a_stream_with_few_sms(program):
-    """A green context's stream has too few SMs for the run's cooperative grid: the frame is
-    tracked in a launch per iteration, with the same result."""
+    """A green context's stream has too few SMs for all CTAs of the run at once: those that
+    are there make it, with the same result."""
     program("few_sms")

@@ -147,8 +147,8 @@ int lost(Frames &f) {
     return 0;
 }
 
-// A stream of a green context with a few of the SMs, where the run's grid does not fit:
-// the frames are those of a stream with all of them.
+// A stream of a green context with a few of the SMs, on which the run's CTAs do not fit
+// at once: the frames are those of a stream with all of them.
 int few_sms(Frames &f) {
     CUdevResource all{}, few{}, rest{};
     CUdevResourceDesc desc{};
