@@ -30,23 +30,17 @@ struct Extent {
 // their launches are 0.5 us apart, and the CTAs that wait early would take the places of the
 // other branch's.
 template <class... P, class... A>
-inline void launch_kernel_smem(void (*kernel)(P...), dim3 grid, int threads, size_t smem, bool chain, cudaStream_t st,
-                               A... args) {
+inline void launch_kernel(void (*kernel)(P...), dim3 grid, int threads, bool chain, cudaStream_t st, A... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c{};
     c.gridDim = grid;
     c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
     c.stream = st;
     c.attrs = &at;
     c.numAttrs = chain ? 1 : 0;
     cudaLaunchKernelEx(&c, kernel, P(args)...);
-}
-template <class... P, class... A>
-inline void launch_kernel(void (*kernel)(P...), dim3 grid, int threads, bool chain, cudaStream_t st, A... args) {
-    launch_kernel_smem(kernel, grid, threads, 0, chain, st, args...);
 }
 
 inline int ray_tile_width(const Extent &ex) {

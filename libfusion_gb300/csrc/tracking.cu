@@ -1272,8 +1272,11 @@ void prepare_track() { track_run_ctas(); }
 
 void launch_track(const SessionView *d_sv, int nslots, const Extent &ex, int frame_mode, bool alone, cudaStream_t st) {
     if (takes_run(nslots, ex, alone)) {
-        launch_kernel_smem(gn_track_kernel, dim3(track_run_ctas() / nslots, nslots), kTrackThreads, sizeof(TrackSmem),
-                           ex.chain, st, d_sv, frame_mode);
+        // Not chained: its CTAs, a whole SM each, would wait in places that the level maps'
+        // could use (640x480 frames, each pose read back, 366 us chained, 361 so; one after the
+        // other the same).
+        gn_track_kernel<<<dim3(track_run_ctas() / nslots, nslots), kTrackThreads, sizeof(TrackSmem), st>>>(d_sv,
+                                                                                                          frame_mode);
         return;
     }
     track_begin_kernel<<<nslots, 32, 0, st>>>(d_sv, frame_mode);
